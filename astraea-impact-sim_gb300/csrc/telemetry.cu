@@ -15,6 +15,26 @@
 //   pass C   remnant iterations 1..4 (skipped once one finds nothing bound)
 //   pass D   bound-planet / disk / ejecta / bound-impactor masses  :1176-1230
 //
+// Cost.  This GPU executes about two FP64 operations a clock on an SM (128
+// FP32 ones), so the passes are bound by the number of FP64 instructions a
+// particle costs, not by the 28-57 bytes it reads: at 1M, one FP64
+// instruction a particle is 1.6 us.  What is in FP64 is what is summed;
+// everything else avoids it:
+//   * float -> double is exact on the integer pipes (toDouble);
+//   * the decisions (bound? disk? inside the spin radius?) are taken in FP32
+//     with a margin of 1e-5 of the compared magnitudes, some fifty times the
+//     FP32 rounding of these expressions; a particle inside the margin, or
+//     whose FP32 values are not finite, takes the engine's FP64 expression,
+//     so every decision is the FP64 one;
+//   * sums that are sums of others (totals over the bodies, momentum) are
+//     formed once at the end, halves and unit factors are applied there;
+//   * a warp reduces its K sums in about K FP64 adds a lane (each exchange
+//     halves the values a lane carries) instead of 5 K;
+//   * the last block sums the blocks' partials with a warp per slot and does
+//     the divisions of the results on separate lanes.
+// Sum of the seven kernels: 1M particles 959 -> 303 us, 30k 200 -> 106 us (there
+// each pass is one wave of latency: loads, the reduction, the last block).
+//
 // Determinism: each pass is a grid-stride loop over a fixed grid, a block
 // reduction in a fixed order, per-block partials in global memory, and a
 // final sum over the blocks in block order by the last block to finish (an
@@ -23,8 +43,6 @@
 //
 // Scratch (partials, pass state, result) is file-scope device memory: the
 // call allocates nothing, and calls must not overlap on the GPU.
-#include <math_constants.h>
-
 #include "kernels.h"
 
 namespace astraea_gb300 {
@@ -35,54 +53,107 @@ constexpr int kTelMaxBlocks = 512;
 constexpr int kTelSlots = 32;
 constexpr double kGPsu = 6.67430e-11 * 1.0e24 * 1.0e3 * 1.0e3 / (1.0e6 * 1.0e6 * 1.0e6);   // engine/units.hpp:27
 
-// Pass A slot layout.
+// Pass A slot layout: seven sums of body 0, the same seven of the rest, then
+// 2 KE, 2 PE, IE, L and the radiated power.
 enum SlotA {
-    kMass = 0, kSysX, kSysY, kSysZ,
-    kM0, kX0, kY0, kZ0, kVx0, kVy0, kVz0,
+    kM0 = 0, kX0, kY0, kZ0, kVx0, kVy0, kVz0,
     kM1, kX1, kY1, kZ1, kVx1, kVy1, kVz1,
-    kKe, kPe, kIe, kPx, kPy, kPz, kLx, kLy, kLz, kRad,
+    kKe2, kPe2, kIe, kLx, kLy, kLz, kRad,
     kSlotsA
 };
 // Remnant-pass slot layout (passes B and C); B adds two spin slots at the end.
 enum SlotR { kRM = 0, kRX, kRY, kRZ, kRVx, kRVy, kRVz, kRMR2, kSpinL, kSpinI, kSlotsB };
 enum SlotD { kBound = 0, kDisk, kEjecta, kImpBound, kSlotsD };
 
+// (double)f on the integer pipes, exact for every float: a normal number's
+// exponent is rebiased (127 -> 1023) and its fraction moved up 29 bits;
+// subnormals are scaled by 2^24 first; infinities and NaNs take the top exponent.
+__device__ __forceinline__ double toDouble(float f) {
+    const uint32_t raw = __float_as_uint(f);
+    const bool sub = (raw & 0x7f800000u) == 0u;
+    const uint32_t u = sub ? __float_as_uint(f * 16777216.0f) : raw;     // zero stays zero
+    const uint32_t mag = u & 0x7fffffffu;
+    uint32_t hi = (mag >> 3) + (sub ? 0x38000000u - (24u << 20) : 0x38000000u);
+    if (mag >= 0x7f800000u) hi = (mag >> 3) | 0x7ff00000u;
+    if (mag == 0u) hi = 0u;
+    return __hiloint2double(static_cast<int>(hi | (u & 0x80000000u)), static_cast<int>(u << 29));
+}
+
+// A double as two floats (hi + lo), so a float minus it loses nothing that
+// FP32 can hold.
+struct F2 { float hi, lo; };
+__device__ __forceinline__ F2 split(double d) {
+    const float h = static_cast<float>(d);
+    return F2{h, static_cast<float>(d - toDouble(h))};
+}
+__device__ __forceinline__ float minus(float a, F2 b) { return (a - b.hi) - b.lo; }
+
+// The remnant as the FP32 decisions read it, formed once by the block that
+// finds it (FP64 splits in every thread would cost more than the decisions).
+struct Remnant {
+    F2 x, y, z, vx, vy, vz;
+    float gm, rSoft, radius;
+};
+
 struct TelState {
     uint32_t ticket;            // last-block detection, reset by the last block
     uint32_t stop;              // a remnant iteration found nothing bound
     double remX, remY, remZ, remVx, remVy, remVz, remMass, remRadius;
     double x0, y0, z0, vx0, vy0, vz0;   // body-0 COM and mean velocity
+    double rSoft;               // softening of the remnant's potential
+    Remnant q;                  // the remnant in FP32
+    F2 bx, by, bz;              // body-0 COM in FP32
 };
 
 __device__ double g_partials[kTelMaxBlocks * kTelSlots];
-__device__ double g_maxA[kTelMaxBlocks * 3];        // max T, max P [GPa], max damage per block
-__device__ double g_minPhi[kTelMaxBlocks];
-__device__ uint32_t g_minIdx[kTelMaxBlocks];
+__device__ float g_maxA[kTelMaxBlocks * 3];         // max T, max P, max damage per block
+__device__ unsigned long long g_minKey[kTelMaxBlocks];   // lowest finite potential: {ordered phi, index}
 __device__ TelState g_state;
 __device__ AstraeaTelemetry g_out;
 
-__device__ __forceinline__ double warpSum(double v) {
+// Warp sums of kCnt values: each exchange sends one half of the values a
+// lane carries and adds the other half, so after five of them lane l carries
+// the warp's total of value `slot` (valid says whether it carries one).
+template <int kCnt, int kOff>
+struct WarpSums {
+    static __device__ __forceinline__ void run(double* v, int have, int& slot, bool& valid, double& out) {
+        constexpr int kHalf = (kCnt + 1) / 2;
+        const bool up = (threadIdx.x & kOff) != 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+        for (int k = 0; k < kHalf; ++k) {
+            const double a = v[k], b = (k + kHalf < kCnt) ? v[k + kHalf] : 0.0;
+            const double other = __shfl_xor_sync(0xffffffffu, up ? a : b, kOff);
+            v[k] = (up ? b : a) + other;
+        }
+        if (up) slot += kHalf;
+        WarpSums<kHalf, kOff / 2>::run(v, up ? have - kHalf : min(have, kHalf), slot, valid, out);
+    }
+};
+template <int kCnt>
+struct WarpSums<kCnt, 0> {
+    static __device__ __forceinline__ void run(double* v, int have, int&, bool& valid, double& out) {
+        valid = have >= 1;
+        out = v[0];
+    }
+};
 
-// Sums `cnt` per-thread values over the block (fixed order) and stores them
+// Sums kCnt per-thread values over the block (fixed order) and stores them
 // as this block's partials.
 template <int kCnt>
-__device__ __forceinline__ void blockPartials(const double (&v)[kCnt]) {
-    __shared__ double red[kTelThreads / 32][kTelSlots];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < kCnt; ++k) {
-        const double s = warpSum(v[k]);
-        if (lane == 0) red[warp][k] = s;
-    }
+__device__ __forceinline__ void blockPartials(double (&v)[kCnt]) {
+    static_assert(kCnt <= 32, "one value a lane after the exchanges");
+    __shared__ double red[kTelThreads / 32][kCnt];
+    int slot = 0;
+    bool valid = false;
+    double s = 0.0;
+    WarpSums<kCnt, 16>::run(v, kCnt, slot, valid, s);
+    if (valid) red[threadIdx.x >> 5][slot] = s;
     __syncthreads();
     if (threadIdx.x < kCnt) {
-        double s = 0.0;
-        for (int w = 0; w < kTelThreads / 32; ++w) s += red[w][threadIdx.x];
-        g_partials[blockIdx.x * kTelSlots + threadIdx.x] = s;
+        double t = red[0][threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < kTelThreads / 32; ++w) t += red[w][threadIdx.x];
+        g_partials[blockIdx.x * kTelSlots + threadIdx.x] = t;
     }
 }
 
@@ -101,30 +172,48 @@ __device__ __forceinline__ bool lastBlock() {
     return last;
 }
 
-__device__ __forceinline__ double sumPartials(int slot) {
-    double s = 0.0;
-    for (int b = 0; b < static_cast<int>(gridDim.x); ++b) s += __ldcg(&g_partials[b * kTelSlots + slot]);
-    return s;
+// The blocks' partials summed per slot into tot (shared): a warp per slot,
+// lane l over the blocks l, l + 32, ..., then over the lanes.
+template <int kCnt>
+__device__ __forceinline__ void gridTotals(double* tot) {
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < kCnt; k += kTelThreads / 32) {
+        double s = 0.0;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) s += __ldcg(&g_partials[b * kTelSlots + k]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) tot[k] = s;
+    }
+    __syncthreads();
+}
+
+// The derived members of the state, from the remnant the caller has stored
+// (after a barrier): a lane each.
+__device__ __forceinline__ void finishRemnant(TelState& s) {
+    const int t = threadIdx.x;
+    if (t < 6) (&s.q.x)[t] = split((&s.remX)[t]);
+    if (t == 6) s.q.gm = static_cast<float>(kGPsu * s.remMass);
+    if (t == 7) {
+        s.rSoft = fmax(0.5 * s.remRadius, 0.1);
+        s.q.rSoft = static_cast<float>(s.rSoft);
+        s.q.radius = static_cast<float>(s.remRadius);
+    }
+    if (t >= 8 && t < 11) (&s.bx)[t - 8] = split((&s.x0)[t - 8]);
 }
 
 __global__ void __launch_bounds__(kTelThreads) passA(AstraeaParticles p, uint32_t n, double targetRadius) {
     double v[kSlotsA];
 #pragma unroll
     for (int k = 0; k < kSlotsA; ++k) v[k] = 0.0;
-    double maxT = 0.0, maxP = 0.0, maxD = 0.0, minPhi = CUDART_INF;
-    uint32_t minIdx = 0u;
-    bool found = false;
+    float maxT = 0.0f, maxP = 0.0f, maxD = 0.0f;
+    unsigned long long minKey = ~0ull;
     for (uint32_t i = blockIdx.x * kTelThreads + threadIdx.x; i < n; i += gridDim.x * kTelThreads) {
-        const double m = p.mass[i];
-        const double x = p.posX[i], y = p.posY[i], z = p.posZ[i];
-        const double vx = p.velX[i], vy = p.velY[i], vz = p.velZ[i];
-        const double phi = p.phiGrav[i];
-        const double uVal = p.u[i];
-        const double temp = p.tempK[i];
-        const double presGPa = static_cast<double>(p.pressure[i]) * 1000.0;
-        v[kMass] += m;
-        v[kSysX] += m * x; v[kSysY] += m * y; v[kSysZ] += m * z;
-        if (p.bodyId[i] == 0u) {
+        const float fphi = __ldg(&p.phiGrav[i]), temp = __ldg(&p.tempK[i]), pres = __ldg(&p.pressure[i]);
+        const float fw = __ldg(&p.radPowerW[i]);
+        const double m = toDouble(__ldg(&p.mass[i]));
+        const double x = toDouble(__ldg(&p.posX[i])), y = toDouble(__ldg(&p.posY[i])), z = toDouble(__ldg(&p.posZ[i]));
+        const double vx = toDouble(__ldg(&p.velX[i])), vy = toDouble(__ldg(&p.velY[i])), vz = toDouble(__ldg(&p.velZ[i]));
+        if (__ldg(&p.bodyId[i]) == 0u) {
             v[kM0] += m;
             v[kX0] += m * x; v[kY0] += m * y; v[kZ0] += m * z;
             v[kVx0] += m * vx; v[kVy0] += m * vy; v[kVz0] += m * vz;
@@ -133,113 +222,155 @@ __global__ void __launch_bounds__(kTelThreads) passA(AstraeaParticles p, uint32_
             v[kX1] += m * x; v[kY1] += m * y; v[kZ1] += m * z;
             v[kVx1] += m * vx; v[kVy1] += m * vy; v[kVz1] += m * vz;
         }
-        v[kKe] += 0.5 * m * (vx * vx + vy * vy + vz * vz);
-        v[kPe] += 0.5 * m * phi;
-        v[kIe] += m * uVal;
-        v[kPx] += m * vx; v[kPy] += m * vy; v[kPz] += m * vz;
+        v[kKe2] += m * (vx * vx + vy * vy + vz * vz);
+        v[kPe2] += m * toDouble(fphi);
+        v[kIe] += m * toDouble(__ldg(&p.u[i]));
         v[kLx] += m * (y * vz - z * vy);
         v[kLy] += m * (z * vx - x * vz);
         v[kLz] += m * (x * vy - y * vx);
-        const double w = p.radPowerW[i];
-        if (isfinite(w) && w > 0.0) v[kRad] += w;
-        if (isfinite(temp)) maxT = fmax(maxT, temp);
-        if (isfinite(presGPa)) maxP = fmax(maxP, presGPa);
-        maxD = fmax(maxD, static_cast<double>(p.damage[i]));
-        if (isfinite(phi) && (!found || phi < minPhi)) { minPhi = phi; minIdx = i; found = true; }
+        if (isfinite(fw) && fw > 0.0f) v[kRad] += toDouble(fw);
+        if (isfinite(temp)) maxT = fmaxf(maxT, temp);
+        if (isfinite(pres)) maxP = fmaxf(maxP, pres);
+        maxD = fmaxf(maxD, __ldg(&p.damage[i]));
+        if (isfinite(fphi)) {                        // + 0: the two zeros compare equal
+            const unsigned long long key = (static_cast<unsigned long long>(orderedFromFloat(fphi + 0.0f)) << 32) | i;
+            minKey = key < minKey ? key : minKey;
+        }
     }
     blockPartials<kSlotsA>(v);
     // maxima and the first index of the lowest potential, by warp then block
-    __shared__ double smax[3][kTelThreads / 32];
-    __shared__ double sphi[kTelThreads / 32];
-    __shared__ uint32_t sidx[kTelThreads / 32];
-    if (!found) minIdx = 0xffffffffu;
+    __shared__ float smax[3][kTelThreads / 32];
+    __shared__ unsigned long long skey[kTelThreads / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    maxT = warpMaxF(maxT); maxP = warpMaxF(maxP); maxD = warpMaxF(maxD);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        maxT = fmax(maxT, __shfl_xor_sync(0xffffffffu, maxT, o));
-        maxP = fmax(maxP, __shfl_xor_sync(0xffffffffu, maxP, o));
-        maxD = fmax(maxD, __shfl_xor_sync(0xffffffffu, maxD, o));
-        const double oPhi = __shfl_xor_sync(0xffffffffu, minPhi, o);
-        const uint32_t oIdx = __shfl_xor_sync(0xffffffffu, minIdx, o);
-        if (oIdx != 0xffffffffu && (minIdx == 0xffffffffu || oPhi < minPhi || (oPhi == minPhi && oIdx < minIdx))) {
-            minPhi = oPhi;
-            minIdx = oIdx;
-        }
+        const unsigned long long k = __shfl_xor_sync(0xffffffffu, minKey, o);
+        minKey = k < minKey ? k : minKey;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { smax[0][warp] = maxT; smax[1][warp] = maxP; smax[2][warp] = maxD; sphi[warp] = minPhi; sidx[warp] = minIdx; }
+    if (lane == 0) { smax[0][warp] = maxT; smax[1][warp] = maxP; smax[2][warp] = maxD; skey[warp] = minKey; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, bP = 0.0, d = 0.0, ph = CUDART_INF;
-        uint32_t ix = 0xffffffffu;
-        for (int k = 0; k < kTelThreads / 32; ++k) {
-            a = fmax(a, smax[0][k]); bP = fmax(bP, smax[1][k]); d = fmax(d, smax[2][k]);
-            if (sidx[k] != 0xffffffffu && (ix == 0xffffffffu || sphi[k] < ph || (sphi[k] == ph && sidx[k] < ix))) {
-                ph = sphi[k];
-                ix = sidx[k];
-            }
-        }
-        g_maxA[3 * blockIdx.x + 0] = a; g_maxA[3 * blockIdx.x + 1] = bP; g_maxA[3 * blockIdx.x + 2] = d;
-        g_minPhi[blockIdx.x] = ph;
-        g_minIdx[blockIdx.x] = ix;
+    if (threadIdx.x < 3) {
+        float a = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kTelThreads / 32; ++k) a = fmaxf(a, smax[threadIdx.x][k]);
+        g_maxA[3 * blockIdx.x + threadIdx.x] = a;
+    } else if (threadIdx.x == 32) {
+        unsigned long long k0 = ~0ull;
+#pragma unroll
+        for (int k = 0; k < kTelThreads / 32; ++k) k0 = skey[k] < k0 ? skey[k] : k0;
+        g_minKey[blockIdx.x] = k0;
     }
     if (!lastBlock()) return;
     __shared__ double tot[kSlotsA];
-    if (threadIdx.x < kSlotsA) tot[threadIdx.x] = sumPartials(threadIdx.x);
+    __shared__ float sMaxAll[3];
+    __shared__ uint32_t sSeed;
+    gridTotals<kSlotsA>(tot);
+    if (warp < 3) {
+        float a = 0.0f;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) a = fmaxf(a, __ldcg(&g_maxA[3 * b + warp]));
+        a = warpMaxF(a);
+        if (lane == 0) sMaxAll[warp] = a;
+    } else if (warp == 3) {
+        unsigned long long k0 = ~0ull;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) {
+            const unsigned long long k = __ldcg(&g_minKey[b]);
+            k0 = k < k0 ? k : k0;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long k = __shfl_xor_sync(0xffffffffu, k0, o);
+            k0 = k < k0 ? k : k0;
+        }
+        if (lane == 0) sSeed = (k0 == ~0ull) ? 0u : static_cast<uint32_t>(k0);   // :999 (no finite potential)
+    }
     __syncthreads();
-    if (threadIdx.x != 0) return;
     AstraeaTelemetry& o = g_out;
     TelState& s = g_state;
-    double a = 0.0, bP = 0.0, d = 0.0, ph = CUDART_INF;
-    uint32_t seed = 0xffffffffu;
-    for (int k = 0; k < static_cast<int>(gridDim.x); ++k) {
-        a = fmax(a, __ldcg(&g_maxA[3 * k])); bP = fmax(bP, __ldcg(&g_maxA[3 * k + 1]));
-        d = fmax(d, __ldcg(&g_maxA[3 * k + 2]));
-        const uint32_t ix = __ldcg(&g_minIdx[k]);
-        const double pk = __ldcg(&g_minPhi[k]);
-        if (ix != 0xffffffffu && (seed == 0xffffffffu || pk < ph || (pk == ph && ix < seed))) { ph = pk; seed = ix; }
+    const double M = tot[kM0] + tot[kM1];
+    // one division a lane: lanes 0..5 body 0's COM and mean velocity, 6..11
+    // the rest's, 12..14 the system's COM (:1049-1074)
+    __shared__ double com[15];
+    if (threadIdx.x < 15) {
+        const int k = threadIdx.x;
+        const double num = k < 6 ? tot[kX0 + k] : (k < 12 ? tot[kX1 + k - 6] : tot[kX0 + k - 12] + tot[kX1 + k - 12]);
+        const double den = k < 6 ? tot[kM0] : (k < 12 ? tot[kM1] : M);
+        com[k] = den > 0.0 ? num / den : (k < 12 ? num : 0.0);
     }
-    if (seed == 0xffffffffu) seed = 0u;                          // :999 (no finite potential)
-    o.totalMassPsu = tot[kMass];
-    o.kineticPsu = tot[kKe]; o.potentialPsu = tot[kPe]; o.internalPsu = tot[kIe];
-    o.momentumPsu[0] = tot[kPx]; o.momentumPsu[1] = tot[kPy]; o.momentumPsu[2] = tot[kPz];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+    const uint32_t seed = sSeed;
+    o.totalMassPsu = M;
+    o.kineticPsu = 0.5 * tot[kKe2]; o.potentialPsu = 0.5 * tot[kPe2]; o.internalPsu = tot[kIe];
     o.angularMomentumPsu[0] = tot[kLx]; o.angularMomentumPsu[1] = tot[kLy]; o.angularMomentumPsu[2] = tot[kLz];
-    o.maxTempK = a; o.maxPressureGPa = bP; o.maxDamage = d;
+    o.maxTempK = sMaxAll[0]; o.maxPressureGPa = static_cast<double>(sMaxAll[1]) * 1000.0; o.maxDamage = sMaxAll[2];
     o.radiatedPowerW = tot[kRad];
     o.remnantSeedIndex = seed;
-    if (tot[kMass] > 0.0) {                                      // :1049-1056
-        o.sysComPsu[0] = tot[kSysX] / tot[kMass];
-        o.sysComPsu[1] = tot[kSysY] / tot[kMass];
-        o.sysComPsu[2] = tot[kSysZ] / tot[kMass];
-    } else {
-        o.sysComPsu[0] = o.sysComPsu[1] = o.sysComPsu[2] = 0.0;
-    }
-    const double m0 = tot[kM0], m1 = tot[kM1];
-    o.massBody0Psu = m0;
-    o.massOtherPsu = m1;
-    double c0[6], c1[6];
-    for (int k = 0; k < 6; ++k) {
-        c0[k] = tot[kX0 + k];
-        c1[k] = tot[kX1 + k];
-    }
-    if (m0 > 0.0)                                                // :1058-1069
-        for (int k = 0; k < 6; ++k) c0[k] /= m0;
-    if (m1 > 0.0)                                                // :1071-1074
-        for (int k = 0; k < 6; ++k) c1[k] /= m1;
+    o.massBody0Psu = tot[kM0];
+    o.massOtherPsu = tot[kM1];
     for (int k = 0; k < 3; ++k) {
-        o.comBody0Psu[k] = c0[k]; o.velBody0Psu[k] = c0[3 + k];
-        o.comOtherPsu[k] = c1[k]; o.velOtherPsu[k] = c1[3 + k];
-        o.livingComPsu[k] = m0 > 0.0 ? c0[k] : o.sysComPsu[k];
+        o.momentumPsu[k] = tot[kVx0 + k] + tot[kVx1 + k];
+        o.sysComPsu[k] = com[12 + k];
+        o.comBody0Psu[k] = com[k]; o.velBody0Psu[k] = com[3 + k];
+        o.comOtherPsu[k] = com[6 + k]; o.velOtherPsu[k] = com[9 + k];
+        o.livingComPsu[k] = tot[kM0] > 0.0 ? com[k] : com[12 + k];
     }
-    s.x0 = c0[0]; s.y0 = c0[1]; s.z0 = c0[2]; s.vx0 = c0[3]; s.vy0 = c0[4]; s.vz0 = c0[5];
+    s.x0 = com[0]; s.y0 = com[1]; s.z0 = com[2]; s.vx0 = com[3]; s.vy0 = com[4]; s.vz0 = com[5];
     // remnant seed, :1121-1128
     s.remX = p.posX[seed]; s.remY = p.posY[seed]; s.remZ = p.posZ[seed];
     s.remVx = p.velX[seed]; s.remVy = p.velY[seed]; s.remVz = p.velZ[seed];
-    s.remMass = fmax(m0, tot[kMass] * 0.5);
+    s.remMass = fmax(tot[kM0], M * 0.5);
     s.remRadius = fmax(targetRadius, 0.25);
     s.stop = 0u;
     o.spinLPsu = 0.0;
     o.spinIPsu = 0.0;
     o.remnantIterations = 0;
+    }
+    __syncthreads();
+    finishRemnant(s);
+}
+
+// Decisions taken in FP32 where the two sides differ by more than kMargin of
+// their magnitudes (kTiny: an absolute floor far above FP32 underflow).
+constexpr float kMargin = 1.0e-5f, kTiny = 1.0e-28f;
+enum Verdict { kNo = 0, kYes = 1, kUnsure = 2 };
+__device__ __forceinline__ Verdict less(float a, float b, float scale) {   // a < b?
+    const float d = a - b, t = kMargin * scale + kTiny;
+    return d < -t ? kYes : (d > t ? kNo : kUnsure);        // a NaN or infinity compares false twice
+}
+
+struct Rel { float dx, dy, dz, dvx, dvy, dvz, r2, v2, r; };
+__device__ __forceinline__ Rel relative(const Remnant& q, float x, float y, float z, float vx, float vy, float vz) {
+    Rel o;
+    o.dx = minus(x, q.x); o.dy = minus(y, q.y); o.dz = minus(z, q.z);
+    o.dvx = minus(vx, q.vx); o.dvy = minus(vy, q.vy); o.dvz = minus(vz, q.vz);
+    o.r2 = o.dx * o.dx + o.dy * o.dy + o.dz * o.dz;
+    o.v2 = o.dvx * o.dvx + o.dvy * o.dvy + o.dvz * o.dvz;
+    o.r = sqrtf(o.r2);
+    return o;
+}
+// v^2 / 2 < G M / max(r, rSoft), multiplied out.
+__device__ __forceinline__ Verdict boundTest(const Remnant& q, const Rel& d) {
+    const float lhs = 0.5f * d.v2 * fmaxf(d.r, q.rSoft);
+    return less(lhs, q.gm, lhs + q.gm);
+}
+
+// The engine's FP64 specific energy (:1144-1151, :1190-1196).
+static __device__ __noinline__ double energyF64(const TelState& s, double rSoft, float x, float y, float z, float vx,
+                                             float vy, float vz) {
+    const double dx = x - s.remX, dy = y - s.remY, dz = z - s.remZ;
+    const double dvx = vx - s.remVx, dvy = vy - s.remVy, dvz = vz - s.remVz;
+    const double r = sqrt(dx * dx + dy * dy + dz * dz);
+    return 0.5 * (dvx * dvx + dvy * dvy + dvz * dvz) + (-kGPsu * s.remMass / fmax(r, rSoft));
+}
+
+// What a remnant pass reads of a particle; the loops load the next particle
+// before they work on the current one.
+struct TelIn { float x, y, z, vx, vy, vz, m; uint32_t body; };
+template <bool kBody>
+__device__ __forceinline__ TelIn telLoad(const AstraeaParticles& p, uint32_t i) {
+    return TelIn{__ldg(&p.posX[i]), __ldg(&p.posY[i]), __ldg(&p.posZ[i]), __ldg(&p.velX[i]), __ldg(&p.velY[i]),
+                 __ldg(&p.velZ[i]), __ldg(&p.mass[i]), kBody ? static_cast<uint32_t>(__ldg(&p.bodyId[i])) : 0u};
 }
 
 // Remnant iteration (:1131-1174), plus the living-body spin sums in pass B.
@@ -252,30 +383,46 @@ __global__ void __launch_bounds__(kTelThreads) passRemnant(AstraeaParticles p, u
     double v[kCnt];
 #pragma unroll
     for (int k = 0; k < kCnt; ++k) v[k] = 0.0;
-    const double rSoft = fmax(0.5 * s.remRadius, 0.1);
+    const double rSoft = s.rSoft;
+    const Remnant q = s.q;
     const double rLimSq = (1.5 * targetRadius) * (1.5 * targetRadius);
-    for (uint32_t i = blockIdx.x * kTelThreads + threadIdx.x; i < n; i += gridDim.x * kTelThreads) {
-        const double x = p.posX[i], y = p.posY[i], z = p.posZ[i];
-        const double vx = p.velX[i], vy = p.velY[i], vz = p.velZ[i];
-        const double m = p.mass[i];
-        const double dx = x - s.remX, dy = y - s.remY, dz = z - s.remZ;
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double r = sqrt(r2);
-        const double dvx = vx - s.remVx, dvy = vy - s.remVy, dvz = vz - s.remVz;
-        const double v2 = dvx * dvx + dvy * dvy + dvz * dvz;
-        const double phiRem = -kGPsu * s.remMass / fmax(r, rSoft);
-        const double eSpec = 0.5 * v2 + phiRem;
-        if (eSpec < 0.0) {
-            v[kRM] += m;
-            v[kRX] += m * x; v[kRY] += m * y; v[kRZ] += m * z;
-            v[kRVx] += m * vx; v[kRVy] += m * vy; v[kRVz] += m * vz;
-            v[kRMR2] += m * r2;
-        }
+    const F2 bx = s.bx, by = s.by, bz = s.bz;
+    const uint32_t stride = gridDim.x * kTelThreads, i0 = blockIdx.x * kTelThreads + threadIdx.x;
+    TelIn next{};
+    if (i0 < n) next = telLoad<kWithSpin>(p, i0);
+    for (uint32_t i = i0; i < n; i += stride) {
+        const TelIn in = next;
+        if (n - i > stride) next = telLoad<kWithSpin>(p, i + stride);
+        const float fx = in.x, fy = in.y, fz = in.z, fvx = in.vx, fvy = in.vy, fvz = in.vz, fm = in.m;
+        bool spin = kWithSpin && living && in.body == 0u;
+        const Verdict b = boundTest(q, relative(q, fx, fy, fz, fvx, fvy, fvz));
+        const bool bound = b == kUnsure ? energyF64(s, rSoft, fx, fy, fz, fvx, fvy, fvz) < 0.0 : b == kYes;
         if constexpr (kWithSpin) {
-            if (living && p.bodyId[i] == 0u) {                   // :1097-1111
-                const double ex = x - s.x0, ey = y - s.y0, ez = z - s.z0;
-                if (ex * ex + ey * ey + ez * ez <= rLimSq) {
-                    const double evx = vx - s.vx0, evz = vz - s.vz0;
+            if (spin) {                                          // :1097-1111
+                const float gx = minus(fx, bx), gy = minus(fy, by), gz = minus(fz, bz);
+                const float g2 = gx * gx + gy * gy + gz * gz, lim = static_cast<float>(rLimSq);
+                const Verdict near = less(g2, lim, g2 + lim);
+                if (near == kUnsure) {
+                    const double ex = fx - s.x0, ey = fy - s.y0, ez = fz - s.z0;
+                    spin = ex * ex + ey * ey + ez * ez <= rLimSq;
+                } else {
+                    spin = near == kYes;
+                }
+            }
+        }
+        if (bound || spin) {
+            const double m = toDouble(fm), x = toDouble(fx), y = toDouble(fy), z = toDouble(fz);
+            const double vx = toDouble(fvx), vy = toDouble(fvy), vz = toDouble(fvz);
+            if (bound) {
+                const double dx = x - s.remX, dy = y - s.remY, dz = z - s.remZ;
+                v[kRM] += m;
+                v[kRX] += m * x; v[kRY] += m * y; v[kRZ] += m * z;
+                v[kRVx] += m * vx; v[kRVy] += m * vy; v[kRVz] += m * vz;
+                v[kRMR2] += m * (dx * dx + dy * dy + dz * dz);
+            }
+            if constexpr (kWithSpin) {
+                if (spin) {
+                    const double ex = x - s.x0, ez = z - s.z0, evx = vx - s.vx0, evz = vz - s.vz0;
                     v[kSpinL] += m * (ez * evx - ex * evz);
                     v[kSpinI] += m * (ex * ex + ez * ez);
                 }
@@ -285,66 +432,97 @@ __global__ void __launch_bounds__(kTelThreads) passRemnant(AstraeaParticles p, u
     blockPartials<kCnt>(v);
     if (!lastBlock()) return;
     __shared__ double tot[kCnt];
-    if (threadIdx.x < kCnt) tot[threadIdx.x] = sumPartials(threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x != 0) return;
+    gridTotals<kCnt>(tot);
     if constexpr (kWithSpin) {
-        g_out.spinLPsu = tot[kSpinL];
-        g_out.spinIPsu = tot[kSpinI];
+        if (threadIdx.x == 32) {
+            g_out.spinLPsu = tot[kSpinL];
+            g_out.spinIPsu = tot[kSpinI];
+        }
     }
     const double nm = tot[kRM];
     if (nm > 0.0) {                                              // :1162-1173
-        TelState& w = g_state;
-        w.remMass = nm;
-        w.remX = tot[kRX] / nm; w.remY = tot[kRY] / nm; w.remZ = tot[kRZ] / nm;
-        w.remVx = tot[kRVx] / nm; w.remVy = tot[kRVy] / nm; w.remVz = tot[kRVz] / nm;
-        const double rmsR = sqrt(tot[kRMR2] / nm);
-        w.remRadius = fmax(0.5 * targetRadius, sqrt(5.0 / 3.0) * rmsR);
-        g_out.remnantIterations += 1;
-    } else {
+        if (threadIdx.x < 6) (&g_state.remX)[threadIdx.x] = tot[kRX + threadIdx.x] / nm;
+        if (threadIdx.x == 6) {
+            g_state.remMass = nm;
+            g_state.remRadius = fmax(0.5 * targetRadius, sqrt(5.0 / 3.0) * sqrt(tot[kRMR2] / nm));
+            g_out.remnantIterations += 1;
+        }
+        __syncthreads();
+        finishRemnant(g_state);
+    } else if (threadIdx.x == 0) {
         g_state.stop = 1u;
     }
+}
+
+// The engine's FP64 disk test of a bound particle (:1201-1216).
+static __device__ __noinline__ bool diskF64(const TelState& s, double rSoft, float x, float y, float z, float vx,
+                                            float vy, float vz) {
+    const double mu = kGPsu * s.remMass;
+    const double dx = x - s.remX, dy = y - s.remY, dz = z - s.remZ;
+    const double dvx = vx - s.remVx, dvy = vy - s.remVy, dvz = vz - s.remVz;
+    const double r = sqrt(dx * dx + dy * dy + dz * dz);
+    if (!(r > s.remRadius && mu > 0.0)) return false;
+    const double eSpec = 0.5 * (dvx * dvx + dvy * dvy + dvz * dvz) + (-mu / fmax(r, rSoft));
+    const double jx = dy * dvz - dz * dvy, jy = dz * dvx - dx * dvz, jz = dx * dvy - dy * dvx;
+    const double j2 = jx * jx + jy * jy + jz * jz;
+    const double ecc = sqrt(fmax(0.0, 1.0 + (2.0 * eSpec * j2) / (mu * mu)));
+    return j2 / (mu * (1.0 + ecc)) > s.remRadius;
+}
+
+// The same test in FP32.  With p = j^2 / mu the engine's condition
+// p / (1 + e) > R, e^2 = max(0, 1 + 2 E p / mu), squares to
+// j^2 > mu R and j^2 > 2 mu R + 2 E R^2 (E the specific energy): no root, no
+// division by a difference.
+__device__ __forceinline__ Verdict diskTest(const Remnant& q, const Rel& d) {
+    const float R = q.radius;
+    if (!(q.gm > kTiny)) return kUnsure;
+    const Verdict out = less(R, d.r, R + d.r);
+    if (out != kYes) return out;
+    const float jx = d.dy * d.dvz - d.dz * d.dvy, jy = d.dz * d.dvx - d.dx * d.dvz, jz = d.dx * d.dvy - d.dy * d.dvx;
+    const float j2 = jx * jx + jy * jy + jz * jz;
+    const float pot = q.gm / fmaxf(d.r, q.rSoft), R2 = R * R, muR = q.gm * R;
+    const float scale = d.r2 * d.v2 + R2 * (d.v2 + 2.0f * pot) + 2.0f * muR;
+    const Verdict a = less(muR, j2, scale);
+    const Verdict b = less(2.0f * muR + R2 * (d.v2 - 2.0f * pot), j2, scale);
+    if (a == kNo || b == kNo) return kNo;
+    return (a == kYes && b == kYes) ? kYes : kUnsure;
 }
 
 // Final classification (:1176-1230).
 __global__ void __launch_bounds__(kTelThreads) passClassify(AstraeaParticles p, uint32_t n) {
     const TelState s = g_state;
     double v[kSlotsD] = {0.0, 0.0, 0.0, 0.0};
-    const double rSoft = fmax(0.5 * s.remRadius, 0.1);
-    const double mu = kGPsu * s.remMass;
-    for (uint32_t i = blockIdx.x * kTelThreads + threadIdx.x; i < n; i += gridDim.x * kTelThreads) {
-        const double m = p.mass[i];
-        const double dx = static_cast<double>(p.posX[i]) - s.remX;
-        const double dy = static_cast<double>(p.posY[i]) - s.remY;
-        const double dz = static_cast<double>(p.posZ[i]) - s.remZ;
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double dvx = static_cast<double>(p.velX[i]) - s.remVx;
-        const double dvy = static_cast<double>(p.velY[i]) - s.remVy;
-        const double dvz = static_cast<double>(p.velZ[i]) - s.remVz;
-        const double v2 = dvx * dvx + dvy * dvy + dvz * dvz;
-        const double eSpec = 0.5 * v2 + (-mu / fmax(r, rSoft));
-        if (eSpec >= 0.0) {
+    const double rSoft = s.rSoft;
+    const Remnant q = s.q;
+    const uint32_t stride = gridDim.x * kTelThreads, i0 = blockIdx.x * kTelThreads + threadIdx.x;
+    TelIn next{};
+    if (i0 < n) next = telLoad<true>(p, i0);
+    for (uint32_t i = i0; i < n; i += stride) {
+        const TelIn in = next;
+        if (n - i > stride) next = telLoad<true>(p, i + stride);
+        const float fx = in.x, fy = in.y, fz = in.z, fvx = in.vx, fvy = in.vy, fvz = in.vz;
+        const double m = toDouble(in.m);
+        const Rel d = relative(q, fx, fy, fz, fvx, fvy, fvz);
+        const Verdict e = boundTest(q, d);
+        // a NaN energy counts as bound here and as unbound above, as in the engine
+        const bool bound = e == kUnsure ? !(energyF64(s, rSoft, fx, fy, fz, fvx, fvy, fvz) >= 0.0) : e == kYes;
+        bool disk = false;
+        if (bound) {
+            const Verdict k = diskTest(q, d);
+            disk = k == kUnsure ? diskF64(s, rSoft, fx, fy, fz, fvx, fvy, fvz) : k == kYes;
+        }
+        if (!bound) {
             v[kEjecta] += m;
         } else {
-            if (p.bodyId[i] != 0u) v[kImpBound] += m;
-            bool disk = false;
-            if (r > s.remRadius && mu > 0.0) {
-                const double jx = dy * dvz - dz * dvy;
-                const double jy = dz * dvx - dx * dvz;
-                const double jz = dx * dvy - dy * dvx;
-                const double j2 = jx * jx + jy * jy + jz * jz;
-                const double ecc = sqrt(fmax(0.0, 1.0 + (2.0 * eSpec * j2) / (mu * mu)));
-                const double rPeri = j2 / (mu * (1.0 + ecc));
-                disk = rPeri > s.remRadius;
-            }
-            v[disk ? kDisk : kBound] += m;
+            if (in.body != 0u) v[kImpBound] += m;
+            if (disk) v[kDisk] += m;
+            else v[kBound] += m;
         }
     }
     blockPartials<kSlotsD>(v);
     if (!lastBlock()) return;
     __shared__ double tot[kSlotsD];
-    if (threadIdx.x < kSlotsD) tot[threadIdx.x] = sumPartials(threadIdx.x);
-    __syncthreads();
+    gridTotals<kSlotsD>(tot);
     if (threadIdx.x != 0) return;
     AstraeaTelemetry& o = g_out;
     o.boundPlanetMassPsu = tot[kBound];

@@ -211,3 +211,41 @@ def test_gpu_telemetry_empty_and_single_body():
     p = engine.DeviceParticles(len(st["posX"]))
     p.upload(st)
     compare(engine.reduce_telemetry(p, 1.0), oracle.telemetry(st, 1.0), rtol=1e-10)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 33, 255, 257, 4099, 80001])
+def test_gpu_telemetry_decisions_at_the_margin(n):
+    """Particles whose energy and periapsis lie within FP32 rounding of the
+    engine's FP64 decisions, at sizes around a warp, a block and the grid: a
+    decision taken otherwise moves a mass sum by about 1/n of its scale, far
+    above the 1e-10 of the summation order."""
+    from astraea_gb300 import engine
+    rng = np.random.default_rng(n)
+    st = scenarios.empty_state(n)
+    m0 = 10.0
+    st["mass"][:] = 1.0e-6
+    st["mass"][0] = m0                          # the remnant: the heavy particle at rest in the centre
+    st["bodyId"][1:] = rng.integers(0, 3, n - 1)
+    st["phiGrav"][:] = -1.0
+    st["phiGrav"][0] = -5.0
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    r = np.where(rng.random(n) < 0.3, 1.5, rng.uniform(0.3, 20.0, n))    # many at the spin radius too
+    t = np.cross(u, rng.normal(size=(n, 3)))
+    t /= np.linalg.norm(t, axis=1)[:, None]
+    vesc = np.sqrt(2.0 * G_PSU * m0 / r)
+    near = 1.0 + rng.choice([-3e-6, -1e-7, 0.0, 1e-7, 3e-6], n)
+    v = np.where(rng.random(n) < 0.5, vesc * near, vesc * rng.uniform(0.2, 0.99, n))
+    v[0] = r[0] = 0.0
+    for k, (a, b) in enumerate((("posX", "velX"), ("posY", "velY"), ("posZ", "velZ"))):
+        st[a][:] = r * u[:, k]
+        st[b][:] = v * t[:, k]
+    p = engine.DeviceParticles(n)
+    p.upload(st)
+    got, ref = engine.reduce_telemetry(p, 1.0), oracle.telemetry(st, 1.0)
+    for k in ("ejectaMassPsu", "boundPlanetMassPsu", "diskMassPsu", "impactorBoundMassPsu", "remnantMassPsu",
+              "spinIPsu"):
+        assert abs(got[k] - ref[k]) <= 1e-10 * max(abs(ref[k]), 1e-6), (k, got[k], ref[k])
+    for k in EXACT:
+        assert got[k] == ref[k], (k, got[k], ref[k])
