@@ -12,11 +12,27 @@
 
 namespace astraea_gb300 {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;   // 4096 keys per tile
+constexpr int kSortThreads = 512;
 constexpr int kSortBins = 256;
 constexpr int kSortMaxPasses = 8;
+
+// Keys a thread of the tiled passes holds (a tile is 512 times that): small
+// tiles put more blocks on the GPU while there are few, large ones amortise a
+// tile's fixed chain (sort.cu).
+constexpr uint32_t kSortSmallTileMax = 1u << 19, kSortMiddleTileMax = 1u << 22;
+constexpr int sortItems(uint32_t n) { return n <= kSortSmallTileMax ? 4 : (n <= kSortMiddleTileMax ? 8 : 12); }
+constexpr uint32_t sortTilesOf(uint32_t n) {
+    const uint32_t tile = static_cast<uint32_t>(kSortThreads * sortItems(n));
+    return n == 0u ? 1u : (n - 1u) / tile + 1u;
+}
+// The most tiles of any sort of at most n keys (scratch is kept for a
+// capacity, and the tile grows with n).
+constexpr uint32_t sortTiles(uint32_t n) {
+    uint32_t t = sortTilesOf(n);
+    if (n > kSortSmallTileMax && sortTilesOf(kSortSmallTileMax) > t) t = sortTilesOf(kSortSmallTileMax);
+    if (n > kSortMiddleTileMax && sortTilesOf(kSortMiddleTileMax) > t) t = sortTilesOf(kSortMiddleTileMax);
+    return t;
+}
 
 // Onesweep scratch layout (32-bit words):
 //   [0, kSortHistWords)                              digit histograms, one per pass
@@ -24,7 +40,6 @@ constexpr int kSortMaxPasses = 8;
 //   then kSortMaxPasses * tiles * kSortBins          look-back status words
 constexpr size_t kSortHistWords = static_cast<size_t>(kSortMaxPasses) * kSortBins;
 constexpr size_t kSortCounterWords = 8;
-constexpr uint32_t sortTiles(uint32_t n) { return n == 0u ? 1u : (n + kSortTile - 1u) / kSortTile; }
 constexpr size_t sortScratchWordsFor(uint32_t n) {
     return kSortHistWords + kSortCounterWords + static_cast<size_t>(kSortMaxPasses) * sortTiles(n) * kSortBins;
 }

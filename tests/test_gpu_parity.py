@@ -419,3 +419,57 @@ def test_c1_twenty_steps_track_oracle():
         mom = [np.sum(m * s[k].astype(np.float64)) for k in ("velX", "velY", "velZ")]
         scale = np.sum(m * np.sqrt(sum(s[k].astype(np.float64) ** 2 for k in ("velX", "velY", "velZ"))))
         assert max(abs(x) for x in mom) < 1e-4 * scale
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [31, 32, 33, 511, 1025, 16 * 1024, 16 * 1024 + 1, 50_001, 114_687, 114_688, 114_689, 4096 * 65 + 1])
+@pytest.mark.parametrize("end_bit", [7, 40, 64])
+def test_radix_sort_one_launch_and_tiled_sizes(n, end_bit):
+    """Sizes around the one-launch sort's ends (32 and 114,688 keys), its rounds
+    of 1,024 keys a block, and a tiled sort whose look-back crosses several
+    windows; keys with few distinct digits, so runs of equal keys span blocks."""
+    from astraea_gb300 import engine
+    rng = np.random.default_rng(n + end_bit)
+    keys = rng.integers(0, 2 ** 63, n, dtype=np.uint64) & np.uint64(0x8300000000050103 if n % 2 else 2 ** 64 - 1)
+    vals = np.arange(n, dtype=np.int32)
+    ks, vs = engine.radix_sort_pairs(torch.from_numpy(keys.view(np.int64)).cuda(), torch.from_numpy(vals).cuda(), end_bit)
+    bits = min(64, (end_bit + 7) // 8 * 8)                      # whole digits of 8 bits
+    part = keys if bits == 64 else keys & np.uint64(2 ** bits - 1)
+    order = np.argsort(part, kind="stable")
+    assert np.array_equal(vs.cpu().numpy(), vals[order])
+    assert np.array_equal(ks.cpu().numpy().view(np.uint64), keys[order])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [32, 700, 5000, 32_768, 40_001, 65_536, 65_537])
+@pytest.mark.parametrize("far", [0.0, 60.0, 2000.0, 1.0e6])
+def test_morton_sort_with_far_outliers(n, far):
+    """A cloud beside a particle `far` cloud sizes away: the code's cells grow
+    against the cloud, so its top digits tie in short runs, in runs across the
+    blocks of the one-launch sort, and all over; some particles coincide.  The
+    order is the stable order of the 63-bit codes."""
+    rng = np.random.default_rng(n)
+    st = scenarios.empty_state(n)
+    for f in ("posX", "posY", "posZ"):
+        st[f][:] = rng.normal(size=n) * 0.3
+        st[f][n // 2: n // 2 + n // 16] = st[f][n // 2]
+    st["posX"][n - 1] += far
+    st["mass"][:] = 1.0 / n
+    st["h"][:] = st["h0"][:] = 0.02
+    st["rho"][:] = 1.0e-3
+    st["originalId"][:] = np.arange(n, dtype=np.uint32)
+    code = np.zeros(n, np.uint64)
+    for k, f in enumerate(("posX", "posY", "posZ")):
+        lo, hi = st[f].min(), st[f].max()
+        inv = np.float32(2097151.0) / np.float32(hi - lo)
+        q = np.clip((st[f] - lo) * inv, np.float32(0), np.float32(2097151)).astype(np.uint64)
+        for b in range(21):
+            code |= ((q >> np.uint64(b)) & np.uint64(1)) << np.uint64(3 * b + 2 - k)
+    order = np.argsort(code, kind="stable")
+    p, alt, bvh = engine.DeviceParticles(n), engine.DeviceParticles(n), engine.TorchBvh(n)
+    p.upload(st)
+    alt.count = n
+    engine.sort_and_build_bvh(p, alt, bvh)
+    assert np.array_equal(p.download(["originalId"])["originalId"], order)
+    assert np.array_equal(bvh.t["mortonCodesSorted"].cpu().numpy().view(np.uint64), code[order])
+    assert np.array_equal(bvh.t["indicesSorted"].cpu().numpy(), order)
