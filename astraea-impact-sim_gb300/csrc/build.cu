@@ -322,6 +322,15 @@ __device__ __forceinline__ Ext8 extShfl(const Ext8& e, int delta, bool up) {
     return o;
 }
 
+// Square of the distance from a point to the furthest corner of a box, rounded
+// up: a position further from a node's COM than that is outside its box.
+__device__ __forceinline__ float farCorner2(float x, float y, float z, float mnx, float mny, float mnz, float mxx,
+                                            float mxy, float mxz) {
+    const float dx = fmaxf(fabsf(x - mnx), fabsf(mxx - x)), dy = fmaxf(fabsf(y - mny), fabsf(mxy - y)),
+                dz = fmaxf(fabsf(z - mnz), fabsf(mxz - z));
+    return (dx * dx + dy * dy + dz * dz) * 1.00001f;
+}
+
 // Node records from a node's box, h extremes and fixed-point moment sums.
 template <bool kMoments>
 __device__ void writeNode(const AstraeaRadixBvh& bvh, const Work& w, int node, const Ext8& e, const long long* Q,
@@ -362,9 +371,10 @@ __device__ void writeNode(const AstraeaRadixBvh& bvh, const Work& w, int node, c
     const float dNode = fmaxf(e.mxx - e.mnx, fmaxf(e.mxy - e.mny, e.mxz - e.mnz));
     float4* rec = w.node + 4 * static_cast<size_t>(node);
     __stcg(&rec[0], make_float4(cx, cy, cz, mSum));
-    __stcg(&rec[1], make_float4(__fmul_rn(dNode, dNode), __int_as_float(lc), __int_as_float(rc), e.hs));
+    __stcg(&rec[1], make_float4(__fmul_rn(dNode, dNode), __int_as_float(lc), __int_as_float(rc),
+                                farCorner2(cx, cy, cz, e.mnx, e.mny, e.mnz, e.mxx, e.mxy, e.mxz)));
     __stcg(&rec[2], make_float4(e.mnx, e.mny, e.mnz, e.h));
-    __stcg(&rec[3], make_float4(e.mxx, e.mxy, e.mxz, 0.0f));
+    __stcg(&rec[3], make_float4(e.mxx, e.mxy, e.mxz, e.hs));
     if constexpr (kMoments) {
         float s[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (Q[0] > 0) {
@@ -691,7 +701,10 @@ __global__ void __launch_bounds__(256) engineNodeMomentsKernel(AstraeaParticles 
             cy = __fmul_rn(0.5f, __fadd_rn(L.y, R.y));
             cz = __fmul_rn(0.5f, __fadd_rn(L.z, R.z));
         }
-        __stcg(&w.node[4 * static_cast<size_t>(pNode)], make_float4(cx, cy, cz, m));
+        float4* rec = w.node + 4 * static_cast<size_t>(pNode);
+        const float4 mn = __ldcg(&rec[2]), mx = __ldcg(&rec[3]);
+        __stcg(&rec[0], make_float4(cx, cy, cz, m));
+        reinterpret_cast<float*>(&rec[1])[3] = farCorner2(cx, cy, cz, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z);
         if (bvh.aabbMinX != nullptr) {
             bvh.nodeMass[pNode] = m;
             bvh.comX[pNode] = cx; bvh.comY[pNode] = cy; bvh.comZ[pNode] = cz;

@@ -165,7 +165,7 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     auto take = [&](size_t bytes) { const size_t o = off; off += alignUp(bytes); return o; };
     const size_t oLeaf = take(C * 32), oAux = take(C * 16), oRec = take(C * 16 * kRec2Width);
     const size_t nbMax = refitBlocks(static_cast<uint32_t>(C)), levMax = refitLevels(static_cast<uint32_t>(nbMax));
-    const size_t oNode = take(C * 64), oRange = take(C * 8), oLScan = take(C * 64), oMScan = take(C * 80);
+    const size_t oNode = take(C * 64), oPair = take(C * 64), oRange = take(C * 8), oLScan = take(C * 64), oMScan = take(C * 80);
     const size_t oTable = take(levMax * nbMax * 32), oBMom = take(nbMax * 80), oQuad = take(C * 32);
     const size_t oDrift = take(C * 16);
     const size_t oDRec = take(C * 32), oDAux = take(C * 8);
@@ -185,6 +185,7 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     w.leafAux = reinterpret_cast<float4*>(b + oAux);
     w.rec2 = reinterpret_cast<float4*>(b + oRec);
     w.node = reinterpret_cast<float4*>(b + oNode);
+    w.pair = reinterpret_cast<float4*>(b + oPair);
     w.nodeRange = reinterpret_cast<uint2*>(b + oRange);
     w.leafScan = reinterpret_cast<float4*>(b + oLScan);
     w.momScan = reinterpret_cast<long long*>(b + oMScan);

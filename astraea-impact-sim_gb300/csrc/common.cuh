@@ -11,9 +11,10 @@
 //   rec2    [6N]  float4 x6 per particle          pass-2 neighbour record
 //   node    [4(N-1)] float4 x4 per internal node:
 //        r0 {comX, comY, comZ, mass}
-//        r1 {dNode^2 (dNode = largest box side), left (int bits), right (int bits), maxHs}
+//        r1 {dNode^2 (dNode = largest box side), left (int bits), right (int bits), far^2}
+//           far: distance from the COM to the furthest corner of the box, rounded up
 //        r2 {minX, minY, minZ, maxH}             maxH = max 2h (engine field)
-//        r3 {maxX, maxY, maxZ, 0}
+//        r3 {maxX, maxY, maxZ, maxHs}
 //   nodeRange [N-1] uint2 {first, last} sorted leaf range of the node (refit)
 //
 // Search radius: pass 1 (engine/sph_gravity.cu:713) needs r < 2 h_old,
@@ -533,6 +534,7 @@ struct Work {
     float4* leafAux;
     float4* rec2;          // kRec2Width float4 per particle: the pass-2 record
     float4* node;          // 4 x float4 per internal node
+    float4* pair;          // 4 x float4 per internal node: its two children, interleaved (gravity.cu, pairNodesKernel)
     uint2* nodeRange;      // [N-1] {first, last}: the sorted leaf range of each internal node
     float4* leafScan;      // [4N] per leaf: block prefix and block suffix {min xyz, max 2h}, {max xyz, max Hs}
     long long* momScan;    // [10N] per leaf: inclusive block prefix of m, m x (3), m x x^T (6), fixed point

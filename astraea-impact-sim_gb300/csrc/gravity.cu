@@ -8,75 +8,91 @@
 // the node box), otherwise the group descends; leaves are evaluated
 // particle-particle with eps_ij = (eps_i + eps_j)/2, monopoles with eps_i.
 //
-// GB300 restructuring (same sets, different schedule):
-//   * the group walk is node-parallel: up to 32 pending nodes are loaded at
-//     once, one per lane, and decided by three tests of increasing cost:
-//     (1) a sound lower bound on every member's distance to the node's COM
-//     (the larger of the group-box distance and the distance to the group's
-//     26-direction bounding polytope) accepts most far nodes; (2) the exact
-//     test of the member that lies furthest towards the node (looked up per
-//     group for 26 directions) opens most near ones; (3) the few nodes still
-//     undecided are tested by all 32 members at once, two nodes per warp
-//     iteration (f32x2) from a shared-memory list, so no lane loops over the
-//     group;
+// GB300 restructuring (same sets, different schedule).  The kernel is bound by
+// instruction issue (78 % of the issue slots at 262k, DRAM idle), and most
+// instructions are the walk's, so the walk is built to decide a node in few:
+//   * what a walk reads of a node is its two children, side by side in one
+//     64-byte record of its own (pairNodesKernel): one lane opens one node and
+//     has both children's COM, mass, size and reference in two loads, already
+//     in the register pairs of the packed FP32 pipes; a leaf child brings its
+//     particle, so a leaf is never loaded again.  32 opened nodes (64
+//     children) are taken a round, and the stack holds opened nodes only;
+//   * a child is accepted when a sound lower bound on every member's distance
+//     to its COM (the larger of the group-box distance and the distance to the
+//     supporting plane of the group in the octant diagonal the COM lies in)
+//     passes the test, and opened when the exact test of the member that lies
+//     furthest in that diagonal fails; the members and planes of the eight
+//     diagonals are found once a group;
+//   * children neither decides wait in a ring in shared memory; 32 of them at
+//     a time, one a lane, are tested exactly against every member;
 //   * accepted monopoles and reached leaves are appended to two per-warp
 //     interaction lists in shared memory; every 32 entries the warp evaluates
 //     them with each lane summing its own particle's force from broadcast
 //     shared-memory reads, two entries per instruction on the packed FP32
 //     pipes (add/mul/fma.rn.f32x2) plus one rsqrt per pair;
 //   * a persistent grid pulls groups from an atomic counter.
+// 1M impact, theta 0.5, per group of 32: 1,600 opened nodes, 2,940 tested
+// children of which 295 wait for the exact test, 51,254 interactions; warp
+// instructions at 262k 46.1k -> 32.5k a group, of which the evaluation is about
+// half (it runs at the FP32 pipes' rate); launch 1.69 -> 1.34 ms (quadrupole,
+// theta 0.7: 1.63 -> 1.35; 4M Plummer sphere, quadrupole: 9.5 -> 7.9; 60k
+// spheres: 139 -> 110 us), of which the records of the children cost 0.04 ms.
+#include <type_traits>
+
 #include "kernels.h"
 
 namespace astraea_gb300 {
 namespace {
 
 constexpr int kGravWarps = 4;
-constexpr int kGravStack = 768;           // entries per warp (peak use: 274 at 1M, 322 at 16M)
-constexpr int kGravList = 64;
+constexpr int kGravStack = 448;           // opened nodes per warp (peak use: 206 at 1M, 253 on the 1M Plummer sphere)
+// Ring lists: a round appends up to 64 entries behind at most 31 pending ones.
+// The quadrupole's monopole entries are 40 bytes: its list (and mode 3's far
+// list) is emptied between a round's two halves instead.
+constexpr int kGravList = 128, kGravListQ = 64;
+constexpr int kGravCounts = 6;            // interactions, tests, undecided, rounds, group evaluations, bucket leaves
 
-// Interaction lists are stored pair-interleaved so that one 16-byte shared
-// load yields packed (entry 2k, entry 2k+1) operands for the f32x2 pipes:
-// mlist[8k..8k+7] = {xA, xB, yA, yB, zA, zB, -GmA, -GmB}; plist likewise,
-// with peps[2k..2k+1] = {eps_jA / 2, eps_jB / 2}.  With the quadrupole
-// (far-field mode 1) an mlist pair block is 20 floats: the 8 above, then
-// G Q_xx, G Q_yy, G Q_zz, G Q_xy, G Q_xz, G Q_yz of both entries, where
-// Q = 3 S - tr(S) I is the node's traceless quadrupole.  Both lists are
-// rings of 64 entries: a round appends at most 32 behind the pending ones
-// (at most 31), and a flush evaluates the 32 oldest, which start at entry 0
-// or 32 (the head toggles), so no entry is ever moved and the evaluation
-// order is the append order.
-// dirPos[k] (k = 9 (sx + 1) + 3 (sy + 1) + (sz + 1), s in {-1, 0, 1}): the
-// member with the largest projection on the unit direction s / |s| (first
-// member on ties) and, in .w, that projection measured from the group-box
-// centre.  und[] holds the compacted undecided nodes of one walk round; the
-// same storage holds the member positions while dirPos is computed.
-template <bool kInside, bool kQuad, bool kExpand = false>
+// Interaction lists are stored field by field (x, y, z, -G m; with the
+// quadrupole, far-field mode 1, also G Q_xx, G Q_yy, G Q_zz, G Q_xy, G Q_xz,
+// G Q_yz of the traceless Q = 3 S - tr(S) I; particles: x, y, z, -G m, eps / 2),
+// so one 16-byte shared load yields a field of four entries as two packed
+// operands, and an append computes one address.  The lists are rings: a flush
+// evaluates the 32 oldest entries, which start at a multiple of 32 (the head
+// advances by 32), so no entry is ever moved and the evaluation order is the
+// append order.
+// und is the ring of undecided children (2 parent + side in the child
+// records).  memXY / memZ are the members' positions, pair-interleaved
+// ({xA, xB, yA, yB}, {zA, zB}; a short group repeats its first member).
+// dirPos[k] (k = 4 [x < 0] + 2 [y < 0] + [z < 0]): the member with the largest
+// projection on that octant's unit diagonal (first member on ties) and, in
+// .w, that projection measured from the box centre plus the margin of the
+// plane test.
+template <bool kQuad, bool kExpand, bool kLearned>
 struct __align__(16) GravWarpSmem {
     int stack[kGravStack];
-    float mlist[(kQuad ? 20 : 8) * (kGravList / 2)];
-    float plist[8 * (kGravList / 2)];
-    float peps[kGravList];
-    float4 dirPos[27];
-    float4 und[32];                    // {com.x, com.y, com.z, dNode^2}
-    float4 undMin[kInside ? 32 : 1];
-    float4 undMax[kInside ? 32 : 1];
+    float mlist[(kQuad ? 10 * kGravListQ : 4 * kGravList)];
+    float plist[5 * kGravList];
+    uint32_t und[kGravList];
+    unsigned long long counts[kGravCounts];   // the warp's device counters, added up at the end
+    float4 memXY[16];
+    float2 memZ[16];
+    float4 dirPos[8];
+    float4 farDir[kLearned ? 27 : 1];   // mode 2's far test: the extreme members of 26 directions
     // far-field mode 3 only; last, and whole float4s, so the arrays above
     // keep the 16-byte alignment of their vector loads in every variant
-    float4 flist4[kExpand ? 5 * (kGravList / 2) : 1];   // far nodes of the group expansion (mlist layout)
+    float4 flist4[kExpand ? 10 * kGravListQ / 4 : 1];    // far nodes of the group expansion (mlist layout)
     float4 facc4[kExpand ? 5 : 1];                      // the group's expansion coefficients (see farTaylor)
 };
-// the vector loads of the lists (16 bytes) and of peps (8 bytes)
-template <bool kInside, bool kQuad, bool kExpand>
+// the vector loads of the lists and members (16 bytes)
+template <bool kQuad, bool kExpand, bool kLearned>
 constexpr bool gravSmemAligned() {
-    using S = GravWarpSmem<kInside, kQuad, kExpand>;
-    return offsetof(S, mlist) % 16 == 0 && offsetof(S, plist) % 16 == 0 && offsetof(S, peps) % 16 == 0 &&
-           offsetof(S, dirPos) % 16 == 0 && offsetof(S, und) % 16 == 0 && offsetof(S, undMin) % 16 == 0 &&
-           offsetof(S, undMax) % 16 == 0 && offsetof(S, flist4) % 16 == 0 && offsetof(S, facc4) % 16 == 0 &&
-           sizeof(S) % 16 == 0;
+    using S = GravWarpSmem<kQuad, kExpand, kLearned>;
+    return offsetof(S, mlist) % 16 == 0 && offsetof(S, plist) % 16 == 0 && offsetof(S, memXY) % 16 == 0 && offsetof(S, memZ) % 8 == 0 &&
+           offsetof(S, dirPos) % 16 == 0 && offsetof(S, farDir) % 16 == 0 &&
+           offsetof(S, flist4) % 16 == 0 && offsetof(S, facc4) % 16 == 0 && sizeof(S) % 16 == 0;
 }
 static_assert(gravSmemAligned<false, false, false>() && gravSmemAligned<true, false, false>() &&
-              gravSmemAligned<false, true, false>() && gravSmemAligned<true, true, false>() &&
-              gravSmemAligned<false, true, true>() && gravSmemAligned<true, true, true>(),
+              gravSmemAligned<true, true, false>() && gravSmemAligned<false, false, true>(),
               "gravity shared-memory layout must keep 16-byte alignment");
 
 __device__ __forceinline__ uint32_t laneMaskLt() {
@@ -85,70 +101,71 @@ __device__ __forceinline__ uint32_t laneMaskLt() {
     return m;
 }
 
-// The engine's per-member acceptance test (sph_gravity.cu:914-929) with the
-// engine's rounding (len2Engine): dNode^2 < theta^2 r^2, r^2 > 1e-20 and,
-// when checkInside, the member outside the node box.
-__device__ __forceinline__ bool acceptsMember(float px, float py, float pz, float4 com, float dd, float theta2,
-                                              bool checkInside, float4 bmin, float4 bmax) {
-    const float r2 = len2Engine(__fsub_rn(px, com.x), __fsub_rn(py, com.y), __fsub_rn(pz, com.z));
-    bool ok = (dd < __fmul_rn(theta2, r2)) && (r2 > 1.0e-20f);
-    if (ok && checkInside && px >= bmin.x && px <= bmax.x && py >= bmin.y && py <= bmax.y && pz >= bmin.z &&
-        pz <= bmax.z)
-        ok = false;
-    return ok;
+// rsqrtf for arguments that are not subnormal (softened square distances are
+// at least 6.4e-13): the same values without its scaling of subnormals, three
+// instructions more each.
+__device__ __forceinline__ float rsqrtNormal(float v) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
 }
-
 __device__ __forceinline__ f2 rsqrt2(f2 v) {
     float a, b;
     unpack2(v, a, b);
-    return pack2(rsqrtf(a), rsqrtf(b));
+    return pack2(rsqrtNormal(a), rsqrtNormal(b));
 }
 
 struct Accum2 {
     f2 ax, ay, az, phi;   // two partial sums each (even / odd entries)
 };
 
-// Monopole terms: f = -G m / (r^2 + eps_i^2 + 1e-20)^(3/2) (sph_gravity.cu:935-942),
-// two entries per instruction.  `pairs` pairs starting at list pair `first`.
-// E2 = packed eps_i^2 + 1e-20 (eps >= 8e-7, so 1e-20 is below half an ulp of
-// eps^2 and the order of the two additions does not matter).
+// Monopole terms: f = -G m / (r^2 + eps_i^2 + 1e-20)^(3/2) (sph_gravity.cu:935-942)
+// of entries first .. first + count - 1 (a multiple of four) of a list of
+// kRing-entry fields, two entries per instruction.  E2 = packed
+// eps_i^2 + 1e-20 (eps >= 8e-7, so 1e-20 is below half an ulp of eps^2).
 // kQuad adds the quadrupole field of the node, r = x_i - COM, with the same
 // softened 1/r:  a += G [Q r / r^5 - 5/2 (r.Q.r) r / r^7],
 //                phi -= G (r.Q.r) / (2 r^5).
-template <bool kQuad>
-__device__ __forceinline__ void evalMonopoles2(const float* list, int first, int pairs, f2 X, f2 Y, f2 Z, f2 E2,
+template <bool kQuad, int kRing>
+__device__ __forceinline__ void evalMonopoles2(const float* list, int first, int count, f2 X, f2 Y, f2 Z, f2 E2,
                                                Accum2& a) {
-    constexpr int kW = kQuad ? 20 : 8;
     const f2 kHalfNeg = pack2(-0.5f, -0.5f), kFiveHalvesNeg = pack2(-2.5f, -2.5f);
-#pragma unroll 2
-    for (int k = first; k < first + pairs; ++k) {
-        const float* b = list + kW * k;
-        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(b);       // (x), (y)
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(b + 4);   // (z), (-Gm)
-        const f2 dx = sub2(X, u.x), dy = sub2(Y, u.y), dz = sub2(Z, v.x);
-        const f2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-        const f2 inv = rsqrt2(add2(r2, E2));
-        const f2 inv2 = mul2(inv, inv);
-        const f2 inv3 = mul2(inv2, inv);
-        const f2 f = mul2(v.y, inv3);
-        a.ax = fma2(f, dx, a.ax);
-        a.ay = fma2(f, dy, a.ay);
-        a.az = fma2(f, dz, a.az);
-        a.phi = fma2(v.y, inv, a.phi);
+    auto field = [&](int k, int i) { return *reinterpret_cast<const ulonglong2*>(list + kRing * k + i); };
+#pragma unroll 1
+    for (int i = first; i < first + count; i += 4) {
+        const ulonglong2 x = field(0, i), y = field(1, i), z = field(2, i), g = field(3, i);
+        ulonglong2 q[6];
         if constexpr (kQuad) {
-            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(b + 8);    // Qxx, Qyy
-            const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(b + 12);   // Qzz, Qxy
-            const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(b + 16);   // Qxz, Qyz
-            const f2 qr0 = fma2(q2.x, dz, fma2(q1.y, dy, mul2(q0.x, dx)));
-            const f2 qr1 = fma2(q2.y, dz, fma2(q0.y, dy, mul2(q1.y, dx)));
-            const f2 qr2 = fma2(q1.x, dz, fma2(q2.y, dy, mul2(q2.x, dx)));
-            const f2 rqr = fma2(dz, qr2, fma2(dy, qr1, mul2(dx, qr0)));
-            const f2 i5 = mul2(inv3, inv2);
-            const f2 t = mul2(mul2(rqr, mul2(i5, inv2)), kFiveHalvesNeg);
-            a.ax = fma2(t, dx, fma2(qr0, i5, a.ax));
-            a.ay = fma2(t, dy, fma2(qr1, i5, a.ay));
-            a.az = fma2(t, dz, fma2(qr2, i5, a.az));
-            a.phi = fma2(mul2(rqr, i5), kHalfNeg, a.phi);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) q[k] = field(4 + k, i);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            auto half = [&](const ulonglong2& v) { return h == 0 ? v.x : v.y; };
+            const f2 gm = half(g);
+            const f2 dx = sub2(X, half(x)), dy = sub2(Y, half(y)), dz = sub2(Z, half(z));
+            const f2 inv = rsqrt2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2))));
+            const f2 inv2 = mul2(inv, inv);
+            const f2 inv3 = mul2(inv2, inv);
+            const f2 f = mul2(gm, inv3);
+            a.ax = fma2(f, dx, a.ax);
+            a.ay = fma2(f, dy, a.ay);
+            a.az = fma2(f, dz, a.az);
+            a.phi = fma2(gm, inv, a.phi);
+            if constexpr (kQuad) {
+                const f2 xx = half(q[0]), yy = half(q[1]), zz = half(q[2]), xy = half(q[3]), xz = half(q[4]),
+                         yz = half(q[5]);
+                const f2 qr0 = fma2(xz, dz, fma2(xy, dy, mul2(xx, dx)));
+                const f2 qr1 = fma2(yz, dz, fma2(yy, dy, mul2(xy, dx)));
+                const f2 qr2 = fma2(zz, dz, fma2(yz, dy, mul2(xz, dx)));
+                const f2 rqr = fma2(dz, qr2, fma2(dy, qr1, mul2(dx, qr0)));
+                const f2 i5 = mul2(inv3, inv2);
+                const f2 t = mul2(mul2(rqr, mul2(i5, inv2)), kFiveHalvesNeg);
+                a.ax = fma2(t, dx, fma2(qr0, i5, a.ax));
+                a.ay = fma2(t, dy, fma2(qr1, i5, a.ay));
+                a.az = fma2(t, dz, fma2(qr2, i5, a.az));
+                a.phi = fma2(mul2(rqr, i5), kHalfNeg, a.phi);
+            }
         }
     }
 }
@@ -156,43 +173,46 @@ __device__ __forceinline__ void evalMonopoles2(const float* list, int first, int
 // Particle-particle terms with eps_ij = (eps_i + eps_j)/2 (sph_gravity.cu:875-889).
 // The list includes the particle itself; its term adds exactly zero force
 // (dx = dy = dz = 0) and a potential the caller subtracts again.
-__device__ __forceinline__ void evalParticles2(const float* list, const float* peps, int first, int pairs, f2 X,
-                                               f2 Y, f2 Z, f2 HE, Accum2& a) {
-#pragma unroll 2
-    for (int k = first; k < first + pairs; ++k) {
-        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(list + 8 * k);
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(list + 8 * k + 4);
-        const f2 ej = *reinterpret_cast<const f2*>(peps + 2 * k);
-        const f2 dx = sub2(X, u.x), dy = sub2(Y, u.y), dz = sub2(Z, v.x);
-        const f2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-        const f2 eij = add2(HE, ej);
-        const f2 inv = rsqrt2(fma2(eij, eij, r2));
-        const f2 f = mul2(v.y, mul2(inv, mul2(inv, inv)));
-        a.ax = fma2(f, dx, a.ax);
-        a.ay = fma2(f, dy, a.ay);
-        a.az = fma2(f, dz, a.az);
-        a.phi = fma2(v.y, inv, a.phi);
+__device__ __forceinline__ void evalParticles2(const float* list, int first, int count, f2 X, f2 Y, f2 Z, f2 HE,
+                                               Accum2& a) {
+    auto field = [&](int k, int i) { return *reinterpret_cast<const ulonglong2*>(list + kGravList * k + i); };
+#pragma unroll 1
+    for (int i = first; i < first + count; i += 4) {
+        const ulonglong2 x = field(0, i), y = field(1, i), z = field(2, i), g = field(3, i), e = field(4, i);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            auto half = [&](const ulonglong2& v) { return h == 0 ? v.x : v.y; };
+            const f2 gm = half(g);
+            const f2 dx = sub2(X, half(x)), dy = sub2(Y, half(y)), dz = sub2(Z, half(z));
+            const f2 eij = add2(HE, half(e));
+            const f2 inv = rsqrt2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, mul2(eij, eij)))));
+            const f2 f = mul2(gm, mul2(inv, mul2(inv, inv)));
+            a.ax = fma2(f, dx, a.ax);
+            a.ay = fma2(f, dy, a.ay);
+            a.az = fma2(f, dz, a.az);
+            a.phi = fma2(gm, inv, a.phi);
+        }
     }
 }
 
-// Store entry `slot` of a pair-interleaved list.
-__device__ __forceinline__ void putEntry(float* list, int slot, float x, float y, float z, float w) {
-    float* b = list + 8 * (slot >> 1) + (slot & 1);
-    b[0] = x; b[2] = y; b[4] = z; b[6] = w;
+// Store entry `slot` of a particle list.
+__device__ __forceinline__ void putParticle(float* list, int slot, float x, float y, float z, float gm, float halfEps) {
+    float* b = list + slot;
+    b[0] = x; b[kGravList] = y; b[2 * kGravList] = z; b[3 * kGravList] = gm; b[4 * kGravList] = halfEps;
 }
 
-// Monopole entry of the mlist; with kQuad also its six quadrupole terms.
-template <bool kQuad>
+// Monopole entry of a list; with kQuad also its six quadrupole terms.
+template <bool kQuad, int kRing>
 __device__ __forceinline__ void putMono(float* list, int slot, const float (&e)[10]) {
-    float* b = list + (kQuad ? 20 : 8) * (slot >> 1) + (slot & 1);
+    float* b = list + slot;
 #pragma unroll
-    for (int k = 0; k < (kQuad ? 10 : 4); ++k) b[2 * k] = e[k];
+    for (int k = 0; k < (kQuad ? 10 : 4); ++k) b[kRing * k] = e[k];
 }
-template <bool kQuad>
+template <bool kQuad, int kRing>
 __device__ __forceinline__ void getMono(const float* list, int slot, float (&e)[10]) {
-    const float* b = list + (kQuad ? 20 : 8) * (slot >> 1) + (slot & 1);
+    const float* b = list + slot;
 #pragma unroll
-    for (int k = 0; k < (kQuad ? 10 : 4); ++k) e[k] = b[2 * k];
+    for (int k = 0; k < (kQuad ? 10 : 4); ++k) e[k] = b[kRing * k];
 }
 
 // Far-field mode 3: the field of a far node about the group centre c, to
@@ -210,7 +230,7 @@ __device__ __forceinline__ void farTaylor(const float (&e)[10], float cx, float 
                                           float (&t)[20]) {
     const float rx = cx - e[0], ry = cy - e[1], rz = cz - e[2];
     const float s2 = rx * rx + ry * ry + rz * rz + epsG2;
-    const float is = rsqrtf(s2), is2 = is * is, is3 = is * is2, is5 = is3 * is2, is7 = is5 * is2;
+    const float is = rsqrtNormal(s2), is2 = is * is, is3 = is * is2, is5 = is3 * is2, is7 = is5 * is2;
     const float gm = -e[3];                       // e[3] = -G m
     // quadrupole part of phi and a
     const float q0 = e[4] * rx + e[7] * ry + e[8] * rz;
@@ -241,20 +261,97 @@ __device__ __forceinline__ void farTaylor(const float (&e)[10], float cx, float 
 // 1 / |s| for a direction s in {-1, 0, 1}^3 with nz non-zero components.
 __device__ __forceinline__ float invDirNorm(int nz) { return nz == 3 ? 0.57735027f : (nz == 2 ? 0.70710678f : 1.0f); }
 
+// One child: COM, -G m, dNode and index of an internal node; position, -G m,
+// half the softening length and ~j of leaf j (mode 3: the particle count, and
+// whether it is a right child).
+struct Child { float x, y, z, gm, w; int ref; uint32_t cnt = 1u; bool right = false; };
+
+// A node's children (layout: pairNodesKernel) as packed operands.
+struct PairRec { f2 x, y, z, gm, w; int refA, refB; float farA, farB; uint32_t cntA, cntB; };
+template <bool kFar>                     // with the box and count fields
+__device__ __forceinline__ PairRec loadPair(const float4* p) {
+    PairRec r;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.x), "=l"(r.y), "=l"(r.z), "=l"(r.gm) : "l"(p));
+    f2 refs, fars = 0ull, cnts = 0ull;
+    if (kFar)
+        asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.w), "=l"(refs), "=l"(fars), "=l"(cnts) : "l"(p + 2));
+    else
+        asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(r.w), "=l"(refs) : "l"(p + 2));
+    float a, b;
+    unpack2(refs, a, b);
+    r.refA = __float_as_int(a);
+    r.refB = __float_as_int(b);
+    unpack2(fars, r.farA, r.farB);
+    unpack2(cnts, a, b);
+    r.cntA = __float_as_uint(a);
+    r.cntB = __float_as_uint(b);
+    return r;
+}
+
+// The pair record of every internal node p: {xA, xB, yA, yB} {zA, zB, gmA, gmB}
+// {wA, wB, refA, refB} {far^2 A, B, count A, B}, A the left and B the right
+// child: COM, -G m, dNode and the reference of an internal child, position,
+// -G m, half the softening length and ~j of a leaf j; far^2 (furthest corner
+// of the box) and the particle count of an internal child, which for the left
+// child c ends at sorted particle c, for the right child begins there.
+// dNode is the root of the refit's rounded
+// square, so dNode * dNode rounds to that square again.  Written by every
+// gravity call from the node and leaf records it finds.  Bound by the memory
+// system: ~180 bytes read and written a node, most of it still in L2 from the
+// refit; 38 us at 1M, where it saves the gravity walk 350.
+__global__ void __launch_bounds__(256) pairNodesKernel(Work w, uint32_t n) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p + 1u >= n) return;
+    const float4 r1 = __ldg(&w.node[4 * static_cast<size_t>(p) + 1]);
+    float v[2][5], farC[2] = {0.0f, 0.0f};
+    uint32_t cnt[2] = {1u, 1u};
+    int ref[2] = {__float_as_int(r1.y), __float_as_int(r1.z)};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int c = ref[s];
+        if (c >= 0 && c < static_cast<int>(n) - 1) {
+            const float4 a = __ldg(&w.node[4 * static_cast<size_t>(c)]);
+            const float4 b = __ldg(&w.node[4 * static_cast<size_t>(c) + 1]);
+            v[s][0] = a.x; v[s][1] = a.y; v[s][2] = a.z; v[s][3] = -kGPsuF * a.w; v[s][4] = __fsqrt_rn(b.x);
+            farC[s] = b.w;
+            const uint2 r = __ldg(&w.nodeRange[c]);
+            cnt[s] = r.y - r.x + 1u;
+        } else {                                    // a leaf; out of range only in a corrupted tree
+            const uint32_t j = min(static_cast<uint32_t>(~c), n - 1u);
+            const float4 a = __ldg(&w.leaf[j].a);
+            const float4 b = __ldg(&w.leafAux[j]);
+            v[s][0] = a.x; v[s][1] = a.y; v[s][2] = a.z; v[s][3] = -kGPsuF * b.w; v[s][4] = 0.5f * b.y;
+            ref[s] = ~static_cast<int>(j);
+        }
+    }
+    float4* o = w.pair + 4 * static_cast<size_t>(p);
+    o[0] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+    o[1] = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
+    o[2] = make_float4(v[0][4], v[1][4], __int_as_float(ref[0]), __int_as_float(ref[1]));
+    o[3] = make_float4(farC[0], farC[1], __uint_as_float(cnt[0]), __uint_as_float(cnt[1]));
+}
+
 // kDebug: the variant that serves the debugging calls (per-group interaction
 // counts, the trace of one group's accepted nodes and leaves); their checks
 // are kept out of the production variants, where they cost 2 % of the walk.
+// kWarpsPerSm: the resident warps the registers are bounded for (72, 80 and 96
+// registers, no spills).  At 1M, theta 0.5: 28 warps 1.39 ms, 24 1.43, 32 (spills)
+// 1.41; quadrupole, theta 0.7: 24 warps 1.36, 20 1.44; expansion: 20 warps 1.58,
+// 16 1.63, 24 (spills) 1.91.
+template <bool kQuad, bool kExpand>
+constexpr int kWarpsPerSm = kExpand ? 20 : (kQuad ? 24 : 28);
 template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = false, bool kDebug = false>
-__global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p, Work w, uint32_t n,
+__global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWarps) gravityKernel(AstraeaParticles p, Work w, uint32_t n,
                                                                  float theta2, uint32_t numGroups,
                                                                  uint32_t* groupCounter, FarCapture ff) {
     static_assert(!kExpand || kQuad, "the group expansion is a quadrupole mode");
-    __shared__ GravWarpSmem<kInside, kQuad, kExpand> smem[kWarps];
+    constexpr int kMRing = kQuad ? kGravListQ : kGravList;
+    __shared__ GravWarpSmem<kQuad, kExpand, kLearned> smem[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    GravWarpSmem<kInside, kQuad, kExpand>& S = smem[warp];
-    unsigned long long nInter = 0, nTests = 0, nUndecided = 0, nRounds = 0, nGroupEvals = 0, nBucketLeaves = 0;
+    GravWarpSmem<kQuad, kExpand, kLearned>& S = smem[warp];
     int spPeak = 0;
     bool overflowed = false;
+    if (lane < kGravCounts) S.counts[lane] = 0ull;
 
     if (w.runIf != nullptr && *w.runIf == 0u) return;   // the gate of the learned mode passed
     if (n == 1u) {                                   // sph_gravity.cu:824-832
@@ -263,8 +360,7 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
         }
         return;
     }
-    const float4 rootR1 = __ldg(&w.node[1]);
-    const int rootL = __float_as_int(rootR1.y), rootR = __float_as_int(rootR1.z);
+    const float invTheta = 1.0f / sqrtf(theta2);     // theta = 0: infinite, nothing is accepted early
 
     for (;;) {
         uint32_t g = 0;
@@ -274,7 +370,6 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
         const uint32_t i = g * 32u + static_cast<uint32_t>(lane);
         const bool active = i < n;                  // active members are lanes 0 .. act-1
         const int act = static_cast<int>(min(32u, n - g * 32u));
-        const unsigned long long interBefore = nInter;
         float4 me = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float epsI = 0.8e-6f;
         if (active) {
@@ -288,41 +383,75 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
         const float gminx = warpMinF(active ? xi : 3.0e38f), gmaxx = warpMaxF(active ? xi : -3.0e38f);
         const float gminy = warpMinF(active ? yi : 3.0e38f), gmaxy = warpMaxF(active ? yi : -3.0e38f);
         const float gminz = warpMinF(active ? zi : 3.0e38f), gmaxz = warpMaxF(active ? zi : -3.0e38f);
-        const float cxg = 0.5f * (gminx + gmaxx), cyg = 0.5f * (gminy + gmaxy), czg = 0.5f * (gminz + gmaxz);
         const float gExt = (gmaxx - gminx) + (gmaxy - gminy) + (gmaxz - gminz);
+        // c: the box centre; hx, hy, hz: its half sides.  Rounding of the box
+        // term max(|u| - h, 0): relative 1.2e-5 of it at most where |u| is
+        // under a hundred times |u| - h, else under 1.3e-7 of h; the sides
+        // carry 1e-6 of the group's extent and the squared bound 1e-4.
+        const float cx = 0.5f * (gminx + gmaxx), cy = 0.5f * (gminy + gmaxy), cz = 0.5f * (gminz + gmaxz);
+        const float slack = 1.0e-6f * gExt;
+        const float hx = fmaxf(gmaxx - cx, cx - gminx) + slack, hy = fmaxf(gmaxy - cy, cy - gminy) + slack,
+                    hz = fmaxf(gmaxz - cz, cz - gminz) + slack;
+        const f2 CX = pack2(cx, cx), CY = pack2(cy, cy), CZ = pack2(cz, cz);
         const bool emitFar = kLearned && (g % ff.groupStride) == 0u;
-        if (kLearned && lane == 0) ff.groups[g] = make_float4(cxg, cyg, czg, gExt);
+        if (kLearned && lane == 0) ff.groups[g] = make_float4(cx, cy, cz, gExt);
 
-        // Per-direction extreme members (dirPos); member positions staged in und[].
-        S.und[lane] = make_float4(xi, yi, zi, 0.0f);
-        __syncwarp();
-        if (lane < 27) {
+        // Extreme member of each octant diagonal: lanes 4 k .. 4 k + 3 search
+        // diagonal k, every fourth member each.
+        {
+            const int k = lane >> 2;
+            const float sx = (k & 4) ? -1.0f : 1.0f, sy = (k & 2) ? -1.0f : 1.0f, sz = (k & 1) ? -1.0f : 1.0f;
+            float best = -3.0e38f;
+            int bi = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int m = 4 * q + (lane & 3);
+                const float px = __shfl_sync(0xffffffffu, xi, m), py = __shfl_sync(0xffffffffu, yi, m),
+                            pz = __shfl_sync(0xffffffffu, zi, m);
+                const float pr = (sx * (px - cx) + sy * (py - cy) + sz * (pz - cz)) * 0.57735027f;
+                if (m < act && pr > best) { best = pr; bi = m; }
+            }
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+            }
+            const float px = __shfl_sync(0xffffffffu, xi, bi), py = __shfl_sync(0xffffffffu, yi, bi),
+                        pz = __shfl_sync(0xffffffffu, zi, bi);
+            if ((lane & 3) == 0) S.dirPos[k] = make_float4(px, py, pz, best + slack);
+        }
+        {
+            // every lane shuffles (also those that keep their own position)
+            const float fx = __shfl_sync(0xffffffffu, xi, 0), fy = __shfl_sync(0xffffffffu, yi, 0),
+                        fz = __shfl_sync(0xffffffffu, zi, 0);
+            float* xy = reinterpret_cast<float*>(&S.memXY[lane >> 1]) + (lane & 1);
+            xy[0] = active ? xi : fx;
+            xy[2] = active ? yi : fy;
+            reinterpret_cast<float*>(&S.memZ[lane >> 1])[lane & 1] = active ? zi : fz;
+        }
+        if (kLearned) {                          // projections on s / |s|, s in {-1, 0, 1}^3
             const float sx = static_cast<float>(lane / 9 - 1), sy = static_cast<float>((lane / 3) % 3 - 1),
                         sz = static_cast<float>(lane % 3 - 1);
             const float inv = invDirNorm(static_cast<int>(fabsf(sx) + fabsf(sy) + fabsf(sz)));
             float best = -3.0e38f;
-            int bi = 0;
             for (int m = 0; m < act; ++m) {
-                const float4 q = S.und[m];
-                const float pr = (sx * (q.x - cxg) + sy * (q.y - cyg) + sz * (q.z - czg)) * inv;
-                if (pr > best) { best = pr; bi = m; }
+                const float px = __shfl_sync(0xffffffffu, xi, m), py = __shfl_sync(0xffffffffu, yi, m),
+                            pz = __shfl_sync(0xffffffffu, zi, m);
+                best = fmaxf(best, (sx * (px - cx) + sy * (py - cy) + sz * (pz - cz)) * inv);
             }
-            const float4 q = S.und[bi];
-            S.dirPos[lane] = make_float4(q.x, q.y, q.z, best);
+            if (lane < 27) S.farDir[lane] = make_float4(0.0f, 0.0f, 0.0f, best);
         }
-        if (lane == 0) { S.stack[0] = rootL; S.stack[1] = rootR; }
-        int sp = 2, mCount = 0, pCount = 0, fCount = 0;
-        int mHead = 0, pHead = 0;   // first pending entry of each ring list (0 or 32)
-        uint32_t rounds = 0;
-        // group expansion: the group's radius about its box centre c (IEEE
+        if (lane == 0) S.stack[0] = 0;   // the root is opened by every group
+        int sp = 1, mCount = 0, pCount = 0, uCount = 0, fCount = 0;
+        int mHead = 0, pHead = 0, uHead = 0;   // first pending entry of each ring
+        uint32_t rounds = 0, entries = 0, tests = 0, undecidedTests = 0, groupEvals = 0, bucketLeaves = 0;
+        // group expansion: the group's radius about its box centre (IEEE
         // operations, so the far decision is reproducible) and mean eps^2
         float rg2 = 0.0f, epsG2 = 0.0f;
         if (kExpand) {
-            rg2 = warpMaxF(active ? len2Exact(__fsub_rn(xi, cxg), __fsub_rn(yi, cyg), __fsub_rn(zi, czg)) : 0.0f);
-            float e2 = active ? epsI * epsI : 0.0f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-            epsG2 = e2 / static_cast<float>(act);
+            rg2 = warpMaxF(active ? len2Exact(__fsub_rn(xi, cx), __fsub_rn(yi, cy), __fsub_rn(zi, cz)) : 0.0f);
+            epsG2 = warpSumF(active ? epsI * epsI : 0.0f) / static_cast<float>(act);
             if (lane < 20) reinterpret_cast<float*>(S.facc4)[lane] = 0.0f;
         }
         const f2 X = pack2(xi, xi), Y = pack2(yi, yi), Z = pack2(zi, zi);
@@ -337,8 +466,8 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
             float t[20];
             if (lane < cnt) {
                 float e[10];
-                getMono<true>(reinterpret_cast<const float*>(S.flist4), lane, e);
-                farTaylor(e, cxg, cyg, czg, epsG2, t);
+                getMono<true, kGravListQ>(reinterpret_cast<const float*>(S.flist4), lane, e);
+                farTaylor(e, cx, cy, cz, epsG2, t);
             } else {
 #pragma unroll
                 for (int k = 0; k < 20; ++k) t[k] = 0.0f;
@@ -346,213 +475,44 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
             float mine = 0.0f;
 #pragma unroll
             for (int k = 0; k < 20; ++k) {
-                float v = t[k];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                const float v = warpSumF(t[k]);
                 if (lane == k) mine = v;
             }
             if (lane < 20) reinterpret_cast<float*>(S.facc4)[lane] += mine;
             __syncwarp();
         };
         auto flushP = [&]() {                 // evaluate the 32 entries from pHead
-            if (active) evalParticles2(S.plist, S.peps, pHead >> 1, 16, X, Y, Z, HE, acc);
-            nInter += static_cast<unsigned long long>(act) * 32u;
+            if (active) evalParticles2(S.plist, pHead, 32, X, Y, Z, HE, acc);
+            entries += 32u;
             __syncwarp();
             pCount -= 32;
-            pHead ^= 32;
+            pHead = (pHead + 32) & (kGravList - 1);
         };
         __syncwarp();
 
-        while (sp > 0) {
-            if (++rounds > 2u * n + 64u) {     // only reachable on a corrupted tree
-                overflowed = true;
-                break;
-            }
-            spPeak = max(spPeak, sp);
-            const int take = min(sp, 32);
-            const int c = (lane < take) ? S.stack[sp - take + lane] : 0;
-            sp -= take;
+        auto flushM = [&]() {                 // evaluate the 32 entries from mHead
+            if (active) evalMonopoles2<kQuad, kMRing>(S.mlist, mHead, 32, X, Y, Z, E2, acc);
+            entries += 32u;
             __syncwarp();
-            // child references outside [~(n-1), n-2] cannot come from a valid tree
-            const bool has = lane < take && c >= -static_cast<int>(n) && c < static_cast<int>(n) - 1;
-            const bool isLeaf = has && c < 0;
-            const bool isNode = has && c >= 0;
-            bool accept = false;
-            float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            int cl = 0, cr = 0;
-            bool undecided = false;
-            bool farOk = false;
-            float dd = 0.0f;
-            float4 bmin = make_float4(0.f, 0.f, 0.f, 0.f), bmax = bmin;
-            // Without the inside-box rule the tests run on every lane, the
-            // results kept only where isNode (a lane without a node reads the
-            // root's record): as a branch around them the walk was 2.4 % slower
-            // at 1M.  With the rule (theta^2 > 1/3) the branch stays: there the
-            // masked form needs more registers and was slower.
-            if (kInside ? isNode : true) {
-                const int cn = isNode ? c : 0;
-                const float4* rec = w.node + 4 * static_cast<size_t>(cn);
-                r0 = __ldg(&rec[0]);
-                const float4 r1 = __ldg(&rec[1]);
-                cl = __float_as_int(r1.y);
-                cr = __float_as_int(r1.z);
-                dd = r1.x;                       // dNode^2, rounded once by the refit
-                bool disjoint = true;   // the inside-box rule of the theta test (kInside)
-                bool boxApart = true;   // the same rule for the far test (theta_far^2 > 1/3)
-                if (kInside || kLearned) {
-                    bmin = __ldg(&rec[2]);
-                    bmax = __ldg(&rec[3]);
-                    boxApart = bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy ||
-                               bmax.z < gminz || bmin.z > gmaxz;
-                    if (kInside) disjoint = boxApart;
-                }
-                // (1) Sound lower bound on every member's distance to the COM:
-                // the group-box distance, or the distance to the supporting
-                // plane of the group in the direction s of the COM (all
-                // members lie behind it).  Rounding: the box terms are single
-                // subtractions (relative error 2^-24), the plane term carries
-                // an absolute margin of 1e-6 (|u|_1 + group extent), several
-                // times its error bound; 0.99999 covers the final products.
-                const float bx = fmaxf(0.0f, fmaxf(gminx - r0.x, r0.x - gmaxx));
-                const float by = fmaxf(0.0f, fmaxf(gminy - r0.y, r0.y - gmaxy));
-                const float bz = fmaxf(0.0f, fmaxf(gminz - r0.z, r0.z - gmaxz));
-                const float D2 = bx * bx + by * by + bz * bz;
-                const float ux = r0.x - cxg, uy = r0.y - cyg, uz = r0.z - czg;
-                const float ax = fabsf(ux), ay = fabsf(uy), az = fabsf(uz);
-                const float t = 0.41421356f * fmaxf(ax, fmaxf(ay, az));
-                const int sx = (ux >= t) - (ux <= -t), sy = (uy >= t) - (uy <= -t), sz = (uz >= t) - (uz <= -t);
-                const float4 dp = S.dirPos[13 + 9 * sx + 3 * sy + sz];
-                const float inv = invDirNorm(abs(sx) + abs(sy) + abs(sz));
-                const float L = (static_cast<float>(sx) * ux + static_cast<float>(sy) * uy +
-                                 static_cast<float>(sz) * uz) * inv - dp.w - 1.0e-6f * (ax + ay + az + gExt);
-                const float Lb2 = fmaxf(D2, L > 0.0f ? L * L : 0.0f);
-                // far test of mode 2: every member passes theta_far (by the
-                // sound bound) and the node is far against the group's size
-                if (kLearned)
-                    farOk = isNode && emitFar && boxApart && Lb2 > 2.0e-20f && dd < ff.thetaFar2 * Lb2 * 0.99999f &&
-                            gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);
-                // (1) accepts; else (2) the member furthest towards the node
-                // opens it; else (3) the whole group decides below
-                const bool boundAccepts = disjoint && Lb2 > 2.0e-20f && dd < theta2 * Lb2 * 0.99999f;
-                if (kInside) {
-                    if (boundAccepts)
-                        accept = true;
-                    else if (acceptsMember(dp.x, dp.y, dp.z, r0, dd, theta2, kInside, bmin, bmax))
-                        undecided = true;
-                } else {
-                    const bool extremeAccepts = acceptsMember(dp.x, dp.y, dp.z, r0, dd, theta2, kInside, bmin, bmax);
-                    accept = isNode && boundAccepts;
-                    undecided = isNode && !boundAccepts && extremeAccepts;
-                }
-            }
-            // (3) exact test of each undecided node by all members at once
-            const unsigned und = __ballot_sync(0xffffffffu, undecided);
-            if (und) {
-                const int nu = __popc(und);
-                nUndecided += nu;
-                const int slot = __popc(und & laneMaskLt());
-                // pair-interleaved in und's storage: {comxA, comxB, comyA,
-                // comyB, comzA, comzB, ddA, ddB} for undecided nodes 2k, 2k+1
-                float* undP = reinterpret_cast<float*>(S.und);
-                if (undecided) {
-                    float* ub = undP + 8 * (slot >> 1) + (slot & 1);
-                    ub[0] = r0.x; ub[2] = r0.y; ub[4] = r0.z; ub[6] = dd;
-                    if (kInside) { S.undMin[slot] = bmin; S.undMax[slot] = bmax; }
-                }
-                __syncwarp();
-                unsigned bits = 0u;
-                // the engine's member test (acceptsMember) on two nodes per
-                // iteration, rounded as the engine rounds it (len2Engine:
-                // explicit __fmaf_rn / __fmul_rn, which the compiler neither
-                // splits nor re-fuses, so a member on the theta boundary is
-                // decided as the engine decides it)
-                for (int k = 0; k < nu; k += 2) {
-                    const float* ub = undP + 4 * k;
-                    const float4 pa = *reinterpret_cast<const float4*>(ub);       // com xA, xB, yA, yB
-                    const float4 pb = *reinterpret_cast<const float4*>(ub + 4);   // com zA, zB, ddA, ddB
-                    const float r2a = len2Engine(__fsub_rn(xi, pa.x), __fsub_rn(yi, pa.z), __fsub_rn(zi, pb.x));
-                    const float r2b = len2Engine(__fsub_rn(xi, pa.y), __fsub_rn(yi, pa.w), __fsub_rn(zi, pb.y));
-                    const float ta = __fmul_rn(theta2, r2a), tb = __fmul_rn(theta2, r2b);
-                    const float dda = pb.z, ddb = pb.w;
-                    bool okA = dda < ta && r2a > 1.0e-20f, okB = ddb < tb && r2b > 1.0e-20f;
-                    if (kInside) {
-                        const float4 mnA = S.undMin[k], mxA = S.undMax[k];
-                        const float4 mnB = S.undMin[k + 1], mxB = S.undMax[k + 1];
-                        if (okA && xi >= mnA.x && xi <= mxA.x && yi >= mnA.y && yi <= mxA.y && zi >= mnA.z &&
-                            zi <= mxA.z)
-                            okA = false;
-                        if (okB && xi >= mnB.x && xi <= mxB.x && yi >= mnB.y && yi <= mxB.y && zi >= mnB.z &&
-                            zi <= mxB.z)
-                            okB = false;
-                    }
-                    bits |= (__all_sync(0xffffffffu, !active || okA) ? 1u : 0u) << k;
-                    if (k + 1 < nu) bits |= (__all_sync(0xffffffffu, !active || okB) ? 1u : 0u) << (k + 1);
-                }
-                if (undecided) accept = (bits >> slot) & 1u;
-                __syncwarp();
-            }
-            if (kLearned) {
-                // a node the theta test opens but the far test takes: a
-                // monopole plus the learned correction of this (group, node)
-                bool far = isNode && !accept && farOk;
-                const unsigned farMask = __ballot_sync(0xffffffffu, far);
-                if (farMask) {
-                    uint32_t fb = 0;
-                    if (lane == 0) fb = atomicAdd(ff.count, static_cast<uint32_t>(__popc(farMask)));
-                    fb = __shfl_sync(0xffffffffu, fb, 0);
-                    if (far) {
-                        const uint32_t slot = fb + static_cast<uint32_t>(__popc(farMask & laneMaskLt()));
-                        if (slot < ff.cap) {                     // full buffer: the node is opened
-                            ff.pairs[slot] = make_uint2(g, static_cast<uint32_t>(c));
-                            accept = true;
-                        }
-                    }
-                }
-            }
-            bool open = isNode && !accept;
-            // mode 3: an opened node of at most leafBucket particles is not
-            // descended; its sorted leaf range is evaluated particle-particle
-            uint2 brng = make_uint2(1u, 0u);
-            if (kExpand && open && w.leafBucket > 0u) {
-                const uint2 r = __ldg(&w.nodeRange[c]);
-                if (r.x <= r.y && r.y < n && r.y - r.x < w.leafBucket) {
-                    brng = r;
-                    open = false;
-                }
-            }
-            unsigned openMask = __ballot_sync(0xffffffffu, open);
-            if (sp + 2 * __popc(openMask) > kGravStack) {
-                // Out of stack: the group takes these nodes as monopoles, the
-                // rule of the engine kernel when its stack is full (:933).
-                if (open) { open = false; accept = true; }
-                openMask = 0u;
-                overflowed = true;
-            }
-            if (open) {
-                const int pos = sp + 2 * __popc(openMask & laneMaskLt());
-                S.stack[pos] = cl;
-                S.stack[pos + 1] = cr;
-            }
-            sp += 2 * __popc(openMask);
-            // mode 3: an accepted node far against the group (group radius <=
-            // gamma |c - COM|) joins the group's expansion instead of being
-            // evaluated by every member
+            mCount -= 32;
+            mHead = (mHead + 32) & (kMRing - 1);
+        };
+        // An accepted node of each lane that has one, into the monopole list
+        // (mode 3: or into the group's expansion, where the node is far against
+        // the group: group radius <= gamma |c - COM|).
+        auto putAccepted = [&](bool accept, const Child& c) {
             bool far = false;
             if (kExpand && accept) {
-                const float R2 = len2Exact(__fsub_rn(cxg, r0.x), __fsub_rn(cyg, r0.y), __fsub_rn(czg, r0.z));
+                const float R2 = len2Exact(__fsub_rn(cx, c.x), __fsub_rn(cy, c.y), __fsub_rn(cz, c.z));
                 far = rg2 <= __fmul_rn(w.expandGamma2, R2);
             }
             const unsigned accMask = __ballot_sync(0xffffffffu, accept && !far);
             const unsigned farMask = kExpand ? __ballot_sync(0xffffffffu, far) : 0u;
-            if (kDebug && w.traceList != nullptr && g == w.traceGroup && (accept || isLeaf)) {
-                const uint32_t k = atomicAdd(reinterpret_cast<uint32_t*>(w.traceList), 1u);
-                if (k < w.traceCap) w.traceList[1 + k] = c;
-            }
             if (accept) {
-                float e[10] = {r0.x, r0.y, r0.z, -kGPsuF * r0.w, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                float e[10] = {c.x, c.y, c.z, c.gm, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 if (kQuad) {
-                    const float4 s0 = __ldg(&w.nodeQuad[2 * static_cast<size_t>(c)]);      // Sxx Syy Szz Sxy
-                    const float4 s1 = __ldg(&w.nodeQuad[2 * static_cast<size_t>(c) + 1]);  // Sxz Syz
+                    const float4 s0 = __ldg(&w.nodeQuad[2 * static_cast<size_t>(c.ref)]);      // Sxx Syy Szz Sxy
+                    const float4 s1 = __ldg(&w.nodeQuad[2 * static_cast<size_t>(c.ref) + 1]);  // Sxz Syz
                     const float tr = s0.x + s0.y + s0.z;
                     e[4] = kGPsuF * (3.0f * s0.x - tr);
                     e[5] = kGPsuF * (3.0f * s0.y - tr);
@@ -561,101 +521,329 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
                     e[8] = kGPsuF * 3.0f * s1.x;
                     e[9] = kGPsuF * 3.0f * s1.y;
                 }
+                const int slot = (mHead + mCount + __popc(accMask & laneMaskLt())) & (kMRing - 1);
                 if constexpr (kExpand) {
                     if (far)
-                        putMono<true>(reinterpret_cast<float*>(S.flist4), fCount + __popc(farMask & laneMaskLt()), e);
+                        putMono<true, kGravListQ>(reinterpret_cast<float*>(S.flist4), fCount + __popc(farMask & laneMaskLt()), e);
                     else
-                        putMono<kQuad>(S.mlist, (mHead + mCount + __popc(accMask & laneMaskLt())) & 63, e);
+                        putMono<kQuad, kMRing>(S.mlist, slot, e);
                 } else {
-                    putMono<kQuad>(S.mlist, (mHead + mCount + __popc(accMask & laneMaskLt())) & 63, e);
+                    putMono<kQuad, kMRing>(S.mlist, slot, e);
                 }
             }
             mCount += __popc(accMask);
             if (kExpand) {
                 fCount += __popc(farMask);
-                nGroupEvals += __popc(farMask);
+                groupEvals += static_cast<uint32_t>(__popc(farMask));
                 __syncwarp();
                 if (fCount >= 32) {
                     flushFar(32);
                     fCount -= 32;
                     if (lane < fCount) {
                         float e2[10];
-                        getMono<true>(reinterpret_cast<const float*>(S.flist4), 32 + lane, e2);
-                        putMono<true>(reinterpret_cast<float*>(S.flist4), lane, e2);
+                        getMono<true, kGravListQ>(reinterpret_cast<const float*>(S.flist4), 32 + lane, e2);
+                        putMono<true, kGravListQ>(reinterpret_cast<float*>(S.flist4), lane, e2);
                     }
                     __syncwarp();
                 }
             }
-            const unsigned leafMask = __ballot_sync(0xffffffffu, isLeaf);
-            unsigned selfBit = 0u;
-            if (isLeaf) {
-                const int j = ~c;
-                const float4 pa = __ldg(&w.leaf[j].a);
-                const float4 aux = __ldg(&w.leafAux[j]);
-                const float4 pm = make_float4(pa.x, pa.y, pa.z, aux.w);
-                const float ej = aux.y;
-                const int slot = (pHead + pCount + __popc(leafMask & laneMaskLt())) & 63;
-                putEntry(S.plist, slot, pm.x, pm.y, pm.z, -kGPsuF * pm.w);
-                S.peps[slot] = 0.5f * ej;
-                const uint32_t rel = static_cast<uint32_t>(j) - base;
-                if (rel < 32u) selfBit = 1u << rel;
-            }
-            selfSeen |= __reduce_or_sync(0xffffffffu, selfBit);
-            pCount += __popc(leafMask);
-            nTests += __popc(__ballot_sync(0xffffffffu, isNode));
-            __syncwarp();
-            if (mCount >= 32) {                 // evaluate the 32 entries from mHead
-                if (active) evalMonopoles2<kQuad>(S.mlist, mHead >> 1, 16, X, Y, Z, E2, acc);
-                nInter += static_cast<unsigned long long>(act) * 32u;
+            if (kQuad) {
                 __syncwarp();
-                mCount -= 32;
-                mHead ^= 32;
+                if (mCount >= 32) flushM();
             }
-            if (pCount >= 32) flushP();
-            if (kExpand) {
-                // leaf buckets of this round: each range (at most 32 sorted
-                // particles) appended to the particle list by the warp at once
-                unsigned bucketMask = __ballot_sync(0xffffffffu, brng.x <= brng.y);
-                while (bucketMask) {
-                    const int src = __ffs(bucketMask) - 1;
-                    bucketMask &= bucketMask - 1u;
-                    const uint32_t first = __shfl_sync(0xffffffffu, brng.x, src);
-                    const uint32_t last = __shfl_sync(0xffffffffu, brng.y, src);
-                    const uint32_t j = first + static_cast<uint32_t>(lane);
-                    const bool has = j <= last;
-                    const unsigned hm = __ballot_sync(0xffffffffu, has);
-                    unsigned sb = 0u;
-                    if (has) {
-                        const float4 pm = __ldg(&w.leaf[j].a);
-                        const float4 aux = __ldg(&w.leafAux[j]);
-                        const int slot = (pHead + pCount + __popc(hm & laneMaskLt())) & 63;
-                        putEntry(S.plist, slot, pm.x, pm.y, pm.z, -kGPsuF * aux.w);
-                        S.peps[slot] = 0.5f * aux.y;
-                        const uint32_t rel = j - base;
-                        if (rel < 32u) sb = 1u << rel;
-                    }
-                    const unsigned selfHere = __reduce_or_sync(0xffffffffu, sb);
-                    selfSeen |= selfHere;
-                    pCount += __popc(hm);
-                    nBucketLeaves += static_cast<unsigned long long>(act) * __popc(hm) - __popc(selfHere);
-                    __syncwarp();
-                    if (pCount >= 32) flushP();
+        };
+        // mode 3: an opened node of at most leafBucket particles is not
+        // descended; its sorted leaf range is evaluated particle-particle
+        auto bucketOf = [&](bool& open, const Child& c) {
+            uint2 brng = make_uint2(1u, 0u);
+            if (kExpand && open && c.cnt <= w.leafBucket) {
+                const uint32_t first = static_cast<uint32_t>(c.ref) - (c.right ? 0u : c.cnt - 1u);
+                if (c.cnt - 1u < 32u && first < n && n - first >= c.cnt) {   // always, for a valid tree
+                    brng = make_uint2(first, first + c.cnt - 1u);
+                    open = false;
                 }
             }
+            return brng;
+        };
+        auto putBuckets = [&](uint2 brng) {   // each range (at most 32 sorted particles) by the warp at once
+            unsigned bucketMask = __ballot_sync(0xffffffffu, brng.x <= brng.y);
+            while (bucketMask) {
+                const int src = __ffs(bucketMask) - 1;
+                bucketMask &= bucketMask - 1u;
+                const uint32_t first = __shfl_sync(0xffffffffu, brng.x, src);
+                const uint32_t last = __shfl_sync(0xffffffffu, brng.y, src);
+                const uint32_t j = first + static_cast<uint32_t>(lane);
+                const bool has = j <= last;
+                const unsigned hm = __ballot_sync(0xffffffffu, has);
+                unsigned sb = 0u;
+                if (has) {
+                    const float4 pm = __ldg(&w.leaf[j].a);
+                    const float4 aux = __ldg(&w.leafAux[j]);
+                    const int slot = (pHead + pCount + __popc(hm & laneMaskLt())) & (kGravList - 1);
+                    putParticle(S.plist, slot, pm.x, pm.y, pm.z, -kGPsuF * aux.w, 0.5f * aux.y);
+                    const uint32_t rel = j - base;
+                    if (rel < 32u) sb = 1u << rel;
+                }
+                const unsigned selfHere = __reduce_or_sync(0xffffffffu, sb);
+                selfSeen |= selfHere;
+                pCount += __popc(hm);
+                bucketLeaves += static_cast<uint32_t>(act * __popc(hm) - __popc(selfHere));
+                __syncwarp();
+                if (pCount >= 32) flushP();
+            }
+        };
+        // Puts the decided nodes among up to two children a lane (kTwo) where
+        // they belong: opened ones on the stack, accepted ones into the lists.
+        auto place = [&](auto two, bool openA, bool accA, const Child& A, bool openB, bool accB, const Child& B) {
+            constexpr bool kTwo = decltype(two)::value;
+            const uint2 brA = bucketOf(openA, A), brB = kTwo ? bucketOf(openB, B) : make_uint2(1u, 0u);
+            unsigned mA = __ballot_sync(0xffffffffu, openA), mB = kTwo ? __ballot_sync(0xffffffffu, openB) : 0u;
+            if (sp + __popc(mA) + __popc(mB) > kGravStack) {
+                // Out of stack: the group takes these nodes as monopoles, the
+                // rule of the engine kernel when its stack is full (:933).
+                accA = accA || openA;
+                accB = accB || openB;
+                openA = openB = false;
+                mA = mB = 0u;
+                overflowed = true;
+            }
+            if (openA) S.stack[sp + __popc(mA & laneMaskLt())] = A.ref;
+            sp += __popc(mA);
+            if (kTwo && openB) S.stack[sp + __popc(mB & laneMaskLt())] = B.ref;
+            sp += __popc(mB);
+            if (kDebug && w.traceList != nullptr && g == w.traceGroup && (accA || accB)) {
+                const uint32_t k = atomicAdd(reinterpret_cast<uint32_t*>(w.traceList), (accA ? 1u : 0u) + (accB ? 1u : 0u));
+                if (accA && k < w.traceCap) w.traceList[1 + k] = A.ref;
+                const uint32_t k2 = k + (accA ? 1u : 0u);
+                if (accB && k2 < w.traceCap) w.traceList[1 + k2] = B.ref;
+            }
+            putAccepted(accA, A);
+            if (kTwo) putAccepted(accB, B);
+            __syncwarp();
+            if (!kQuad)
+                while (mCount >= 32) flushM();
+            if (kExpand) {
+                putBuckets(brA);
+                if (kTwo) putBuckets(brB);
+            }
+        };
+        // The cheap tests of one child (u = COM - c): accepted by the bound,
+        // opened by the extreme member, or left undecided.
+        auto decide = [&](bool isNode, float x, float y, float z, float dd, float ux, float uy, float uz, int ref,
+                          float far2, bool& accept, bool& open, bool& undecided) {
+            const float ax = fabsf(ux), ay = fabsf(uy), az = fabsf(uz);
+            const float bx = fmaxf(ax - hx, 0.0f), by = fmaxf(ay - hy, 0.0f), bz = fmaxf(az - hz, 0.0f);
+            const float D2 = bx * bx + by * by + bz * bz;
+            const float4 dp = S.dirPos[((__float_as_uint(ux) >> 29) & 4u) | ((__float_as_uint(uy) >> 30) & 2u) |
+                                       (__float_as_uint(uz) >> 31)];
+            // distance to the octant's supporting plane, |u|_1 with its 1e-6 margin
+            const float L = (ax + ay + az) * (0.57735027f - 1.0e-6f) - dp.w;
+            const float Lb2 = fmaxf(D2, L * fabsf(L)) * 0.9999f;
+            const float r2 = len2Engine(__fsub_rn(dp.x, x), __fsub_rn(dp.y, y), __fsub_rn(dp.z, z));
+            bool boundAccepts = Lb2 > 2.0e-20f && dd < theta2 * Lb2;
+            bool extreme = dd < __fmul_rn(theta2, r2) && r2 > 1.0e-20f;     // the engine's test, without its box
+            bool boxApart = true;               // no member can lie in the node's box
+            if (kInside || kLearned) {
+                // the box is only looked at where a member may be as near the
+                // COM as its furthest corner
+                if (isNode && (kLearned || ((boundAccepts || extreme) && !(Lb2 > far2)))) {
+                    const float4 bmin = __ldg(&w.node[4 * static_cast<size_t>(ref) + 2]);
+                    const float4 bmax = __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]);
+                    boxApart = bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy || bmax.z < gminz ||
+                               bmin.z > gmaxz;
+                    if (kInside) {
+                        boundAccepts = boundAccepts && boxApart;
+                        if (dp.x >= bmin.x && dp.x <= bmax.x && dp.y >= bmin.y && dp.y <= bmax.y && dp.z >= bmin.z &&
+                            dp.z <= bmax.z)
+                            extreme = false;
+                    }
+                }
+            }
+            accept = isNode && boundAccepts;
+            undecided = isNode && !boundAccepts && extreme;
+            open = isNode && !boundAccepts && !extreme;
+            if (kLearned) {
+                // far test of mode 2 on the nodes the theta test may open: every
+                // member passes theta_far (by a sound bound: the box distance or
+                // the supporting plane of the nearest of 26 directions) and the
+                // node is far against the group's size.  Such a node is decided here: a
+                // monopole plus the learned correction of this (group, node),
+                // unless every member accepts it anyway.
+                const float gx = fmaxf(0.0f, fmaxf(gminx - x, x - gmaxx)), gy = fmaxf(0.0f, fmaxf(gminy - y, y - gmaxy)),
+                            gz = fmaxf(0.0f, fmaxf(gminz - z, z - gmaxz));
+                const float t = 0.41421356f * fmaxf(ax, fmaxf(ay, az));
+                const int sx = (ux >= t) - (ux <= -t), sy = (uy >= t) - (uy <= -t), sz = (uz >= t) - (uz <= -t);
+                const float Lf = (static_cast<float>(sx) * ux + static_cast<float>(sy) * uy + static_cast<float>(sz) * uz) *
+                                     invDirNorm(abs(sx) + abs(sy) + abs(sz)) -
+                                 S.farDir[13 + 9 * sx + 3 * sy + sz].w - 1.0e-6f * (ax + ay + az + gExt);
+                const float Fb2 = fmaxf(gx * gx + gy * gy + gz * gz, Lf > 0.0f ? Lf * Lf : 0.0f);
+                const bool farOk = !accept && isNode && emitFar && boxApart && Fb2 > 2.0e-20f &&
+                                   dd < ff.thetaFar2 * Fb2 * 0.99999f &&
+                                   gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);
+                unsigned todo = __ballot_sync(0xffffffffu, farOk);
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const float qx = __shfl_sync(0xffffffffu, x, src), qy = __shfl_sync(0xffffffffu, y, src),
+                                qz = __shfl_sync(0xffffffffu, z, src), qd = __shfl_sync(0xffffffffu, dd, src);
+                    const float m2 = len2Engine(__fsub_rn(xi, qx), __fsub_rn(yi, qy), __fsub_rn(zi, qz));
+                    // boxApart holds for it: no member is inside its box
+                    const bool all = __all_sync(0xffffffffu, !active || (qd < __fmul_rn(theta2, m2) && m2 > 1.0e-20f));
+                    uint32_t slot = 0xffffffffu;
+                    if (!all && lane == src) {
+                        slot = atomicAdd(ff.count, 1u);
+                        if (slot < ff.cap) ff.pairs[slot] = make_uint2(g, static_cast<uint32_t>(ref));
+                    }
+                    if (lane == src) {
+                        accept = all || slot < ff.cap;       // full buffer: the node is opened
+                        open = !accept;
+                        undecided = false;
+                    }
+                }
+            }
+        };
+        while (sp > 0 || uCount > 0) {
+            if (++rounds > 4u * n + 64u) {     // only reachable on a corrupted tree
+                overflowed = true;
+                break;
+            }
+            if (uCount >= 32 || sp == 0) {
+                // The oldest undecided children, up to 32, one a lane, against every
+                // member: the engine's member test (sph_gravity.cu:914-929) with
+                // the engine's rounding of r^2 (len2Engine's operations, packed).
+                // fl(theta^2 r^2) grows with r^2, so all members accept when the
+                // smallest r^2 does.
+                const int take = min(uCount, 32);
+                const bool has = lane < take;
+                undecidedTests += static_cast<uint32_t>(take);
+                Child c;
+                float far2 = 0.0f;
+                {
+                    const uint32_t id = has ? S.und[uHead + lane] : 0u;
+                    const float* r = reinterpret_cast<const float*>(w.pair + 4 * static_cast<size_t>(id >> 1)) + (id & 1u);
+                    c.x = __ldg(r); c.y = __ldg(r + 2); c.z = __ldg(r + 4); c.gm = __ldg(r + 6); c.w = __ldg(r + 8);
+                    c.ref = __float_as_int(__ldg(r + 10));
+                    if (kInside) far2 = __ldg(r + 12);
+                    if (kExpand) c.cnt = __float_as_uint(__ldg(r + 14));
+                    c.right = (id & 1u) != 0u;
+                }
+                uCount -= take;
+                uHead = (uHead + 32) & (kGravList - 1);   // take < 32 empties the ring: any head will do
+                const f2 NX = pack2(c.x, c.x), NY = pack2(c.y, c.y), NZ = pack2(c.z, c.z);
+                float rmin = 3.4e38f;
+#pragma unroll 4
+                for (int k = 0; k < 16; ++k) {
+                    const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(&S.memXY[k]);
+                    const f2 dx = sub2(xy.x, NX), dy = sub2(xy.y, NY),
+                             dz = sub2(*reinterpret_cast<const f2*>(&S.memZ[k]), NZ);
+                    float ra, rb;
+                    unpack2(fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))), ra, rb);
+                    rmin = fminf(rmin, fminf(ra, rb));
+                }
+                bool all = __fmul_rn(c.w, c.w) < __fmul_rn(theta2, rmin) && rmin > 1.0e-20f;
+                if (kInside) {                  // nor may a member lie in the node's box
+                    float4 bmin = make_float4(0.f, 0.f, 0.f, 0.f), bmax = bmin;
+                    bool near = has && all && rmin <= far2;
+                    if (near) {
+                        bmin = __ldg(&w.node[4 * static_cast<size_t>(c.ref) + 2]);
+                        bmax = __ldg(&w.node[4 * static_cast<size_t>(c.ref) + 3]);
+                        near = !(bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy ||
+                                 bmax.z < gminz || bmin.z > gmaxz);
+                    }
+                    if (__any_sync(0xffffffffu, near)) {
+                        for (int k = 0; k < 16; ++k) {
+                            const float4 xy = S.memXY[k];
+                            const float2 zz = S.memZ[k];
+                            if (near && ((xy.x >= bmin.x && xy.x <= bmax.x && xy.z >= bmin.y && xy.z <= bmax.y &&
+                                          zz.x >= bmin.z && zz.x <= bmax.z) ||
+                                         (xy.y >= bmin.x && xy.y <= bmax.x && xy.w >= bmin.y && xy.w <= bmax.y &&
+                                          zz.y >= bmin.z && zz.y <= bmax.z)))
+                                all = false;
+                        }
+                    }
+                }
+                place(std::false_type{}, has && !all, has && all, c, false, false, c);
+                continue;
+            }
+            // open up to 32 nodes: both children of each
+            spPeak = max(spPeak, sp);
+            const int take = min(sp, 32);
+            sp -= take;
+            int node = (lane < take) ? S.stack[sp + lane] : 0;
+            __syncwarp();
+            // indices outside [0, n-2] cannot come from a valid tree
+            const bool has = lane < take && static_cast<uint32_t>(node) < n - 1u;
+            node = has ? node : 0;
+            const PairRec rec = loadPair<kInside || kExpand>(w.pair + 4 * static_cast<size_t>(node));
+            const f2 du = sub2(rec.x, CX), dv = sub2(rec.y, CY), dw = sub2(rec.z, CZ), dd = mul2(rec.w, rec.w);
+            tests += 2u * static_cast<uint32_t>(take);
+            Child A, B;
+            unpack2(rec.x, A.x, B.x);
+            unpack2(rec.y, A.y, B.y);
+            unpack2(rec.z, A.z, B.z);
+            unpack2(rec.gm, A.gm, B.gm);
+            unpack2(rec.w, A.w, B.w);
+            A.ref = rec.refA;
+            B.ref = rec.refB;
+            A.cnt = rec.cntA;
+            B.cnt = rec.cntB;
+            A.right = false;
+            B.right = true;
+            float uxA, uxB, uyA, uyB, uzA, uzB, ddA, ddB;
+            unpack2(du, uxA, uxB);
+            unpack2(dv, uyA, uyB);
+            unpack2(dw, uzA, uzB);
+            unpack2(dd, ddA, ddB);
+            bool accA, openA, undA, accB, openB, undB;
+            decide(has && A.ref >= 0, A.x, A.y, A.z, ddA, uxA, uyA, uzA, A.ref, rec.farA, accA, openA, undA);
+            decide(has && B.ref >= 0, B.x, B.y, B.z, ddB, uxB, uyB, uzB, B.ref, rec.farB, accB, openB, undB);
+            // undecided children of both sides
+            const unsigned uA = __ballot_sync(0xffffffffu, undA), uB = __ballot_sync(0xffffffffu, undB);
+            if (uA | uB) {
+                const int s0 = uHead + uCount + __popc(uA & laneMaskLt());
+                if (undA) S.und[s0 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node);
+                const int s1 = uHead + uCount + __popc(uA) + __popc(uB & laneMaskLt());
+                if (undB) S.und[s1 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node) + 1u;
+                uCount += __popc(uA) + __popc(uB);
+            }
+            // leaves of both sides
+            const bool leafA = has && A.ref < 0, leafB = has && B.ref < 0;
+            const unsigned lA = __ballot_sync(0xffffffffu, leafA), lB = __ballot_sync(0xffffffffu, leafB);
+            if (lA | lB) {
+                unsigned selfBit = 0u;
+                auto putLeaf = [&](const Child& c, int slot) {
+                    putParticle(S.plist, slot, c.x, c.y, c.z, c.gm, c.w);
+                    const uint32_t rel = static_cast<uint32_t>(~c.ref) - base;
+                    if (rel < 32u) selfBit |= 1u << rel;
+                    if (kDebug && w.traceList != nullptr && g == w.traceGroup) {
+                        const uint32_t k = atomicAdd(reinterpret_cast<uint32_t*>(w.traceList), 1u);
+                        if (k < w.traceCap) w.traceList[1 + k] = c.ref;
+                    }
+                };
+                if (leafA) putLeaf(A, (pHead + pCount + __popc(lA & laneMaskLt())) & (kGravList - 1));
+                if (leafB) putLeaf(B, (pHead + pCount + __popc(lA) + __popc(lB & laneMaskLt())) & (kGravList - 1));
+                selfSeen |= __reduce_or_sync(0xffffffffu, selfBit);
+                const int cnt = __popc(lA) + __popc(lB);
+                pCount += cnt;
+                tests -= static_cast<uint32_t>(cnt);
+                __syncwarp();
+                while (pCount >= 32) flushP();
+            }
+            place(std::true_type{}, openA, accA, A, openB, accB, B);
         }
         if (kExpand && fCount > 0) flushFar(fCount);
-        // odd tails: pad with a massless entry (adds exactly zero)
-        if (lane == 0) {
-            if (mCount & 1) {
+        // tails: pad to fours with massless entries (they add exactly zero)
+        if (lane < 3) {
+            if (lane < ((4 - mCount) & 3)) {
                 const float zero[10] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                putMono<kQuad>(S.mlist, mHead + mCount, zero);
+                putMono<kQuad, kMRing>(S.mlist, mHead + mCount + lane, zero);
             }
-            if (pCount & 1) { putEntry(S.plist, pHead + pCount, 0.0f, 0.0f, 0.0f, 0.0f); S.peps[pHead + pCount] = 0.0f; }
+            if (lane < ((4 - pCount) & 3)) putParticle(S.plist, pHead + pCount + lane, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f);
         }
         __syncwarp();
         if (active) {
-            evalMonopoles2<kQuad>(S.mlist, mHead >> 1, (mCount + 1) >> 1, X, Y, Z, E2, acc);
-            evalParticles2(S.plist, S.peps, pHead >> 1, (pCount + 1) >> 1, X, Y, Z, HE, acc);
+            evalMonopoles2<kQuad, kMRing>(S.mlist, mHead, (mCount + 3) & ~3, X, Y, Z, E2, acc);
+            evalParticles2(S.plist, pHead, (pCount + 3) & ~3, X, Y, Z, HE, acc);
             float a0, a1, b0, b1, c0, c1, d0, d1;
             unpack2(acc.ax, a0, a1);
             unpack2(acc.ay, b0, b1);
@@ -664,12 +852,12 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
             float phi = d0 + d1;
             if (selfSeen & (1u << lane)) {
                 // the self term added to phi: -G m_i / sqrt(eps_i^2), exactly as evaluated
-                phi -= (-kGPsuF * me.w) * rsqrtf(__fmul_rn(epsI, epsI));
+                phi -= (-kGPsuF * me.w) * rsqrtNormal(__fmul_rn(epsI, epsI));
             }
             float ax = a0 + a1, ay = b0 + b1, az = c0 + c1;
             if (kExpand) {                     // the group's far field at this member (farTaylor)
                 const float* t = reinterpret_cast<const float*>(S.facc4);
-                const float dx = xi - cxg, dy = yi - cyg, dz = zi - czg;
+                const float dx = xi - cx, dy = yi - cy, dz = zi - cz;
                 const float jx = t[4] * dx + t[7] * dy + t[8] * dz;      // J d
                 const float jy = t[7] * dx + t[5] * dy + t[9] * dz;
                 const float jz = t[8] * dx + t[9] * dy + t[6] * dz;
@@ -687,24 +875,32 @@ __global__ void __launch_bounds__(kWarps * 32) gravityKernel(AstraeaParticles p,
             p.accZ[i] = az;
             p.phiGrav[i] = phi;
         }
-        nRounds += rounds;
-        nInter += static_cast<unsigned long long>(act) * static_cast<unsigned>(mCount + pCount);
         if (lane == 0) {
-            nInter -= static_cast<unsigned long long>(__popc(selfSeen));
-            if (kDebug && w.groupCounts != nullptr) w.groupCounts[g] = static_cast<uint32_t>(nInter - interBefore);
+            const unsigned long long inter = static_cast<unsigned long long>(act) *
+                                                 (entries + static_cast<unsigned>(mCount + pCount)) -
+                                             static_cast<unsigned long long>(__popc(selfSeen));
+            S.counts[0] += inter;
+            S.counts[1] += tests;
+            S.counts[2] += undecidedTests;
+            S.counts[3] += rounds;
+            if (kExpand) {
+                S.counts[4] += groupEvals;
+                S.counts[5] += bucketLeaves;
+            }
+            if (kDebug && w.groupCounts != nullptr) w.groupCounts[g] = static_cast<uint32_t>(inter);
         }
         __syncwarp();
     }
     if (lane == 0) {
         DevStatus* st = reinterpret_cast<DevStatus*>(w.status);
-        atomicAdd(&st->counters[kCntGravityInteractions], nInter);
-        atomicAdd(&st->counters[kCntGravityNodeTests], nTests);
-        atomicAdd(&st->counters[kCntGravityUndecided], nUndecided);
+        atomicAdd(&st->counters[kCntGravityInteractions], S.counts[0]);
+        atomicAdd(&st->counters[kCntGravityNodeTests], S.counts[1]);
+        atomicAdd(&st->counters[kCntGravityUndecided], S.counts[2]);
         if (kExpand) {
-            atomicAdd(&st->counters[kCntGravityGroupEvals], nGroupEvals);
-            atomicAdd(&st->counters[kCntGravityBucketLeaves], nBucketLeaves);
+            atomicAdd(&st->counters[kCntGravityGroupEvals], S.counts[4]);
+            atomicAdd(&st->counters[kCntGravityBucketLeaves], S.counts[5]);
         }
-        atomicAdd(&st->counters[kCntGravityRounds], nRounds);
+        atomicAdd(&st->counters[kCntGravityRounds], S.counts[3]);
         atomicMax(&st->counters[kCntGravityStackPeak], static_cast<unsigned long long>(spPeak));
         if (overflowed) atomicOr(&st->flags, kFlagStackOverflow);
     }
@@ -722,6 +918,8 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     uint32_t* counter = w.words + kWGroupCounter;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
+    // (the learned mode's fallback, runIf, walks the records its first walk wrote)
+    if (n >= 2u && w.runIf == nullptr) pairNodesKernel<<<(n - 1u + 255u) / 256u, 256, 0, st>>>(w, n);
     FarCapture ff{};
     using GravFn = void (*)(AstraeaParticles, Work, uint32_t, float, uint32_t, uint32_t*, FarCapture);
     GravFn kernel = nullptr;

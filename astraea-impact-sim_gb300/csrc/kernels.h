@@ -21,6 +21,12 @@ __device__ __forceinline__ float warpMaxF(float v) {
     return v;
 }
 
+__device__ __forceinline__ float warpSumF(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // Reduce each thread's partial AABB over the block and merge it into the
 // ordered-uint bound words with atomics (engine/sph_gravity.cu:300-324).
 // Every thread of the block must call it.

@@ -264,14 +264,14 @@ __global__ void __launch_bounds__(kSortThreads, kItems <= 4 ? 3 : 2) onesweepKer
     uint64_t key[kItems];
     uint32_t rank[kItems];
     const uint32_t myFirst = warpBase + static_cast<uint32_t>(lane);
-    auto digitOf = [&](int k) {                     // 0x100 behind the end of the input
-        return myFirst + 32u * static_cast<uint32_t>(k) < n ? static_cast<uint32_t>(key[k] >> shift) & 0xFFu : 0x100u;
-    };
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
         const uint32_t idx = myFirst + 32u * static_cast<uint32_t>(k);
         key[k] = idx < n ? keysIn[idx] : 0ull;
     }
+    auto digitOf = [&](int k) {                     // 0x100 behind the end of the input
+        return myFirst + 32u * static_cast<uint32_t>(k) < n ? static_cast<uint32_t>(key[k] >> shift) & 0xFFu : 0x100u;
+    };
     // global start of every bin for this pass (exclusive scan of the histogram)
     const uint32_t binStart = binExclusiveScan(binCount, s.scanTmp);
 #pragma unroll

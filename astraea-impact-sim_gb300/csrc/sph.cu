@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kWarps * 32) buildNeighborsKernel(Work w, uint
                 bmax = __ldg(&rec[3]);
                 cl = __float_as_int(r1.y);
                 cr = __float_as_int(r1.z);
-                nodeHs = r1.w;
+                nodeHs = bmax.w;
                 // (1) box-box distance bounds every member's point-box distance
                 const float dx = fmaxf(0.0f, fmaxf(bmin.x - gmaxx, gminx - bmax.x));
                 const float dy = fmaxf(0.0f, fmaxf(bmin.y - gmaxy, gminy - bmax.y));
@@ -360,7 +360,7 @@ __device__ __forceinline__ void forEachCandidate(const Work& w, uint32_t i, F&& 
         const float4 r1 = __ldg(&rec[1]);
         const float4 bmin = __ldg(&rec[2]);
         const float4 bmax = __ldg(&rec[3]);
-        const float R = fmaxf(Hs, r1.w);
+        const float R = fmaxf(Hs, bmax.w);
         if (pointBoxDist2(me.x, me.y, me.z, bmin.x, bmin.y, bmin.z, bmax.x, bmax.y, bmax.z) <= R * R * 1.00001f) {
             if (sp + 2 <= kTreeStack) {
                 stack[sp++] = __float_as_int(r1.y);

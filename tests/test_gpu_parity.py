@@ -473,3 +473,45 @@ def test_morton_sort_with_far_outliers(n, far):
     assert np.array_equal(p.download(["originalId"])["originalId"], order)
     assert np.array_equal(bvh.t["mortonCodesSorted"].cpu().numpy().view(np.uint64), code[order])
     assert np.array_equal(bvh.t["indicesSorted"].cpu().numpy(), order)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 31, 63, 97, 1000, 4111])
+@pytest.mark.parametrize("shape", ["cloud", "line", "shell", "far", "clumps"])
+def test_gravity_walk_sets_at_edges(n, shape):
+    """Each group's interaction count equals the oracle's (short last groups,
+    flat and hollow groups whose box, octant planes and extreme members bound
+    them badly, groups far from the origin, coincident members), for angles on
+    both sides of the inside-box rule and at 0; the forces agree with it."""
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(n, 3))
+    if shape == "line":
+        x[:, 1:] *= 1.0e-4
+    elif shape == "shell":
+        x /= np.linalg.norm(x, axis=1)[:, None]
+    elif shape == "far":
+        x = x * 0.05 + np.array([40.0, -30.0, 20.0])
+    elif shape == "clumps":
+        x = x[rng.integers(0, max(n // 8, 1), n)] + rng.normal(size=(n, 3)) * rng.choice([0.0, 1.0e-3], n)[:, None]
+    st = scenarios.empty_state(n)
+    for k, f in enumerate(("posX", "posY", "posZ")):
+        st[f][:] = x[:, k]
+    st["mass"][:] = rng.uniform(0.5, 1.5, n) / n
+    st["h"][:] = st["h0"][:] = rng.uniform(0.01, 0.03, n)
+    st["rho"][:] = 1.0e-3
+    st["originalId"][:] = np.arange(n, dtype=np.uint32)
+    p, alt, bvh = gpu_setup(st)
+    o = oracle.Oracle(st)
+    engine.set_node_rounding(1)
+    try:
+        engine.sort_and_build_bvh(p, alt, bvh)
+    finally:
+        engine.set_node_rounding(0)
+    o.sort_and_build()
+    for theta in (0.0, 0.3, 0.5, 0.6, 1.0):
+        assert np.array_equal(engine.gravity_group_counts(p, bvh, theta), o.gravity_group_counts(theta)), theta
+        engine.gravity_barnes_hut(p, bvh, theta)
+        o.gravity(theta)
+        g, c = p.download(), o.state()
+        for f in ("accX", "accY", "accZ", "phiGrav"):
+            assert rel_rms(g[f], c[f]) < TOL, (theta, f)
