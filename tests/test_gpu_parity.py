@@ -515,3 +515,30 @@ def test_gravity_walk_sets_at_edges(n, shape):
         g, c = p.download(), o.state()
         for f in ("accX", "accY", "accZ", "phiGrav"):
             assert rel_rms(g[f], c[f]) < TOL, (theta, f)
+
+
+@pytest.mark.parametrize("n", [(1 << 20) + 1, (1 << 20) + 63])
+@pytest.mark.parametrize("theta", [0.3, 0.5, 0.7])
+def test_gravity_walk_of_large_scenes(n, theta):
+    """Above 2^20 particles the terms are added in another order: the walk takes
+    the interactions of the general one, which the counting call runs, and the
+    forces agree within the parity bound (they differ in rounding only)."""
+    rng = np.random.default_rng(n)
+    st = scenarios.empty_state(n)
+    for f in ("posX", "posY", "posZ"):
+        st[f][:] = rng.normal(size=n)
+    st["mass"][:] = rng.uniform(0.5, 1.5, n) / n
+    st["h"][:] = st["h0"][:] = rng.uniform(0.01, 0.03, n)
+    st["rho"][:] = 1.0e-3
+    st["originalId"][:] = np.arange(n, dtype=np.uint32)
+    p, alt, bvh = gpu_setup(st)
+    engine.sort_and_build_bvh(p, alt, bvh)
+    engine.reset_device_status()
+    engine.gravity_barnes_hut(p, bvh, theta)
+    flags, counters = engine.read_device_status()
+    a = p.download(["accX", "accY", "accZ", "phiGrav"])
+    counts = engine.gravity_group_counts(p, bvh, theta)
+    b = p.download(["accX", "accY", "accZ", "phiGrav"])
+    assert flags == 0 and counters["gravity_interactions"] == int(counts.astype(np.int64).sum())
+    for f in a:
+        assert rel_rms(a[f], b[f]) < TOL, f
