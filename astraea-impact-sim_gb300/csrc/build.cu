@@ -61,11 +61,18 @@ __device__ __forceinline__ int karrasDelta(const uint64_t* __restrict__ codes, i
             X(curlVY) X(curlVZ) X(shepardC) X(surfFactor) X(phiGrav)
 #define AG_DEAD_OTHER(X) X(phaseId)
 
+// Clears the words of the next neighbour build (one thread; instead of a memset
+// in front of it).
+__device__ __forceinline__ void armNeighborBuild(const Work& w) {
+    for (int k = 0; k < 4; ++k) w.words[kWNbrCounter + k] = 0u;
+}
+
 template <bool kAllFields>
 __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticles p, AstraeaParticles alt,
                                                                  AstraeaRadixBvh bvh, const float4* __restrict__ posSrc,
                                                                  Work w, uint32_t n, uint32_t* livingFlags) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0u) armNeighborBuild(w);
     bool tracer = false, intact = false;
     uint32_t massBits = 0u;                         // |m| as bits: ordered like the values
     if (i < n) {
@@ -162,6 +169,7 @@ __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticle
 __global__ void __launch_bounds__(256) refreshLeavesKernel(AstraeaParticles p, Work w, uint32_t n, bool withVelRho) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i == 0u) armNeighborBuild(w);
     const float hI = fmaxf(__ldg(&p.h[i]), 1.0e-6f);
     const float h0I = fmaxf(__ldg(&p.h0[i]), 1.0e-6f);
     const float m = __ldg(&p.mass[i]);
@@ -170,7 +178,7 @@ __global__ void __launch_bounds__(256) refreshLeavesKernel(AstraeaParticles p, W
     w.leafAux[i] = make_float4(Hs, 0.8f * h0I, 2.0f * __ldg(&p.h[i]), m);
     const float H = 2.0f * hI;                                      // the drift's 2 max(h, 1e-6)
     w.drift[i].a = make_float4(__ldg(&p.posX[i]), __ldg(&p.posY[i]), __ldg(&p.posZ[i]), H);
-    w.driftAux[i] = make_float2(__ldg(&p.mass[i]), wendlandNorm(H));
+    w.driftAux[i] = make_float2(__ldg(&p.mass[i]), 1.0f / H);
     if (withVelRho) {
         const float4 vr = make_float4(__ldg(&p.velX[i]), __ldg(&p.velY[i]), __ldg(&p.velZ[i]), __ldg(&p.rho[i]));
         w.leaf[i].b = make_float4(vr.x, vr.y, vr.z, __fdividef(m, fmaxf(vr.w, 1.0e-9f)));

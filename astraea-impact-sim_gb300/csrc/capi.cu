@@ -169,7 +169,10 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     const size_t oTable = take(levMax * nbMax * 32), oBMom = take(nbMax * 80), oQuad = take(C * 32);
     const size_t oDrift = take(C * 16);
     const size_t oDRec = take(C * 32), oDAux = take(C * 8);
-    const size_t oCnt = take(C * 4), oList = take((C + 31) / 32 * 32 * maxNbr * 4), oWords = take(kWCount * 4);
+    const size_t oCnt = take(C * 4), oList = take((C + 31) / 32 * 32 * maxNbr * 4);
+    // lists above maxNbr entries: rare; what does not fit here is walked in each pass
+    const size_t heavyCap = C / 64 + 256, poolCap = std::min<size_t>(C * 4 + 65536, 0xfffffff0u);
+    const size_t oHeavy = take(heavyCap * 16), oPool = take(poolCap * 4), oWords = take(kWCount * 4);
     const size_t oSort = take(sortWords * 4), oDt = take(64);
     void* block = nullptr;
     AG_CUDA(cudaMalloc(&block, off));
@@ -197,6 +200,10 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     w.driftAux = reinterpret_cast<float2*>(b + oDAux);
     w.nbrCount = reinterpret_cast<uint32_t*>(b + oCnt);
     w.nbrList = reinterpret_cast<uint32_t*>(b + oList);
+    w.heavy = reinterpret_cast<uint4*>(b + oHeavy);
+    w.heavyCap = static_cast<uint32_t>(heavyCap);
+    w.pool = reinterpret_cast<uint32_t*>(b + oPool);
+    w.poolCap = static_cast<uint32_t>(poolCap);
     w.words = reinterpret_cast<uint32_t*>(b + oWords);
     w.sortScratch = reinterpret_cast<uint32_t*>(b + oSort);
     w.sortScratchWords = sortWords;
@@ -744,7 +751,7 @@ AstraeaStatus astraea_gb300_sph_pass1_neighbors(AstraeaParticles* p, const Astra
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
     AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
-    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps)));
+    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchPass1(*p, ws->w, n, st));
     ws->stepCacheValid = false;
     return ASTRAEA_OK;
@@ -830,7 +837,7 @@ AstraeaStatus astraea_gb300_sph_pass2_forces(AstraeaParticles* p, const AstraeaR
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
     AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
-    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps)));
+    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchPackPass2Records(*p, ws->w, n, st));
     const uint32_t* living = (bvh->livingFlags != nullptr) ? bvh->livingFlags : ds->zeroWords;   // :2104
     AG_LAUNCH(launchPass2(*p, ws->w, n, living, st));
@@ -866,7 +873,7 @@ AstraeaStatus astraea_gb300_leapfrog_drift(AstraeaParticles* p, float dtPsu, con
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
     AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
-    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps)));
+    AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchDrift(*p, ws->w, n, nullptr, dtPsu, true, false, nullptr, st));
     ws->stepCacheValid = false;
     return ASTRAEA_OK;
@@ -1505,7 +1512,7 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
         AG_LAUNCH(launchSetDtSlots(ws->dtSlots, q, prevDtPsu, ws->rawMin, st));
         AG_LAUNCH(launchReduceDt(*p, n, ws->rawMin + q, sms, st));
         AG_LAUNCH(launchRefreshLeaves(*p, w, n, false, st));
-        if (useBvh) AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps)));
+        if (useBvh) AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps), true));
     }
     // 1. opening half kick; dt resolved on the device
     marks.mark(ASTRAEA_STAGE_KICK);
@@ -1528,7 +1535,7 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
     if (s != ASTRAEA_OK) return s;
     // 4. neighbour lists for pass 1, pass 2 and the next drift
     marks.mark(ASTRAEA_STAGE_NEIGHBOURS);
-    AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps)));
+    AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps), true));
     marks.mark(ASTRAEA_STAGE_PASS1);
     AG_LAUNCH(launchPass1(*p, w, n, st));
     marks.mark(ASTRAEA_STAGE_EOS);

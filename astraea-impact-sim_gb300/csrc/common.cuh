@@ -518,6 +518,7 @@ __device__ __forceinline__ EosOut evaluateEosF32(uint8_t matRaw, float rhoIn, fl
 }
 
 constexpr int kRec2Width = 6;   // float4 per pass-2 record
+constexpr uint32_t kHeavyMark = 0xffffffffu;   // Work::nbrCount of a particle whose list is in the pool
 
 // Two float4 of one particle in one 32-byte aligned record, read whole by
 // ldg256 in the SPH pair loops.
@@ -545,9 +546,13 @@ struct Work {
     float4* driftPos;      // {x, y, z, 0} after the drift
     Rec32* drift;          // for the next drift: a {x, y, z, H = 2 max(h, 1e-6)} (pass 1 / leaf refresh),
                            // b {vx, vy, vz, rho} (opening kick / leaf refresh)
-    float2* driftAux;      // {m, 21 / (2 pi H^3)} (the Wendland norm of H)
-    uint32_t* nbrCount;
+    float2* driftAux;      // {m, 1 / H}
+    uint32_t* nbrCount;    // entries of each list; above maxNbr: no list (kHeavyMark: one in the pool)
     uint32_t* nbrList;     // group-interleaved: entry k of particle i at ((i/32) maxNbr + k) 32 + i%32
+    uint4* heavy;          // lists in the pool: {particle, first word, entries (0: no place), 0}
+    uint32_t heavyCap;
+    uint32_t* pool;
+    uint32_t poolCap;      // words
     uint32_t* words;       // small words, see WordIndex
     uint32_t* sortScratch; // histograms + look-back + tile counters
     size_t sortScratchWords;
@@ -569,9 +574,11 @@ enum WordIndex : int {
     kWDtMin = 8,         // 2 dt-min bit words (step parity)
     kWDtState = 10,      // 2 float dt slots (step parity)
     kWGroupCounter = 12, // persistent-grid work counter (gravity)
-    kWNbrCounter = 13,   // persistent-grid work counter (neighbour build)
     kWMassMax = 14,      // bits of the largest |mass| (set by the permutation, read by the refit)
     kWBoundsF = 16,      // 6 floats: decoded bounds
+    kWNbrCounter = 24,   // persistent-grid work counter (neighbour build), cleared with the next three
+    kWHeavyCount = 25,   // particles whose list did not fit its capacity
+    kWPoolUsed = 26,     // 64 bits: pool words they asked for
     kWCount = 32
 };
 

@@ -7,16 +7,21 @@
 //   * one group walk per step (buildNeighborsKernel) writes, for every
 //     particle, the list of j with r_ij < max(Hs_i, Hs_j) -- a superset of the
 //     pass-1, pass-2 and next-drift neighbour sets (see common.cuh);
-//   * pass 1, pass 2 and the drift run one thread per particle over its own
-//     list, re-applying the engine's exact FP32 range test, so every lane
-//     works on its own pairs;
+//   * pass 1, pass 2 and the drift work on the lists, re-applying the engine's
+//     exact FP32 range test, one thread per particle in a large scene; in a
+//     small one, whose threads would not fill the GPU, two or four lanes share
+//     a particle's list and add up their sums (lanesFor);
 //   * neighbour data is read from packed records (pass 1: position + Hs
 //     and velocity + volume m/rho in one 32-byte record; drift: position + H and
 //     velocity + density; pass 2: a 96-byte record written by the EOS
 //     kernel, read in three 32-byte pieces), one 256-bit load per piece
-//     instead of one gather per field.
-// A particle whose list overflowed the per-particle capacity is served by a
-// per-thread depth-first walk with the same superset test (rare path).
+//     instead of one gather per field;
+//   * a particle whose list does not fit its capacity (a lone particle with a
+//     large h beside a dense body has thousands of neighbours) gets a list in a
+//     shared pool, and whole warps work on those lists in the first blocks of
+//     each pass: one thread over such a list holds up the launch.
+// When the pool is exhausted too, a particle is served by a per-thread
+// depth-first walk with the same superset test.
 #include "kernels.h"
 
 namespace astraea_gb300 {
@@ -58,6 +63,7 @@ __device__ __forceinline__ void storeIf(uint32_t* p, uint32_t v, bool pred) {
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) buildNeighborsKernel(Work w, uint32_t n, uint32_t numGroups,
                                                                     uint32_t* groupCounter) {
+    chained();
     __shared__ NbWarpSmem smem[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     NbWarpSmem& S = smem[warp];
@@ -299,7 +305,11 @@ __global__ void __launch_bounds__(kWarps * 32) buildNeighborsKernel(Work w, uint
         flush((cCount + 1) >> 1);
         if (active) {
             w.nbrCount[i] = cnt;
-            if (cnt > maxNbr) overflow = true;
+            if (cnt > maxNbr) {                     // poolListsKernel goes on with it
+                overflow = true;
+                const uint32_t slot = atomicAdd(&w.words[kWHeavyCount], 1u);
+                if (slot < w.heavyCap) w.heavy[slot] = make_uint4(i, 0u, cnt, 0u);
+            }
         }
         nEntries += cnt;
         __syncwarp();
@@ -314,24 +324,23 @@ __global__ void __launch_bounds__(kWarps * 32) buildNeighborsKernel(Work w, uint
     }
 }
 
+// Where a list is: the k-th entry at list[k stride].
+struct List {
+    const uint32_t* list;
+    uint32_t stride, count;
+};
 // Neighbour lists are group-interleaved: entry k of particle i is word
-// ((i / 32) maxNbr + k) 32 + i % 32, so the 32 particles of a group (the
-// lanes of one warp in every pass) read their k-th entries as one 128-byte
-// row and a lane's list never shares a sector with another lane's.
-__device__ __forceinline__ const uint32_t* listOf(const Work& w, uint32_t i) {
-    return w.nbrList + static_cast<size_t>(i >> 5) * w.maxNbr * 32u + (i & 31u);
+// ((i / 32) maxNbr + k) 32 + i % 32, so the 32 particles of a group read their
+// k-th entries as one 128-byte row and a lane's list never shares a sector with
+// another lane's.
+__device__ __forceinline__ List listOf(const Work& w, uint32_t i, uint32_t count) {
+    return List{w.nbrList + static_cast<size_t>(i >> 5) * w.maxNbr * 32u + (i & 31u), 32u, count};
 }
 
-// Visit every j of particle i's superset list; when the list overflowed,
-// walk the tree depth-first with the same superset test instead.
+// Visit every j with r_ij < max(Hs_i, Hs_j) by a depth-first tree walk: a
+// particle without a list.
 template <class F>
-__device__ __forceinline__ void forEachCandidate(const Work& w, uint32_t i, F&& f) {
-    const uint32_t c = __ldg(&w.nbrCount[i]);
-    if (c <= w.maxNbr) {
-        const uint32_t* list = listOf(w, i);
-        for (uint32_t k = 0; k < c; ++k) f(__ldg(&list[static_cast<size_t>(k) * 32u]));
-        return;
-    }
+__device__ __forceinline__ void walkNeighbors(const Work& w, uint32_t i, F&& f) {
     atomicAdd(&w.status->counters[kCntFallbackWalks], 1ull);
     const float4 me = __ldg(&w.leaf[i].a);
     const float Hs = me.w;
@@ -374,43 +383,57 @@ __device__ __forceinline__ void forEachCandidate(const Work& w, uint32_t i, F&& 
 
 // List words are read once per pass and the lists (308 B per particle) do
 // not fit in L1: read them without allocating in L1, which keeps L1 for the
-// neighbour records.  Four consecutive entries of one particle (32 words
-// apart in the group-interleaved layout).
+// neighbour records.
 __device__ __forceinline__ uint32_t ldWordNoL1(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ uint4 ldListNoL1(const uint32_t* list, uint32_t k) {
-    const uint32_t* p = list + static_cast<size_t>(k) * 32u;
-    return make_uint4(ldWordNoL1(p), ldWordNoL1(p + 32), ldWordNoL1(p + 64), ldWordNoL1(p + 96));
+__device__ __forceinline__ uint4 ldListNoL1(const List& l, uint32_t k) {
+    const uint32_t* p = l.list + static_cast<size_t>(k) * l.stride;
+    return make_uint4(ldWordNoL1(p), ldWordNoL1(p + l.stride), ldWordNoL1(p + 2u * l.stride), ldWordNoL1(p + 3u * l.stride));
 }
 
-// Same candidate set as forEachCandidate, with each candidate's first record
-// loaded by `load(j)` for four list entries before any `body(j, rec)` runs,
-// so four independent gathers are in flight per thread, and the next four
-// list entries loaded before those four bodies run.
-template <class L, class B>
-__device__ __forceinline__ void forEachCandidatePrefetched(const Work& w, uint32_t i, L&& load, B&& body) {
-    const uint32_t c = __ldg(&w.nbrCount[i]);
-    if (c <= w.maxNbr) {
-        const uint32_t* list = listOf(w, i);
-        uint32_t k = 0;
-        uint4 q = c >= 4 ? ldListNoL1(list, 0u) : make_uint4(0u, 0u, 0u, 0u);
-        for (; k + 4 <= c; k += 4) {
-            const uint4 next = (k + 8 <= c) ? ldListNoL1(list, k + 4) : q;
-            const auto r0 = load(q.x), r1 = load(q.y), r2 = load(q.z), r3 = load(q.w);
-            body(q.x, r0); body(q.y, r1); body(q.z, r2); body(q.w, r3);
-            q = next;
-        }
-        for (; k < c; ++k) {
-            const uint32_t j = __ldg(&list[static_cast<size_t>(k) * 32u]);
-            body(j, load(j));
-        }
-        return;
+// Lane `sub` of the kLanes that share a list visits its fours sub, sub +
+// kLanes, ...: each candidate's first record loaded by `load(j)` for four
+// entries before any `body(j, rec)` runs, so four independent gathers are in
+// flight per thread, and the next four entries loaded before those four
+// bodies run.
+template <int kLanes, class L, class B>
+__device__ __forceinline__ void forEachListed(const List& l, uint32_t sub, L&& load, B&& body) {
+    const uint32_t c = l.count;
+    uint32_t k = 4u * sub;
+    uint4 q = k + 4u <= c ? ldListNoL1(l, k) : make_uint4(0u, 0u, 0u, 0u);
+    for (; k + 4u <= c; k += 4u * kLanes) {
+        const uint32_t kn = k + 4u * kLanes;
+        const uint4 next = (kn + 4u <= c) ? ldListNoL1(l, kn) : q;
+        const auto r0 = load(q.x), r1 = load(q.y), r2 = load(q.z), r3 = load(q.w);
+        body(q.x, r0); body(q.y, r1); body(q.z, r2); body(q.w, r3);
+        q = next;
     }
-    forEachCandidate(w, i, [&](uint32_t j) { body(j, load(j)); });
+    for (; k < c; ++k) {                             // the last, shorter four: one lane's
+        const uint32_t j = __ldg(l.list + static_cast<size_t>(k) * l.stride);
+        body(j, load(j));
+    }
 }
+
+// Sum over the kLanes lanes of a particle (every lane of the warp calls it).
+template <int kLanes>
+__device__ __forceinline__ void sumLanes(float& v) {
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+}
+template <int kLanes>
+__device__ __forceinline__ void sumLanes(uint32_t& v) {
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+}
+
+// The blocks of a pass: the first kHeavyBlocks work on the pool's lists, a warp
+// per particle; then kLanes threads per particle.
+constexpr uint32_t kHeavyBlocks = 38, kPassThreads = 128;
+constexpr uint32_t kHeavyWarps = kHeavyBlocks * kPassThreads / 32;
+__device__ __forceinline__ uint32_t heavyCount(const Work& w) { return min(__ldg(&w.words[kWHeavyCount]), w.heavyCap); }
 
 // Adds a per-thread count to a device counter with one atomic per group of
 // threads that reach the call together (the running threads of a warp).
@@ -421,11 +444,87 @@ __device__ __forceinline__ void addCount(DevStatus* st, int which, uint32_t v) {
         atomicAdd(&st->counters[which], static_cast<unsigned long long>(tot));
 }
 
+// The lists in the pool: a warp per particle walks the tree with its own radius,
+// 32 nodes at a time from a stack in shared memory, and appends the particles
+// inside, which are those the group walk counted (the node test has the same
+// margin; a list never grows past its count).  Latency bound: a walk is some
+// twenty rounds of two dependent loads, and there are few of them; almost always
+// there is none, and the launch, chained to the kernels around it, costs less than 1 us
+// (2.5 to 4 as a plain one).
+constexpr int kPoolStack = 1024, kPoolWarps = 4;
+__global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint32_t n) {
+    chained();
+    __shared__ int stacks[kPoolWarps][kPoolStack];
+    const uint32_t lane = threadIdx.x & 31u, total = heavyCount(w);
+    int* stack = stacks[threadIdx.x >> 5];
+    for (uint32_t e = blockIdx.x * kPoolWarps + (threadIdx.x >> 5); e < total; e += gridDim.x * kPoolWarps) {
+        const uint4 h = w.heavy[e];
+        unsigned long long place = 0;                    // 64 bits: the sum of what is asked for can pass 2^32
+        if (lane == 0u)
+            place = atomicAdd(reinterpret_cast<unsigned long long*>(&w.words[kWPoolUsed]), static_cast<unsigned long long>(h.z));
+        place = __shfl_sync(0xffffffffu, place, 0);
+        if (place + h.z > w.poolCap) {                 // served by its own walk in each pass
+            if (lane == 0u) w.heavy[e].z = 0u;
+            continue;
+        }
+        const float4 me = __ldg(&w.leaf[h.x].a);
+        uint32_t* list = w.pool + place;
+        uint32_t cnt = 0u, rounds = 0u;
+        int sp = 1;
+        if (lane == 0u) stack[0] = 0;
+        __syncwarp();
+        while (sp > 0 && ++rounds <= 2u * n) {
+            const int take = min(sp, 32);
+            const int c = static_cast<int>(lane) < take ? stack[sp - take + lane] : static_cast<int>(n);
+            sp -= take;
+            __syncwarp();
+            uint32_t hitJ = 0u;
+            bool hit = false, open = false;
+            int cl = 0, cr = 0;
+            if (c < 0 && c >= -static_cast<int>(n)) {
+                hitJ = static_cast<uint32_t>(~c);
+                const float4 q = __ldg(&w.leaf[hitJ].a);
+                const float dx = me.x - q.x, dy = me.y - q.y, dz = me.z - q.z;
+                const float R = fmaxf(me.w, q.w);
+                hit = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < R * R && hitJ != h.x;
+            } else if (c >= 0 && c < static_cast<int>(n) - 1) {
+                const float4* rec = w.node + 4 * static_cast<size_t>(c);
+                const float4 r1 = __ldg(&rec[1]), bmin = __ldg(&rec[2]), bmax = __ldg(&rec[3]);
+                const float R = fmaxf(me.w, bmax.w);
+                open = pointBoxDist2(me.x, me.y, me.z, bmin.x, bmin.y, bmin.z, bmax.x, bmax.y, bmax.z) <=
+                       R * R * 1.00001f;
+                cl = __float_as_int(r1.y);
+                cr = __float_as_int(r1.z);
+            }
+            const unsigned hits = __ballot_sync(0xffffffffu, hit), opens = __ballot_sync(0xffffffffu, open);
+            const uint32_t at = cnt + __popc(hits & laneMaskLt());
+            if (hit && at < h.z) list[at] = hitJ;
+            cnt += __popc(hits);
+            if (sp + 2 * __popc(opens) > kPoolStack) {      // cannot happen for trees of depth < 32
+                if (lane == 0u) atomicOr(&w.status->flags, kFlagStackOverflow);
+                break;
+            }
+            if (open) {
+                const int pos = sp + 2 * __popc(opens & laneMaskLt());
+                stack[pos] = cl;
+                stack[pos + 1] = cr;
+            }
+            sp += 2 * __popc(opens);
+            __syncwarp();
+        }
+        if (lane == 0u) {
+            w.heavy[e] = make_uint4(h.x, static_cast<uint32_t>(place), min(cnt, h.z), 0u);
+            w.nbrCount[h.x] = kHeavyMark;
+        }
+        __syncwarp();
+    }
+}
+
 // ---------------------------------------------------------------- pass 1 ---
-// 6 blocks per SM (80 registers): no spills; 7 blocks (72) spilled and ran 1.6 % slower
-__global__ void __launch_bounds__(128, 6) pass1Kernel(AstraeaParticles p, Work w, uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// One particle's pass 1; called by its kLanes lanes, `sub` their number.
+template <int kLanes>
+__device__ __forceinline__ void pass1Particle(const AstraeaParticles& p, const Work& w, uint32_t n, uint32_t i,
+                                              const List& l, uint32_t sub, bool walk, bool write) {
     const F8 rec = ldg256(&w.leaf[i].a);
     const float4 me = rec.a, vr = rec.b;
     const float mi = __ldg(&p.mass[i]);
@@ -438,39 +537,50 @@ __global__ void __launch_bounds__(128, 6) pass1Kernel(AstraeaParticles p, Work w
     const float Hi5 = (Hi * Hi) * (Hi * Hi) * Hi;
     const float gNormI = 210.0f / (kPiF * Hi5);
     const float invHi = 1.0f / Hi;
-    float shep = (mi / rhoI) * w0;
-    int ngb = 1;
+    float shep = (sub == 0u) ? (mi / rhoI) * w0 : 0.0f;
+    uint32_t ngb = (sub == 0u) ? 1u : 0u;
     float nsX = 0.f, nsY = 0.f, nsZ = 0.f;
     float gXX = 0.f, gXY = 0.f, gXZ = 0.f, gYX = 0.f, gYY = 0.f, gYZ = 0.f, gZX = 0.f, gZY = 0.f, gZZ = 0.f;
+    // one 32-byte record per candidate: {x, y, z, Hs}, {vx, vy, vz, m / max(rho, 1e-9)}
+    auto load = [&](uint32_t j) { return ldg256(&w.leaf[j].a); };
+    auto body = [&](uint32_t, const F8& rj) {
+        const float4 q = rj.a;
+        const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
+        const float r2 = len2Engine(dx, dy, dz);
+        if (!(r2 < Hi2)) return;                       // sph_gravity.cu:713
+        ++ngb;
+        const float4 vj = rj.b;
+        const float r = sqrtf(r2);
+        const float volJ = vj.w;
+        const float wij = wendlandC2I(r, Hi, invHi, w0);
+        shep += volJ * wij;
+        nsX -= volJ * dx * wij;
+        nsY -= volJ * dy * wij;
+        nsZ -= volJ * dz * wij;
+        const float gc = wendlandC2GradI(r, Hi, invHi, gNormI);
+        const float gx = gc * dx, gy = gc * dy, gz = gc * dz;
+        const float dvx = vj.x - vr.x, dvy = vj.y - vr.y, dvz = vj.z - vr.z;
+        gXX += volJ * dvx * gx; gXY += volJ * dvx * gy; gXZ += volJ * dvx * gz;
+        gYX += volJ * dvy * gx; gYY += volJ * dvy * gy; gYZ += volJ * dvy * gz;
+        gZX += volJ * dvz * gx; gZY += volJ * dvz * gy; gZZ += volJ * dvz * gz;
+    };
     if (n >= 2u) {
-        // one 32-byte record per candidate: {x, y, z, Hs}, {vx, vy, vz, m / max(rho, 1e-9)}
-        forEachCandidatePrefetched(w, i, [&](uint32_t j) { return ldg256(&w.leaf[j].a); }, [&](uint32_t j, const F8& rj) {
-            const float4 q = rj.a;
-            const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
-            const float r2 = len2Engine(dx, dy, dz);
-            if (!(r2 < Hi2)) return;                       // sph_gravity.cu:713
-            ++ngb;
-            const float4 vj = rj.b;
-            const float r = sqrtf(r2);
-            const float volJ = vj.w;
-            const float wij = wendlandC2I(r, Hi, invHi, w0);
-            shep += volJ * wij;
-            nsX -= volJ * dx * wij;
-            nsY -= volJ * dy * wij;
-            nsZ -= volJ * dz * wij;
-            const float gc = wendlandC2GradI(r, Hi, invHi, gNormI);
-            const float gx = gc * dx, gy = gc * dy, gz = gc * dz;
-            const float dvx = vj.x - vr.x, dvy = vj.y - vr.y, dvz = vj.z - vr.z;
-            gXX += volJ * dvx * gx; gXY += volJ * dvx * gy; gXZ += volJ * dvx * gz;
-            gYX += volJ * dvy * gx; gYY += volJ * dvy * gy; gYZ += volJ * dvy * gz;
-            gZX += volJ * dvz * gx; gZY += volJ * dvz * gy; gZZ += volJ * dvz * gz;
-        });
+        forEachListed<kLanes>(l, sub, load, body);
+        if (walk && sub == 0u) walkNeighbors(w, i, [&](uint32_t j) { body(j, load(j)); });
     }
-    addCount(w.status, kCntPass1Pairs, static_cast<uint32_t>(ngb - 1));
+    if constexpr (kLanes > 1) {
+        sumLanes<kLanes>(shep); sumLanes<kLanes>(ngb);
+        sumLanes<kLanes>(nsX); sumLanes<kLanes>(nsY); sumLanes<kLanes>(nsZ);
+        sumLanes<kLanes>(gXX); sumLanes<kLanes>(gXY); sumLanes<kLanes>(gXZ);
+        sumLanes<kLanes>(gYX); sumLanes<kLanes>(gYY); sumLanes<kLanes>(gYZ);
+        sumLanes<kLanes>(gZX); sumLanes<kLanes>(gZY); sumLanes<kLanes>(gZZ);
+    }
+    if (sub != 0u || !write) return;
+    addCount(w.status, kCntPass1Pairs, ngb - 1u);
     p.shepardC[i] = shep;                                   // sph_gravity.cu:772-787
     const float normNs = sqrtf(nsX * nsX + nsY * nsY + nsZ * nsZ);
     float fs = fminf(1.0f, fmaxf(0.0f, 1.6f * fmaxf(1.0f - shep, normNs / hi) - 0.15f));
-    if (ngb <= 2) fs = 1.0f;
+    if (ngb <= 2u) fs = 1.0f;
     p.surfFactor[i] = fs;
     p.divV[i] = gXX + gYY + gZZ;
     p.curlVX[i] = gZY - gYZ;
@@ -483,17 +593,37 @@ __global__ void __launch_bounds__(128, 6) pass1Kernel(AstraeaParticles p, Work w
     // records of the next drift (positions and h do not change before it)
     const float Hd = 2.0f * fmaxf(hNew, 1.0e-6f);
     w.drift[i].a = make_float4(me.x, me.y, me.z, Hd);
-    w.driftAux[i] = make_float2(mi, wendlandNorm(Hd));
+    w.driftAux[i] = make_float2(mi, 1.0f / Hd);
+}
+
+// 6 blocks per SM (80 registers): no spills; 7 blocks (72) spilled and ran 1.6 % slower
+template <int kLanes>
+__global__ void __launch_bounds__(kPassThreads, 6) pass1Kernel(AstraeaParticles p, Work w, uint32_t n) {
+    chained();
+    if (blockIdx.x < kHeavyBlocks) {
+        const uint32_t lane = threadIdx.x & 31u, total = heavyCount(w);
+        for (uint32_t e = blockIdx.x * (kPassThreads / 32u) + (threadIdx.x >> 5); e < total; e += kHeavyWarps) {
+            const uint4 h = __ldg(&w.heavy[e]);
+            if (h.z != 0u) pass1Particle<32>(p, w, n, h.x, List{w.pool + h.y, 1u, h.z}, lane, false, true);
+        }
+        return;
+    }
+    const uint32_t t = (blockIdx.x - kHeavyBlocks) * kPassThreads + threadIdx.x;
+    const uint32_t i = min(t / kLanes, n - 1u), c = __ldg(&w.nbrCount[i]);
+    if (kLanes == 1 && t >= n) return;
+    const bool listed = c <= w.maxNbr;
+    pass1Particle<kLanes>(p, w, n, i, listOf(w, i, listed ? c : 0u), t % kLanes,
+                          !listed && c != kHeavyMark, t / kLanes < n && c != kHeavyMark);
 }
 
 // ---------------------------------------------------------------- pass 2 ---
 // Reads the pass-2 records written by the EOS kernel (layout and derived
 // values: integrate.cu, writePass2Record): one 256-bit load per 32-byte
 // piece, and no per-pair division for quantities of the neighbour alone.
-__global__ void __launch_bounds__(128, 4) pass2Kernel(AstraeaParticles p, Work w, uint32_t n,
-                                                   const uint32_t* livingFlags) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+template <int kLanes>
+__device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const Work& w, uint32_t n, uint32_t i,
+                                              const List& l, uint32_t sub, bool walk, bool write,
+                                              const uint32_t* livingFlags) {
     const float4* R = w.rec2;
     const float4 a0 = __ldg(&R[kRec2Width * static_cast<size_t>(i) + 0]);
     const float4 a1 = __ldg(&R[kRec2Width * static_cast<size_t>(i) + 1]);
@@ -508,87 +638,99 @@ __global__ void __launch_bounds__(128, 4) pass2Kernel(AstraeaParticles p, Work w
     const int matI = __float_as_int(a4.z);
     const float Ri = a4.w;
     const float gradNormI = a5.y, invRhoI2 = a5.z, invHi = a5.w;
-    const float pI = effectivePressure(__ldg(&p.pressure[i]), __ldg(&p.phaseId[i]));   // the record's P_eff
     const float sXXr = sXXi * invRhoI2, sYYr = sYYi * invRhoI2, sZZr = sZZi * invRhoI2;
     const float sXYr = sXYi * invRhoI2, sXZr = sXZi * invRhoI2, sYZr = sYZi * invRhoI2;
-    const float tempI = __ldg(&p.tempK[i]);
-    const float damI = __ldg(&p.damage[i]);
-    const float fSurf = __ldg(&p.surfFactor[i]);
 
     float axS = 0.f, ayS = 0.f, azS = 0.f, drC = 0.f, drD = 0.f, duP = 0.f, duAv = 0.f, duT = 0.f, duS = 0.f;
     float gXX = 0.f, gXY = 0.f, gXZ = 0.f, gYX = 0.f, gYY = 0.f, gYZ = 0.f, gZX = 0.f, gZY = 0.f, gZZ = 0.f;
     uint32_t nPairs = 0;
+    // records in 32-byte pieces: {q0, q1} for every candidate (one sector),
+    // {q2, q3} and {q4, q5} for the candidates in range
+    auto first = [&](uint32_t j) { return ldg256(&R[kRec2Width * static_cast<size_t>(j)]); };
+    auto tested = [&](uint32_t j, const F8& q01) {
+        const float4 b0 = q01.a;
+        const float dx = __fsub_rn(xi, b0.x), dy = __fsub_rn(yi, b0.y), dz = __fsub_rn(zi, b0.z);
+        const float r2 = len2Engine(dx, dy, dz);
+        const float hj = b0.w, Hj = 2.0f * hj;
+        const float Hm = fmaxf(Hi, Hj);
+        if (!(r2 < __fmul_rn(Hm, Hm))) return;          // sph_gravity.cu:1071
+        ++nPairs;
+        const F8 q23 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 2]);
+        const F8 q45 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 4]);
+        const float4 b1 = q01.b, b2 = q23.a, b3 = q23.b, b4 = q45.a, b5 = q45.b;
+        const float mj = b1.w, rhoJ = b2.x, pOverRho2J = b2.y, csJ = b2.z, fBalJ = b2.w;
+        const float volJ = b5.x;
+        const float dvx = vxi - b1.x, dvy = vyi - b1.y, dvz = vzi - b1.z;
+        const float vDotR = dvx * dx + dvy * dy + dvz * dz;
+        const float r = sqrtf(r2);
+        const float gI = wendlandC2GradI(r, Hi, invHi, gradNormI), gJ = wendlandC2GradI(r, Hj, b5.w, b5.y);
+        const float gb = 0.5f * (gI + gJ);
+        const float gx = gb * dx, gy = gb * dy, gz = gb * dz;
+        const float vDotG = dvx * gx + dvy * gy + dvz * gz;
+        drC += volJ * vDotG;                               // continuity (:1114)
+        // The delta-SPH and viscosity terms are evaluated for every pair in
+        // range and kept by a select (the engine's conditions, the same
+        // values): as branches they cost pass 2 11 % at 1M.
+        {                                                  // delta-SPH diffusion (:1115-1119)
+            const float rDotG = -(dx * gx + dy * gy + dz * gz);
+            const float dd = r2 + 0.01f * Hi * Hi;
+            const float t = drD + volJ * (2.0f * (rhoJ - rhoI) / dd) * rDotG;
+            drD = (__float_as_int(b4.z) == matI) ? t : drD;
+        }
+        float piIJ;                                        // Monaghan AV x Balsara (:1121-1128)
+        {
+            const float hB = 0.5f * (hi + hj), cB = 0.5f * (csI + csJ), rB = 0.5f * (rhoI + rhoJ);
+            const float muIJ = __fdividef(hB * vDotR, r2 + 0.01f * hB * hB);
+            const float t = __fdividef(-1.0f * cB * muIJ + 2.0f * muIJ * muIJ, rB) * (0.5f * (fBalI + fBalJ));
+            piIJ = (vDotR < 0.0f) ? t : 0.0f;
+        }
+        float tens = 0.0f;                                 // tensile correction (:1130-1142)
+        const float Rj = b4.w;
+        if (Ri + Rj > 0.0f) {
+            const float Hb = 0.5f * (Hi + Hj);
+            if (r < Hb) {
+                const float qb = __fdividef(r, Hb), om = 1.0f - qb, om2 = om * om;
+                const float fr = (om2 * om2 * (1.0f + 4.0f * qb)) * (1.0f / 0.6328125f);
+                const float fr2 = fr * fr;
+                tens = (Ri + Rj) * (fr2 * fr2);
+            }
+        }
+        const float iso = -mj * ((pOverRho2I + pOverRho2J) + piIJ + tens);
+        axS += iso * gx; ayS += iso * gy; azS += iso * gz;
+        duP += mj * vDotG;
+        duAv += 0.5f * mj * piIJ * vDotG;
+        duT += 0.5f * mj * tens * vDotG;
+        const float tXX = sXXr + b3.x, tYY = sYYr + b3.y, tZZ = sZZr + b3.z, tXY = sXYr + b3.w;
+        const float tXZ = sXZr + b4.x, tYZ = sYZr + b4.y;
+        axS += mj * (tXX * gx + tXY * gy + tXZ * gz);      // deviatoric stress (:1161-1163)
+        ayS += mj * (tXY * gx + tYY * gy + tYZ * gz);
+        azS += mj * (tXZ * gx + tYZ * gy + tZZ * gz);
+        const float wx = -dvx, wy = -dvy, wz = -dvz;
+        duS += mj * ((sXXi * wx + sXYi * wy + sXZi * wz) * gx + (sXYi * wx + sYYi * wy + sYZi * wz) * gy +
+                     (sXZi * wx + sYZi * wy + sZZi * wz) * gz);
+        const float gxi = gI * dx, gyi = gI * dy, gzi = gI * dz;   // velocity gradient (:1173-1179)
+        gXX += volJ * wx * gxi; gXY += volJ * wx * gyi; gXZ += volJ * wx * gzi;
+        gYX += volJ * wy * gxi; gYY += volJ * wy * gyi; gYZ += volJ * wy * gzi;
+        gZX += volJ * wz * gxi; gZY += volJ * wz * gyi; gZZ += volJ * wz * gzi;
+    };
     if (n >= 2u) {
-        // records in 32-byte pieces: {q0, q1} for every candidate (one sector),
-        // {q2, q3} and {q4, q5} for the candidates in range
-        forEachCandidatePrefetched(w, i, [&](uint32_t j) { return ldg256(&R[kRec2Width * static_cast<size_t>(j)]); },
-                                   [&](uint32_t j, const F8& q01) {
-            const float4 b0 = q01.a;
-            const float dx = __fsub_rn(xi, b0.x), dy = __fsub_rn(yi, b0.y), dz = __fsub_rn(zi, b0.z);
-            const float r2 = len2Engine(dx, dy, dz);
-            const float hj = b0.w, Hj = 2.0f * hj;
-            const float Hm = fmaxf(Hi, Hj);
-            if (!(r2 < __fmul_rn(Hm, Hm))) return;          // sph_gravity.cu:1071
-            ++nPairs;
-            const F8 q23 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 2]);
-            const F8 q45 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 4]);
-            const float4 b1 = q01.b, b2 = q23.a, b3 = q23.b, b4 = q45.a, b5 = q45.b;
-            const float mj = b1.w, rhoJ = b2.x, pOverRho2J = b2.y, csJ = b2.z, fBalJ = b2.w;
-            const float volJ = b5.x;
-            const float dvx = vxi - b1.x, dvy = vyi - b1.y, dvz = vzi - b1.z;
-            const float vDotR = dvx * dx + dvy * dy + dvz * dz;
-            const float r = sqrtf(r2);
-            const float gI = wendlandC2GradI(r, Hi, invHi, gradNormI), gJ = wendlandC2GradI(r, Hj, b5.w, b5.y);
-            const float gb = 0.5f * (gI + gJ);
-            const float gx = gb * dx, gy = gb * dy, gz = gb * dz;
-            const float vDotG = dvx * gx + dvy * gy + dvz * gz;
-            drC += volJ * vDotG;                               // continuity (:1114)
-            // The delta-SPH and viscosity terms are evaluated for every pair in
-            // range and kept by a select (the engine's conditions, the same
-            // values): as branches they cost pass 2 11 % at 1M.
-            {                                                  // delta-SPH diffusion (:1115-1119)
-                const float rDotG = -(dx * gx + dy * gy + dz * gz);
-                const float dd = r2 + 0.01f * Hi * Hi;
-                const float t = drD + volJ * (2.0f * (rhoJ - rhoI) / dd) * rDotG;
-                drD = (__float_as_int(b4.z) == matI) ? t : drD;
-            }
-            float piIJ;                                        // Monaghan AV x Balsara (:1121-1128)
-            {
-                const float hB = 0.5f * (hi + hj), cB = 0.5f * (csI + csJ), rB = 0.5f * (rhoI + rhoJ);
-                const float muIJ = __fdividef(hB * vDotR, r2 + 0.01f * hB * hB);
-                const float t = __fdividef(-1.0f * cB * muIJ + 2.0f * muIJ * muIJ, rB) * (0.5f * (fBalI + fBalJ));
-                piIJ = (vDotR < 0.0f) ? t : 0.0f;
-            }
-            float tens = 0.0f;                                 // tensile correction (:1130-1142)
-            const float Rj = b4.w;
-            if (Ri + Rj > 0.0f) {
-                const float Hb = 0.5f * (Hi + Hj);
-                if (r < Hb) {
-                    const float qb = __fdividef(r, Hb), om = 1.0f - qb, om2 = om * om;
-                    const float fr = (om2 * om2 * (1.0f + 4.0f * qb)) * (1.0f / 0.6328125f);
-                    const float fr2 = fr * fr;
-                    tens = (Ri + Rj) * (fr2 * fr2);
-                }
-            }
-            const float iso = -mj * ((pOverRho2I + pOverRho2J) + piIJ + tens);
-            axS += iso * gx; ayS += iso * gy; azS += iso * gz;
-            duP += mj * vDotG;
-            duAv += 0.5f * mj * piIJ * vDotG;
-            duT += 0.5f * mj * tens * vDotG;
-            const float tXX = sXXr + b3.x, tYY = sYYr + b3.y, tZZ = sZZr + b3.z, tXY = sXYr + b3.w;
-            const float tXZ = sXZr + b4.x, tYZ = sYZr + b4.y;
-            axS += mj * (tXX * gx + tXY * gy + tXZ * gz);      // deviatoric stress (:1161-1163)
-            ayS += mj * (tXY * gx + tYY * gy + tYZ * gz);
-            azS += mj * (tXZ * gx + tYZ * gy + tZZ * gz);
-            const float wx = -dvx, wy = -dvy, wz = -dvz;
-            duS += mj * ((sXXi * wx + sXYi * wy + sXZi * wz) * gx + (sXYi * wx + sYYi * wy + sYZi * wz) * gy +
-                         (sXZi * wx + sYZi * wy + sZZi * wz) * gz);
-            const float gxi = gI * dx, gyi = gI * dy, gzi = gI * dz;   // velocity gradient (:1173-1179)
-            gXX += volJ * wx * gxi; gXY += volJ * wx * gyi; gXZ += volJ * wx * gzi;
-            gYX += volJ * wy * gxi; gYY += volJ * wy * gyi; gYZ += volJ * wy * gzi;
-            gZX += volJ * wz * gxi; gZY += volJ * wz * gyi; gZZ += volJ * wz * gzi;
-        });
+        forEachListed<kLanes>(l, sub, first, tested);
+        if (walk && sub == 0u) walkNeighbors(w, i, [&](uint32_t j) { tested(j, first(j)); });
     }
+    if constexpr (kLanes > 1) {
+        sumLanes<kLanes>(axS); sumLanes<kLanes>(ayS); sumLanes<kLanes>(azS);
+        sumLanes<kLanes>(drC); sumLanes<kLanes>(drD);
+        sumLanes<kLanes>(duP); sumLanes<kLanes>(duAv); sumLanes<kLanes>(duT); sumLanes<kLanes>(duS);
+        sumLanes<kLanes>(gXX); sumLanes<kLanes>(gXY); sumLanes<kLanes>(gXZ);
+        sumLanes<kLanes>(gYX); sumLanes<kLanes>(gYY); sumLanes<kLanes>(gYZ);
+        sumLanes<kLanes>(gZX); sumLanes<kLanes>(gZY); sumLanes<kLanes>(gZZ);
+        sumLanes<kLanes>(nPairs);
+    }
+    if (sub != 0u || !write) return;
+    const float pI = effectivePressure(__ldg(&p.pressure[i]), __ldg(&p.phaseId[i]));   // the record's P_eff
+    const float tempI = __ldg(&p.tempK[i]);
+    const float damI = __ldg(&p.damage[i]);
+    const float fSurf = __ldg(&p.surfFactor[i]);
     addCount(w.status, kCntPass2Pairs, nPairs);
     p.accX[i] += axS;                                          // sph_gravity.cu:1213-1218
     p.accY[i] += ayS;
@@ -646,70 +788,136 @@ __global__ void __launch_bounds__(128, 4) pass2Kernel(AstraeaParticles p, Work w
     }
 }
 
+template <int kLanes>
+__global__ void __launch_bounds__(kPassThreads, 4) pass2Kernel(AstraeaParticles p, Work w, uint32_t n,
+                                                              const uint32_t* livingFlags) {
+    chained();
+    if (blockIdx.x < kHeavyBlocks) {
+        const uint32_t lane = threadIdx.x & 31u, total = heavyCount(w);
+        for (uint32_t e = blockIdx.x * (kPassThreads / 32u) + (threadIdx.x >> 5); e < total; e += kHeavyWarps) {
+            const uint4 h = __ldg(&w.heavy[e]);
+            if (h.z != 0u) pass2Particle<32>(p, w, n, h.x, List{w.pool + h.y, 1u, h.z}, lane, false, true, livingFlags);
+        }
+        return;
+    }
+    const uint32_t t = (blockIdx.x - kHeavyBlocks) * kPassThreads + threadIdx.x;
+    const uint32_t i = min(t / kLanes, n - 1u), c = __ldg(&w.nbrCount[i]);
+    if (kLanes == 1 && t >= n) return;
+    const bool listed = c <= w.maxNbr;
+    pass2Particle<kLanes>(p, w, n, i, listOf(w, i, listed ? c : 0u), t % kLanes, !listed && c != kHeavyMark,
+                          t / kLanes < n && c != kHeavyMark, livingFlags);
+}
+
 // ----------------------------------------------------------------- drift ---
 // XSPH position update (sph_gravity.cu:1376-1489).  Neighbour positions come
-// from the leaf records (the positions before this drift), so no thread reads
+// from the drift records (the positions before this drift), so no thread reads
 // a position another thread is moving.  The position add is done in FP64.
-__global__ void __launch_bounds__(128) driftKernel(AstraeaParticles p, Work w, uint32_t n, const float* dtDev,
-                                                   float dtHost, bool useList, bool toScratch,
-                                                   uint32_t* boundsWords) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float mn[3] = {1.0e30f, 1.0e30f, 1.0e30f}, mx[3] = {-1.0e30f, -1.0e30f, -1.0e30f};
-    if (i < n) {
-        const float dt = (dtDev != nullptr) ? *dtDev : dtHost;
-        const F8 rec = ldg256(&w.drift[i].a);
-        const float4 me = rec.a, vr = rec.b;               // {x, y, z, H}, {vx, vy, vz, rho}
-        const float Hi = me.w;
-        const float normI = __ldg(&w.driftAux[i]).y;
-        const float invHi = 1.0f / Hi;
-        const float rhoI = fmaxf(vr.w, 1.0e-9f);
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-        uint32_t nPairs = 0;
-        if (useList && n >= 2u) {
-            // one 32-byte record per candidate: {x, y, z, H}, {vx, vy, vz, rho}
-            forEachCandidatePrefetched(w, i, [&](uint32_t j) { return ldg256(&w.drift[j].a); }, [&](uint32_t j, const F8& rj) {
-                const float4 q = rj.a;
-                const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
-                const float r2 = len2Engine(dx, dy, dz);
-                const float Hj = q.w;
-                const float Hm = fmaxf(Hi, Hj);
-                if (!(r2 < __fmul_rn(Hm, Hm))) return;
-                ++nPairs;
-                const float4 vj = rj.b;
-                const float2 aj = __ldg(&w.driftAux[j]);          // {m, Wendland norm of H_j}
-                const float r = sqrtf(r2);
-                const float wb = 0.5f * (wendlandC2I(r, Hi, invHi, normI) + wendlandC2N(r, Hj, aj.y));
-                const float rb = 0.5f * (rhoI + fmaxf(vj.w, 1.0e-9f));
-                const float co = __fdividef(aj.x, rb) * wb;
-                sx += co * (vj.x - vr.x);
-                sy += co * (vj.y - vr.y);
-                sz += co * (vj.z - vr.z);
-            });
-        }
-        addCount(w.status, kCntDriftPairs, nPairs);
-        const double d = static_cast<double>(dt);
-        const float nx = static_cast<float>(static_cast<double>(me.x) + d * (static_cast<double>(vr.x) + 0.25 * static_cast<double>(sx)));
-        const float ny = static_cast<float>(static_cast<double>(me.y) + d * (static_cast<double>(vr.y) + 0.25 * static_cast<double>(sy)));
-        const float nz = static_cast<float>(static_cast<double>(me.z) + d * (static_cast<double>(vr.z) + 0.25 * static_cast<double>(sz)));
-        if (toScratch) {
-            w.driftPos[i] = make_float4(nx, ny, nz, 0.0f);
-        } else {
-            p.posX[i] = nx; p.posY[i] = ny; p.posZ[i] = nz;
-        }
-        mn[0] = mx[0] = nx; mn[1] = mx[1] = ny; mn[2] = mx[2] = nz;
+struct DriftArgs {
+    const float* dtDev;
+    float dtHost;
+    bool useList, toScratch;
+};
+template <int kLanes>
+__device__ __forceinline__ void driftParticle(const AstraeaParticles& p, const Work& w, uint32_t n, uint32_t i,
+                                              const List& l, uint32_t sub, bool walk, bool write, const DriftArgs& a,
+                                              float (&at)[3]) {
+    const float dt = (a.dtDev != nullptr) ? *a.dtDev : a.dtHost;
+    const F8 rec = ldg256(&w.drift[i].a);
+    const float4 me = rec.a, vr = rec.b;               // {x, y, z, H}, {vx, vy, vz, rho}
+    const float Hi = me.w;
+    const float invHi = __ldg(&w.driftAux[i]).y;
+    const float normI = wendlandNorm(Hi);
+    const float rhoI = fmaxf(vr.w, 1.0e-9f);
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    uint32_t nPairs = 0;
+    // one 32-byte record per candidate: {x, y, z, H}, {vx, vy, vz, rho}, and {m, 1 / H} beside it
+    struct Rec { F8 r; float2 aux; };
+    auto load = [&](uint32_t j) { return Rec{ldg256(&w.drift[j].a), __ldg(&w.driftAux[j])}; };
+    auto body = [&](uint32_t, const Rec& both) {
+        const F8& rj = both.r;
+        const float4 q = rj.a;
+        const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
+        const float r2 = len2Engine(dx, dy, dz);
+        const float Hm = fmaxf(Hi, q.w);
+        if (!(r2 < __fmul_rn(Hm, Hm))) return;
+        ++nPairs;
+        const float2 aj = both.aux;
+        const float4 vj = rj.b;
+        const float r = sqrtf(r2);
+        const float normJ = (aj.y * aj.y) * (aj.y * (21.0f / (2.0f * kPiF)));
+        const float wb = 0.5f * (wendlandC2I(r, Hi, invHi, normI) + wendlandC2I(r, q.w, aj.y, normJ));
+        const float rb = 0.5f * (rhoI + fmaxf(vj.w, 1.0e-9f));
+        const float co = __fdividef(aj.x, rb) * wb;
+        sx += co * (vj.x - vr.x);
+        sy += co * (vj.y - vr.y);
+        sz += co * (vj.z - vr.z);
+    };
+    if (a.useList && n >= 2u) {
+        forEachListed<kLanes>(l, sub, load, body);
+        if (walk && sub == 0u) walkNeighbors(w, i, [&](uint32_t j) { body(j, load(j)); });
     }
-    if (boundsWords != nullptr) blockBoundsToWords(mn, mx, boundsWords);
+    if constexpr (kLanes > 1) {
+        sumLanes<kLanes>(sx); sumLanes<kLanes>(sy); sumLanes<kLanes>(sz); sumLanes<kLanes>(nPairs);
+    }
+    if (sub != 0u || !write) return;
+    addCount(w.status, kCntDriftPairs, nPairs);
+    const double d = static_cast<double>(dt);
+    const float nx = static_cast<float>(static_cast<double>(me.x) + d * (static_cast<double>(vr.x) + 0.25 * static_cast<double>(sx)));
+    const float ny = static_cast<float>(static_cast<double>(me.y) + d * (static_cast<double>(vr.y) + 0.25 * static_cast<double>(sy)));
+    const float nz = static_cast<float>(static_cast<double>(me.z) + d * (static_cast<double>(vr.z) + 0.25 * static_cast<double>(sz)));
+    if (a.toScratch) {
+        w.driftPos[i] = make_float4(nx, ny, nz, 0.0f);
+    } else {
+        p.posX[i] = nx; p.posY[i] = ny; p.posZ[i] = nz;
+    }
+    at[0] = nx; at[1] = ny; at[2] = nz;
+}
+
+// 7 blocks per SM (72 registers, 3 words spilled): 295 us at 1M, 6 blocks 319, 8 blocks
+// (80 registers' worth of spills) 340.  The {m, 1 / H} pair is loaded with the
+// record, before it is known whether the candidate is in range: loaded after the
+// test, its latency stood in every pair (354).  With 1 / H there instead of the
+// norm of H, a division less per pair.
+template <int kLanes>
+__global__ void __launch_bounds__(kPassThreads, 7) driftKernel(AstraeaParticles p, Work w, uint32_t n, DriftArgs a,
+                                                           uint32_t* boundsWords) {
+    chained();
+    if (blockIdx.x < kHeavyBlocks) {
+        const uint32_t lane = threadIdx.x & 31u, total = a.useList ? heavyCount(w) : 0u;
+        for (uint32_t e = blockIdx.x * (kPassThreads / 32u) + (threadIdx.x >> 5); e < total; e += kHeavyWarps) {
+            const uint4 h = __ldg(&w.heavy[e]);
+            float at[3];
+            if (h.z != 0u) driftParticle<32>(p, w, n, h.x, List{w.pool + h.y, 1u, h.z}, lane, false, true, a, at);
+            if (h.z != 0u && lane == 0u && boundsWords != nullptr)
+                for (int k = 0; k < 3; ++k) {
+                    atomicMin(&boundsWords[kWBounds + k], orderedFromFloat(fminf(at[k], 1.0e30f)));
+                    atomicMax(&boundsWords[kWBounds + 3 + k], orderedFromFloat(fmaxf(at[k], -1.0e30f)));
+                }
+        }
+        return;
+    }
+    const uint32_t t = (blockIdx.x - kHeavyBlocks) * kPassThreads + threadIdx.x;
+    const uint32_t i = min(t / kLanes, n - 1u), c = a.useList ? __ldg(&w.nbrCount[i]) : 0u;
+    const bool listed = c <= w.maxNbr, write = t / kLanes < n && c != kHeavyMark;
+    float at[3];
+    if (kLanes > 1 || t < n)
+        driftParticle<kLanes>(p, w, n, i, listOf(w, i, listed ? c : 0u), t % kLanes, !listed && c != kHeavyMark, write, a, at);
+    if (boundsWords == nullptr) return;
+    const bool own = write && t % kLanes == 0u;          // `at` was set
+    const float mn[3] = {own ? at[0] : 1.0e30f, own ? at[1] : 1.0e30f, own ? at[2] : 1.0e30f};
+    const float mx[3] = {own ? at[0] : -1.0e30f, own ? at[1] : -1.0e30f, own ? at[2] : -1.0e30f};
+    blockBoundsToWords(mn, mx, boundsWords);
 }
 
 inline unsigned gridFor(uint32_t n, int block) { return static_cast<unsigned>((n + block - 1) / block); }
 
 }  // namespace
 
-cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_t st, int warps) {
+cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_t st, int warps, bool armed) {
     if (n == 0) return cudaSuccess;
     const uint32_t groups = (n + 31u) / 32u;
-    uint32_t* counter = w.words + kWNbrCounter;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
+    uint32_t* counter = w.words + kWNbrCounter;          // with the pool's words behind it
+    cudaError_t e = armed ? cudaSuccess : cudaMemsetAsync(counter, 0, 4 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     using NbFn = void (*)(Work, uint32_t, uint32_t, uint32_t*);
     const int wps = (warps == 2 || warps == 8) ? warps : kNbWarps;
@@ -720,28 +928,46 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(std::max(1, perSm) * sms),
                                                (groups + wps - 1) / wps);
-    kernel<<<blocks, wps * 32, 0, st>>>(w, n, groups, counter);
-    return cudaGetLastError();
+    e = launchChained(kernel, blocks, static_cast<uint32_t>(wps * 32), st, w, n, groups, counter);
+    if (e != cudaSuccess) return e;
+    return launchChained(poolListsKernel, static_cast<uint32_t>(std::max(1, sms)), kPoolWarps * 32, st, w, n);
 }
+
+// Lanes per particle of the SPH passes: as many as keep all of the launch's
+// threads resident at once (`wave`: blocks per SM x 128 x 152 SMs).  Below that
+// a launch lasts as long as one thread's list; above it a lane more per particle
+// only adds sums and partial last fours.  Drift / pass 1 / pass 2 with 1, 2, 4
+// lanes, us: n = 16k 41.6 / 26.6 / 45.2, 25.9 / 18.4 / 30.7, 19.4 / 15.4 / 26.6
+// (8 lanes: 24.6 / 18.4 / 30.7); 32k 39.4 / 27.1 / 48.6, 27.7 / 20.5 / 38.9,
+// 31.8 / 23.1 / 43.0; 50k 40.0 / 28.7 / 53.2, 30.8 / 25.1 / 59.9, 36.9 / 28.7 /
+// 59.9; 70k 44.2 / 31.7 / 62.0, 47.9 / 34.8 / 65.5; 200k 87.6 / 63.0 / 164,
+// 95.0 / 70.1 / 173.
+constexpr uint32_t kWave6 = 6u * 128u * 152u, kWave4 = 4u * 128u * 152u;
+static uint32_t passBlocks(uint32_t n, int lanes) { return kHeavyBlocks + gridFor(n, static_cast<int>(kPassThreads) / lanes); }
+static int lanesFor(uint32_t n, uint32_t wave) { return n <= wave / 4u ? 4 : (n <= wave / 2u ? 2 : 1); }
 
 cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    pass1Kernel<<<gridFor(n, 128), 128, 0, st>>>(p, w, n);
-    return cudaGetLastError();
+    const int lanes = lanesFor(n, kWave6);
+    const auto kernel = lanes == 4 ? pass1Kernel<4> : (lanes == 2 ? pass1Kernel<2> : pass1Kernel<1>);
+    return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n);
 }
 
 cudaError_t launchPass2(const AstraeaParticles& p, const Work& w, uint32_t n, const uint32_t* livingFlags,
                         cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    pass2Kernel<<<gridFor(n, 128), 128, 0, st>>>(p, w, n, livingFlags);
-    return cudaGetLastError();
+    const int lanes = lanesFor(n, kWave4);
+    const auto kernel = lanes == 4 ? pass2Kernel<4> : (lanes == 2 ? pass2Kernel<2> : pass2Kernel<1>);
+    return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n, livingFlags);
 }
 
 cudaError_t launchDrift(const AstraeaParticles& p, const Work& w, uint32_t n, const float* dtDev, float dtHost,
                         bool useList, bool toScratch, uint32_t* boundsWords, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    driftKernel<<<gridFor(n, 128), 128, 0, st>>>(p, w, n, dtDev, dtHost, useList, toScratch, boundsWords);
-    return cudaGetLastError();
+    const int lanes = lanesFor(n, kWave6);
+    const auto kernel = lanes == 4 ? driftKernel<4> : (lanes == 2 ? driftKernel<2> : driftKernel<1>);
+    return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n,
+                         DriftArgs{dtDev, dtHost, useList, toScratch}, boundsWords);
 }
 
 }  // namespace astraea_gb300

@@ -542,3 +542,40 @@ def test_gravity_walk_of_large_scenes(n, theta):
     assert flags == 0 and counters["gravity_interactions"] == int(counts.astype(np.int64).sum())
     for f in a:
         assert rel_rms(a[f], b[f]) < TOL, f
+
+
+@pytest.mark.parametrize("n", [45, 19_456, 19_457, 29_185, 38_913, 58_369])
+def test_sph_passes_lanes_and_long_lists(n):
+    """Sizes on both sides of each change in the lanes per particle, with every
+    1500th particle's h so large that its neighbours exceed a list (they are
+    kept in the shared pool): pass 1, pass 2 and the drift against the oracle,
+    within the parity bound."""
+    st = c1_state(n_t=n - n // 4, n_i=n // 4)
+    st["h"][::1500] *= 4.0
+    p, alt, bvh = gpu_setup(st)
+    o = oracle.Oracle(st)
+    engine.reset_device_status()
+    engine.clear_stats(p)
+    o.clear_stats()
+    engine.sort_and_build_bvh(p, alt, bvh)
+    o.sort_and_build()
+    engine.sph_pass1_neighbors(p, bvh)
+    o.pass1()
+    engine.evaluate_eos(p)
+    o.eos()
+    engine.sph_pass2_forces(p, bvh)
+    o.pass2()
+    g, c = p.download(), o.state()
+    for f in ("h", "shepardC", "surfFactor", "divV", "curlVX", "accX", "accY", "accZ", "drhoDt", "duDt", "dSXX", "dSXY"):
+        assert rel_rms(g[f], c[f]) < TOL or np.allclose(g[f], c[f], atol=1e-12), (f, rel_rms(g[f], c[f]))
+    p.upload(c)
+    engine.leapfrog_drift(p, 1.0e-2, bvh)
+    o.drift(1.0e-2)
+    g, d = p.download(), o.state()
+    for f in ("posX", "posY", "posZ"):
+        moved = d[f].astype(np.float64) - c[f]
+        ulp = np.spacing(np.abs(c[f]).max())             # positions are stored in FP32
+        assert np.max(np.abs((g[f].astype(np.float64) - c[f]) - moved)) <= ulp + 1e-5 * np.abs(moved).max(), f
+    flags, counters = engine.read_device_status()
+    assert counters["fallback_walks"] == 0
+    assert bool(flags & abi.DEVFLAG_NEIGHBOR_OVERFLOW) == (n > 1000)
