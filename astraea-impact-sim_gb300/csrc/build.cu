@@ -19,6 +19,7 @@ namespace {
 
 // ------------------------------------------------------------- bounds ----
 __global__ void initBoundsKernel(uint32_t* words) {
+    chained();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const uint32_t hi = orderedFromFloat(1.0e30f), lo = orderedFromFloat(-1.0e30f);
         words[kWBounds + 0] = hi; words[kWBounds + 1] = hi; words[kWBounds + 2] = hi;
@@ -29,6 +30,7 @@ __global__ void initBoundsKernel(uint32_t* words) {
 
 __global__ void __launch_bounds__(256) boundsKernel(const float* __restrict__ x, const float* __restrict__ y,
                                                     const float* __restrict__ z, uint32_t n, uint32_t* words) {
+    chained();
     float mn[3] = {1.0e30f, 1.0e30f, 1.0e30f}, mx[3] = {-1.0e30f, -1.0e30f, -1.0e30f};
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -71,6 +73,7 @@ template <bool kAllFields>
 __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticles p, AstraeaParticles alt,
                                                                  AstraeaRadixBvh bvh, const float4* __restrict__ posSrc,
                                                                  Work w, uint32_t n, uint32_t* livingFlags) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0u) armNeighborBuild(w);
     bool tracer = false, intact = false;
@@ -167,6 +170,7 @@ __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticle
 // Leaf records from the caller's current SoA (used before tree walks that are
 // not preceded by this library's own permutation).
 __global__ void __launch_bounds__(256) refreshLeavesKernel(AstraeaParticles p, Work w, uint32_t n, bool withVelRho) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (i == 0u) armNeighborBuild(w);
@@ -412,6 +416,7 @@ __device__ void writeNode(const AstraeaRadixBvh& bvh, const Work& w, int node, c
 
 template <bool kMoments>
 __global__ void __launch_bounds__(kRefitBlock) refitBlockKernel(AstraeaRadixBvh bvh, Work w, uint32_t n) {
+    chained();
     constexpr int kW = kMoments ? kMomW : 4;
     constexpr int kWarps = kRefitBlock / 32;
     __shared__ Ext8 wPre[kRefitBlock], wSuf[kRefitBlock];   // warp-inclusive prefix / suffix extremes
@@ -522,6 +527,7 @@ __global__ void __launch_bounds__(kRefitBlock) refitBlockKernel(AstraeaRadixBvh 
 // loads in flight while the current one is scanned.
 template <bool kMoments>
 __global__ void __launch_bounds__(1024) refitScanKernel(Work w, uint32_t nb) {
+    chained();
     constexpr int kW = kMoments ? kMomW : 4;
     __shared__ long long warpSum[kW][32];
     __shared__ long long carry[kW];
@@ -581,6 +587,7 @@ __global__ void __launch_bounds__(1024) refitScanKernel(Work w, uint32_t nb) {
 // s = 2^(lev-1) and A_k = T[lev-1][b + k s], T[lev-1+j][b] joins
 // A_0 .. A_(2^j - 1) (it covers blocks b .. b + 2^j s - 1), j = 1 .. count.
 __global__ void __launch_bounds__(256) refitLevelKernel(Work w, uint32_t nb, uint32_t lev, uint32_t count) {
+    chained();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t s = 1u << (lev - 1);
     if (b + 2u * s > nb) return;
@@ -602,6 +609,7 @@ __global__ void __launch_bounds__(256) refitLevelKernel(Work w, uint32_t nb, uin
 // Nodes whose range spans blocks.
 template <bool kMoments>
 __global__ void __launch_bounds__(256) refitCrossKernel(AstraeaRadixBvh bvh, Work w, uint32_t n, uint32_t nb) {
+    chained();
     constexpr int kW = kMoments ? kMomW : 4;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i + 1u >= n) return;
@@ -636,30 +644,26 @@ inline unsigned gridFor(uint32_t n, int block) { return static_cast<unsigned>((n
 }  // namespace
 
 cudaError_t launchInitBounds(uint32_t* words, cudaStream_t st) {
-    initBoundsKernel<<<1, 32, 0, st>>>(words);
-    return cudaGetLastError();
+    return launchChained(initBoundsKernel, 1, 32, st, words);
 }
 
 cudaError_t launchBounds(const AstraeaParticles& p, uint32_t n, uint32_t* words, int sms, cudaStream_t st) {
     const unsigned blocks = min(gridFor(n, 256), static_cast<unsigned>(sms * 4));
-    boundsKernel<<<blocks, 256, 0, st>>>(p.posX, p.posY, p.posZ, n, words);
-    return cudaGetLastError();
+    return launchChained(boundsKernel, blocks, 256, st, p.posX, p.posY, p.posZ, n, words);
 }
 
 cudaError_t launchPermuteLeavesKarras(const AstraeaParticles& p, const AstraeaParticles& alt,
                                       const AstraeaRadixBvh& bvh, const float4* posSrc, const Work& w, uint32_t n,
                                       uint32_t* livingFlags, bool allFields, cudaStream_t st) {
     if (allFields)
-        permuteLeavesKarrasKernel<true><<<gridFor(n, 256), 256, 0, st>>>(p, alt, bvh, posSrc, w, n, livingFlags);
+        return launchChained(permuteLeavesKarrasKernel<true>, gridFor(n, 256), 256, st, p, alt, bvh, posSrc, w, n, livingFlags);
     else
-        permuteLeavesKarrasKernel<false><<<gridFor(n, 256), 256, 0, st>>>(p, alt, bvh, posSrc, w, n, livingFlags);
-    return cudaGetLastError();
+        return launchChained(permuteLeavesKarrasKernel<false>, gridFor(n, 256), 256, st, p, alt, bvh, posSrc, w, n, livingFlags);
 }
 
 cudaError_t launchRefreshLeaves(const AstraeaParticles& p, const Work& w, uint32_t n, bool withVelRho,
                                 cudaStream_t st) {
-    refreshLeavesKernel<<<gridFor(n, 256), 256, 0, st>>>(p, w, n, withVelRho);
-    return cudaGetLastError();
+    return launchChained(refreshLeavesKernel, gridFor(n, 256), 256, st, p, w, n, withVelRho);
 }
 
 uint32_t refitBlocks(uint32_t n) { return (n + kRefitBlock - 1) / kRefitBlock; }
@@ -681,6 +685,7 @@ uint32_t refitLevels(uint32_t nb) {
 // replaced; boxes, h extremes and the quadrupole moments stay the refit's.
 __global__ void __launch_bounds__(256) engineNodeMomentsKernel(AstraeaParticles p, AstraeaRadixBvh bvh, Work w,
                                                                 uint32_t n) {
+    chained();
     const uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
     if (leaf >= n || n < 2u) return;
     auto childRec = [&](int c) {
@@ -726,28 +731,23 @@ __global__ void __launch_bounds__(256) engineNodeMomentsKernel(AstraeaParticles 
 cudaError_t launchEngineNodeMoments(const AstraeaParticles& p, const AstraeaRadixBvh& bvh, const Work& w, uint32_t n,
                                     cudaStream_t st) {
     if (n < 2u) return cudaSuccess;
-    engineNodeMomentsKernel<<<gridFor(n, 256), 256, 0, st>>>(p, bvh, w, n);
-    return cudaGetLastError();
+    return launchChained(engineNodeMomentsKernel, gridFor(n, 256), 256, st, p, bvh, w, n);
 }
 
 cudaError_t launchRefit(const AstraeaRadixBvh& bvh, const Work& w, uint32_t n, bool moments, cudaStream_t st) {
     if (n < 2u) return cudaSuccess;
     const uint32_t nb = refitBlocks(n);
     const uint32_t levels = refitLevels(nb);
-    if (moments) {
-        refitBlockKernel<true><<<nb, kRefitBlock, 0, st>>>(bvh, w, n);
-        refitScanKernel<true><<<1, 1024, 0, st>>>(w, nb);
-    } else {
-        refitBlockKernel<false><<<nb, kRefitBlock, 0, st>>>(bvh, w, n);
-        refitScanKernel<false><<<1, 1024, 0, st>>>(w, nb);
-    }
-    for (uint32_t lev = 1; lev < levels; lev += 3)
-        refitLevelKernel<<<gridFor(nb, 256), 256, 0, st>>>(w, nb, lev, std::min(3u, levels - lev));
-    if (moments)
-        refitCrossKernel<true><<<gridFor(n, 256), 256, 0, st>>>(bvh, w, n, nb);
-    else
-        refitCrossKernel<false><<<gridFor(n, 256), 256, 0, st>>>(bvh, w, n, nb);
-    return cudaGetLastError();
+    cudaError_t e = moments ? launchChained(refitBlockKernel<true>, nb, kRefitBlock, st, bvh, w, n)
+                            : launchChained(refitBlockKernel<false>, nb, kRefitBlock, st, bvh, w, n);
+    if (e == cudaSuccess)
+        e = moments ? launchChained(refitScanKernel<true>, 1, 1024, st, w, nb)
+                    : launchChained(refitScanKernel<false>, 1, 1024, st, w, nb);
+    for (uint32_t lev = 1; lev < levels && e == cudaSuccess; lev += 3)
+        e = launchChained(refitLevelKernel, gridFor(nb, 256), 256, st, w, nb, lev, std::min(3u, levels - lev));
+    if (e != cudaSuccess) return e;
+    return moments ? launchChained(refitCrossKernel<true>, gridFor(n, 256), 256, st, bvh, w, n, nb)
+                   : launchChained(refitCrossKernel<false>, gridFor(n, 256), 256, st, bvh, w, n, nb);
 }
 
 }  // namespace astraea_gb300

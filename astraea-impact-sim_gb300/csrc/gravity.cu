@@ -332,7 +332,9 @@ __device__ __forceinline__ PairRec loadPair(const float4* p) {
 // system: ~180 bytes read and written a node, most of it still in L2 from the
 // refit; 38 us at 1M, where it saves the gravity walk 350.
 __global__ void __launch_bounds__(256) pairNodesKernel(Work w, uint32_t n) {
+    chained();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0u) w.words[kWGroupCounter] = 0u;
     if (p + 1u >= n) return;
     const float4 r1 = __ldg(&w.node[4 * static_cast<size_t>(p) + 1]);
     float v[2][5], farC[2] = {0.0f, 0.0f};
@@ -376,6 +378,7 @@ template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = fa
 __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWarps) gravityKernel(AstraeaParticles p, Work w, uint32_t n,
                                                                  float theta2, uint32_t numGroups,
                                                                  uint32_t* groupCounter, FarCapture ff) {
+    chained();
     static_assert(!kExpand || kQuad, "the group expansion is a quadrupole mode");
     constexpr int kMRing = kQuad ? kGravListQ : kGravList;
     __shared__ GravWarpSmem<kQuad, kExpand, kLearned> smem[kWarps];
@@ -942,6 +945,7 @@ template <bool kInside>
 __global__ void __launch_bounds__(kOrdWarps * 32, 28 / kOrdWarps) gravityOrderedKernel(AstraeaParticles p, Work w, uint32_t n,
                                                                                       float theta2, uint32_t numGroups,
                                                                                       uint32_t* groupCounter) {
+    chained();
     __shared__ OrderedSmem smem[kOrdWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     OrderedSmem& S = smem[warp];
@@ -1151,10 +1155,11 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     const bool checkInside = theta2 > 0.333333f;
     const uint32_t groups = (n + 31u) / 32u;
     uint32_t* counter = w.words + kWGroupCounter;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
+    // The pair kernel also clears the counter.  (The learned mode's fallback,
+    // runIf, walks the records its first walk wrote.)
+    cudaError_t e = n >= 2u && w.runIf == nullptr ? launchChained(pairNodesKernel, (n - 1u + 255u) / 256u, 256, st, w, n)
+                                                  : cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    // (the learned mode's fallback, runIf, walks the records its first walk wrote)
-    if (n >= 2u && w.runIf == nullptr) pairNodesKernel<<<(n - 1u + 255u) / 256u, 256, 0, st>>>(w, n);
     if (n > kOrderedAbove && !quadrupole && far == nullptr && w.runIf == nullptr && w.traceList == nullptr &&
         w.groupCounts == nullptr) {
         const auto ordered = checkInside ? gravityOrderedKernel<true> : gravityOrderedKernel<false>;
@@ -1163,8 +1168,7 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
         if (e != cudaSuccess) return e;
         const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(std::max(1, perSm) * sms),
                                                    (groups + kOrdWarps - 1) / kOrdWarps);
-        ordered<<<blocks, kOrdWarps * 32, 0, st>>>(p, w, n, theta2, groups, counter);
-        return cudaGetLastError();
+        return launchChained(ordered, blocks, kOrdWarps * 32u, st, p, w, n, theta2, groups, counter);
     }
     FarCapture ff{};
     using GravFn = void (*)(AstraeaParticles, Work, uint32_t, float, uint32_t, uint32_t*, FarCapture);
@@ -1208,8 +1212,7 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(std::max(1, perSm) * sms),
                                                (groups + wps - 1) / wps);
-    kernel<<<blocks, wps * 32, 0, st>>>(p, w, n, theta2, groups, counter, ff);
-    return cudaGetLastError();
+    return launchChained(kernel, blocks, static_cast<uint32_t>(wps * 32), st, p, w, n, theta2, groups, counter, ff);
 }
 
 }  // namespace astraea_gb300

@@ -91,6 +91,7 @@ __device__ __forceinline__ void writePass2Record(float4* R, float x, float y, fl
 }
 
 __global__ void __launch_bounds__(256) eosKernel(AstraeaParticles p, Work w, bool withRecords, uint32_t n) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint8_t mat = __ldg(&p.materialId[i]);
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(256) eosKernel(AstraeaParticles p, Work w, boo
 }
 
 __global__ void __launch_bounds__(256) kickKernel(AstraeaParticles p, uint32_t n, KickArgs a) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float halfDt = a.halfDtHost;
     if (a.dtMode == 1) {
@@ -210,6 +212,7 @@ __global__ void __launch_bounds__(256) kickKernel(AstraeaParticles p, uint32_t n
 }
 
 __global__ void __launch_bounds__(256) packPass2Kernel(AstraeaParticles p, Work w, uint32_t n) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float h = fmaxf(__ldg(&p.h[i]), 1.0e-6f);
@@ -225,6 +228,7 @@ __global__ void __launch_bounds__(256) packPass2Kernel(AstraeaParticles p, Work 
 }
 
 __global__ void __launch_bounds__(256) driftPlainKernel(AstraeaParticles p, uint32_t n, float dt) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double d = static_cast<double>(dt);
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(256) driftPlainKernel(AstraeaParticles p, uint
 }
 
 __global__ void setDtSlotsKernel(float* slots, int parity, float prevDt, uint32_t* rawMin) {
+    chained();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         slots[parity] = prevDt;
         slots[parity ^ 1] = 0.0f;
@@ -242,6 +247,7 @@ __global__ void setDtSlotsKernel(float* slots, int parity, float prevDt, uint32_
 }
 
 __global__ void __launch_bounds__(256) reduceDtKernel(AstraeaParticles p, uint32_t n, uint32_t* out) {
+    chained();
     float m = 1.0e30f;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -254,6 +260,7 @@ __global__ void __launch_bounds__(256) reduceDtKernel(AstraeaParticles p, uint32
 }
 
 __global__ void __launch_bounds__(256) clearStatsKernel(AstraeaParticles p, uint32_t n) {
+    chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     p.accX[i] = 0.f; p.accY[i] = 0.f; p.accZ[i] = 0.f;
@@ -270,45 +277,38 @@ inline unsigned gridFor(uint32_t n, int block) { return static_cast<unsigned>((n
 
 cudaError_t launchClearStats(const AstraeaParticles& p, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    clearStatsKernel<<<gridFor(n, 256), 256, 0, st>>>(p, n);
-    return cudaGetLastError();
+    return launchChained(clearStatsKernel, gridFor(n, 256), 256, st, p, n);
 }
 
 cudaError_t launchEos(const AstraeaParticles& p, const Work* w, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     Work none{};
-    eosKernel<<<gridFor(n, 256), 256, 0, st>>>(p, w ? *w : none, w != nullptr, n);
-    return cudaGetLastError();
+    return launchChained(eosKernel, gridFor(n, 256), 256, st, p, w ? *w : none, w != nullptr, n);
 }
 
 cudaError_t launchKick(const AstraeaParticles& p, uint32_t n, const KickArgs& a, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    kickKernel<<<gridFor(n, 256), 256, 0, st>>>(p, n, a);
-    return cudaGetLastError();
+    return launchChained(kickKernel, gridFor(n, 256), 256, st, p, n, a);
 }
 
 cudaError_t launchPackPass2Records(const AstraeaParticles& p, const Work& w, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    packPass2Kernel<<<gridFor(n, 256), 256, 0, st>>>(p, w, n);
-    return cudaGetLastError();
+    return launchChained(packPass2Kernel, gridFor(n, 256), 256, st, p, w, n);
 }
 
 cudaError_t launchDriftPlain(const AstraeaParticles& p, uint32_t n, float dt, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    driftPlainKernel<<<gridFor(n, 256), 256, 0, st>>>(p, n, dt);
-    return cudaGetLastError();
+    return launchChained(driftPlainKernel, gridFor(n, 256), 256, st, p, n, dt);
 }
 
 cudaError_t launchSetDtSlots(float* slots, int parity, float prevDt, uint32_t* rawMin, cudaStream_t st) {
-    setDtSlotsKernel<<<1, 32, 0, st>>>(slots, parity, prevDt, rawMin);
-    return cudaGetLastError();
+    return launchChained(setDtSlotsKernel, 1, 32, st, slots, parity, prevDt, rawMin);
 }
 
 cudaError_t launchReduceDt(const AstraeaParticles& p, uint32_t n, uint32_t* rawMinOut, int sms, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const unsigned blocks = std::min(gridFor(n, 256), static_cast<unsigned>(sms) * 4u);
-    reduceDtKernel<<<blocks, 256, 0, st>>>(p, n, rawMinOut);
-    return cudaGetLastError();
+    return launchChained(reduceDtKernel, blocks, 256, st, p, n, rawMinOut);
 }
 
 }  // namespace astraea_gb300

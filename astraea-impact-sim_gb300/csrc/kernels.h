@@ -27,30 +27,6 @@ __device__ __forceinline__ float warpSumF(float v) {
     return v;
 }
 
-// Programmatic dependent launch: a kernel started by launchChained may have its
-// blocks scheduled once every block of the kernel before it in the stream has
-// begun (or ended), so the launch and the scheduling overlap that kernel's
-// tail.  chained() is the first statement of such a kernel, for every thread: it
-// lets the next kernel in, and returns when everything before is complete and
-// visible, so nothing in the body needs care.
-__device__ __forceinline__ void chained() {
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-template <class... P, class... A>
-cudaError_t launchChained(void (*kernel)(P...), uint32_t grid, uint32_t block, cudaStream_t st, A&&... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 // Reduce each thread's partial AABB over the block and merge it into the
 // ordered-uint bound words with atomics (engine/sph_gravity.cu:300-324).
 // Every thread of the block must call it.

@@ -79,6 +79,7 @@ __device__ __forceinline__ double sumRelax(int slot) {
 
 // COM position and velocity, simulation.cpp:640-660.
 __global__ void __launch_bounds__(kRelaxThreads) relaxMomentsKernel(AstraeaParticles p, uint32_t n) {
+    chained();
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     for (uint32_t i = blockIdx.x * kRelaxThreads + threadIdx.x; i < n; i += gridDim.x * kRelaxThreads) {
         const double m = p.mass[i];
@@ -120,6 +121,7 @@ __device__ __forceinline__ void zeroStrength(const AstraeaParticles& p, uint32_t
 // Recentre, damp, re-anchor, clear strength (simulation.cpp:662-705).
 __global__ void __launch_bounds__(kRelaxThreads) relaxApplyKernel(AstraeaParticles p, uint32_t n,
                                                                   const double* anchorT, uint32_t anchorCount) {
+    chained();
     const uint32_t i = blockIdx.x * kRelaxThreads + threadIdx.x;
     if (i >= n) return;
     const double cx = g_rel.com[0], cy = g_rel.com[1], cz = g_rel.com[2];
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kRelaxThreads) relaxApplyKernel(AstraeaParticl
 // v_rms / v_esc of the relaxed body (simulation.cpp:747-767).
 __global__ void __launch_bounds__(kRelaxThreads) relaxDiagnosticKernel(AstraeaParticles p, uint32_t n,
                                                                        double nominalRadius) {
+    chained();
     double v[2] = {0.0, 0.0};
     double rMax = nominalRadius;
     for (uint32_t i = blockIdx.x * kRelaxThreads + threadIdx.x; i < n; i += gridDim.x * kRelaxThreads) {
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(kRelaxThreads) relaxDiagnosticKernel(AstraeaPa
 // Final thermal re-anchoring and strength reset (simulation.cpp:769-780).
 __global__ void __launch_bounds__(kRelaxThreads) relaxAnchorKernel(AstraeaParticles p, uint32_t n,
                                                                    const double* anchorT, uint32_t anchorCount) {
+    chained();
     const uint32_t i = blockIdx.x * kRelaxThreads + threadIdx.x;
     if (i >= n) return;
     p.u[i] = anchoredU(p, i, anchorT, anchorCount);
@@ -199,9 +203,9 @@ cudaError_t launchRelaxRecentre(const AstraeaParticles& p, uint32_t n, const dou
     if (n == 0) return cudaSuccess;
     cudaError_t e = resetTicket(st);
     if (e != cudaSuccess) return e;
-    relaxMomentsKernel<<<reduceBlocks(n, sms), kRelaxThreads, 0, st>>>(p, n);
-    relaxApplyKernel<<<(n + kRelaxThreads - 1) / kRelaxThreads, kRelaxThreads, 0, st>>>(p, n, anchorT, anchorCount);
-    return cudaGetLastError();
+    e = launchChained(relaxMomentsKernel, reduceBlocks(n, sms), kRelaxThreads, st, p, n);
+    if (e != cudaSuccess) return e;
+    return launchChained(relaxApplyKernel, (n + kRelaxThreads - 1) / kRelaxThreads, kRelaxThreads, st, p, n, anchorT, anchorCount);
 }
 
 cudaError_t launchRelaxDiagnostic(const AstraeaParticles& p, uint32_t n, double nominalRadius, int sms,
@@ -210,8 +214,7 @@ cudaError_t launchRelaxDiagnostic(const AstraeaParticles& p, uint32_t n, double 
     if (n == 0) return cudaSuccess;
     cudaError_t e = resetTicket(st);
     if (e != cudaSuccess) return e;
-    relaxDiagnosticKernel<<<reduceBlocks(n, sms), kRelaxThreads, 0, st>>>(p, n, nominalRadius);
-    e = cudaGetLastError();
+    e = launchChained(relaxDiagnosticKernel, reduceBlocks(n, sms), kRelaxThreads, st, p, n, nominalRadius);
     if (e != cudaSuccess) return e;
     e = cudaMemcpyFromSymbolAsync(hostOut, g_rel, sizeof(double), offsetof(RelaxState, vrmsOverVesc),
                                   cudaMemcpyDeviceToHost, st);
@@ -222,8 +225,7 @@ cudaError_t launchRelaxDiagnostic(const AstraeaParticles& p, uint32_t n, double 
 cudaError_t launchRelaxAnchor(const AstraeaParticles& p, uint32_t n, const double* anchorT, uint32_t anchorCount,
                               cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    relaxAnchorKernel<<<(n + kRelaxThreads - 1) / kRelaxThreads, kRelaxThreads, 0, st>>>(p, n, anchorT, anchorCount);
-    return cudaGetLastError();
+    return launchChained(relaxAnchorKernel, (n + kRelaxThreads - 1) / kRelaxThreads, kRelaxThreads, st, p, n, anchorT, anchorCount);
 }
 
 }  // namespace astraea_gb300

@@ -99,6 +99,7 @@ __device__ __forceinline__ void renderRecord(const AstraeaParticles& p, uint32_t
 
 __global__ void __launch_bounds__(kPackThreads) packRenderKernel(AstraeaParticles p, uint32_t n, uint8_t* records,
                                                                  uint8_t* speed, float sx, float sy, float sz) {
+    chained();
     __shared__ uint32_t tile[5 * kPackThreads];   // stride 5 words: conflict-free
     const uint32_t base = blockIdx.x * kPackThreads;
     const uint32_t i = base + threadIdx.x;
@@ -169,6 +170,7 @@ __device__ __forceinline__ void tracerRecord(const AstraeaParticles& p, uint32_t
 __global__ void __launch_bounds__(kPackThreads) extractTracersKernel(AstraeaParticles p, uint32_t n, uint8_t* records,
                                                                      uint32_t tracerCount, float lx, float ly,
                                                                      float lz, float sx, float sy, float sz) {
+    chained();
     const uint32_t i = blockIdx.x * kPackThreads + threadIdx.x;
     if (i >= n) return;
     const int32_t tIdx = __ldg(&p.tracerIndex[i]);
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(kPackThreads) extractTracersKernel(AstraeaPart
 }
 
 __global__ void writeHeaderKernel(uint8_t* frame, PclsHeaderWords h) {
+    chained();
     const int k = threadIdx.x;
     if (k < 10) {
         const uint32_t v = h.w[k];
@@ -204,8 +207,7 @@ __global__ void writeHeaderKernel(uint8_t* frame, PclsHeaderWords h) {
 cudaError_t launchPackRender(const AstraeaParticles& p, uint32_t n, uint8_t* records, uint8_t* speed, float sx, float sy,
                              float sz, cudaStream_t st) {
     if (n == 0 || records == nullptr) return cudaSuccess;
-    packRenderKernel<<<(n + kPackThreads - 1) / kPackThreads, kPackThreads, 0, st>>>(p, n, records, speed, sx, sy, sz);
-    return cudaGetLastError();
+    return launchChained(packRenderKernel, (n + kPackThreads - 1) / kPackThreads, kPackThreads, st, p, n, records, speed, sx, sy, sz);
 }
 
 cudaError_t launchExtractTracers(const AstraeaParticles& p, uint32_t n, uint8_t* records, uint32_t tracerCount,
@@ -213,14 +215,11 @@ cudaError_t launchExtractTracers(const AstraeaParticles& p, uint32_t n, uint8_t*
     if (tracerCount == 0 || records == nullptr) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(records, 0, static_cast<size_t>(tracerCount) * 40u, st);
     if (e != cudaSuccess || n == 0) return e;
-    extractTracersKernel<<<(n + kPackThreads - 1) / kPackThreads, kPackThreads, 0, st>>>(p, n, records, tracerCount,
-                                                                                         lx, ly, lz, sx, sy, sz);
-    return cudaGetLastError();
+    return launchChained(extractTracersKernel, (n + kPackThreads - 1) / kPackThreads, kPackThreads, st, p, n, records, tracerCount, lx, ly, lz, sx, sy, sz);
 }
 
 cudaError_t launchWriteHeader(uint8_t* frame, const PclsHeaderWords& h, cudaStream_t st) {
-    writeHeaderKernel<<<1, 32, 0, st>>>(frame, h);
-    return cudaGetLastError();
+    return launchChained(writeHeaderKernel, 1, 32, st, frame, h);
 }
 
 }  // namespace astraea_gb300

@@ -65,6 +65,7 @@ template <bool kMorton>
 __global__ void __launch_bounds__(256) histogramKernel(const uint64_t* __restrict__ keysIn, MortonSource ms,
                                                        uint64_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut,
                                                        uint32_t n, int passes, uint32_t* __restrict__ hist) {
+    chained();
     __shared__ uint32_t sh[kSortMaxPasses][kSortBins];
     __shared__ float sB[6];
     __shared__ float sInv[3];
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kSortThreads, kItems <= 4 ? 3 : 2) onesweepKer
                                                                uint32_t* __restrict__ tileCounter,
                                                                uint32_t* __restrict__ lookback, DevStatus* status,
                                                                uint32_t spinLimit) {
+    chained();
     extern __shared__ __align__(16) unsigned char smemRaw[];
     SortSmem<kItems>& s = *reinterpret_cast<SortSmem<kItems>*>(smemRaw);
     const int t = threadIdx.x;
@@ -400,6 +402,7 @@ template <bool kMorton, int kThreads, int kItems>
 __global__ void __launch_bounds__(kThreads) clusterSortKernel(const uint64_t* keysIn, const uint32_t* valsIn,
                                                               MortonSource ms, uint64_t* keysOut, uint32_t* valsOut,
                                                               uint32_t n, uint32_t chunk, uint32_t magic, int passes) {
+    chained();
     using Smem = ClusterSmem<kThreads, kItems>;
     constexpr int kWarps = Smem::kWarps;
     extern __shared__ __align__(16) unsigned char smemRaw[];
@@ -583,17 +586,19 @@ cudaError_t launchClusterSort(const uint64_t* keysIn, const uint32_t* valsIn, co
     *done = false;
     if (dev < 0 || dev >= 64) return cudaSuccess;
     const auto kernel = clusterSortKernel<kMorton, kThreads, kItems>;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kClusterBlocks;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kClusterBlocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;    // see chained()
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kClusterBlocks);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = sizeof(ClusterSmem<kThreads, kItems>);
     cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     // 0: not asked yet, 1: fits, 2: does not; every thread that asks gets the same answer
     static std::atomic<int> fits[64] = {};
     int f = fits[dev].load(std::memory_order_acquire);
@@ -677,12 +682,11 @@ cudaError_t radixSortPairs(uint64_t* keysA, uint32_t* valsA, uint64_t* keysB, ui
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int hBlocks = static_cast<int>(std::min<uint32_t>((n + 255) / 256, static_cast<uint32_t>(sms) * 4u));
     if (mortonKeys) {
-        histogramKernel<true><<<hBlocks, 256, 0, stream>>>(nullptr, *morton, keysA, valsA, n, passes, hist);
+        e = launchChained(histogramKernel<true>, hBlocks, 256, stream, nullptr, *morton, keysA, valsA, n, passes, hist);
     } else {
         MortonSource none{};
-        histogramKernel<false><<<hBlocks, 256, 0, stream>>>(keysA, none, nullptr, nullptr, n, passes, hist);
+        e = launchChained(histogramKernel<false>, hBlocks, 256, stream, keysA, none, nullptr, nullptr, n, passes, hist);
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
 
     const auto kernel = items == 4 ? onesweepKernel<4> : (items == 8 ? onesweepKernel<8> : onesweepKernel<12>);
@@ -702,10 +706,8 @@ cudaError_t radixSortPairs(uint64_t* keysA, uint32_t* valsA, uint64_t* keysB, ui
     uint64_t* kout = keysB;
     uint32_t* vout = valsB;
     for (int p = 0; p < passes; ++p) {
-        kernel<<<tiles, kSortThreads, smem, stream>>>(kin, vin, kout, vout, n, p, hist, counters + p,
-                                                      look + static_cast<size_t>(p) * tiles * kSortBins, status,
-                                                      spinLimit);
-        e = cudaGetLastError();
+        e = launchChainedSmem(kernel, tiles, kSortThreads, smem, stream, kin, vin, kout, vout, n, p, hist, counters + p,
+                              look + static_cast<size_t>(p) * tiles * kSortBins, status, spinLimit);
         if (e != cudaSuccess) return e;
         std::swap(kin, kout);
         std::swap(vin, vout);

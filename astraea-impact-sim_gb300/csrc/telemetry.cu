@@ -202,6 +202,7 @@ __device__ __forceinline__ void finishRemnant(TelState& s) {
 }
 
 __global__ void __launch_bounds__(kTelThreads) passA(AstraeaParticles p, uint32_t n, double targetRadius) {
+    chained();
     double v[kSlotsA];
 #pragma unroll
     for (int k = 0; k < kSlotsA; ++k) v[k] = 0.0;
@@ -377,6 +378,7 @@ __device__ __forceinline__ TelIn telLoad(const AstraeaParticles& p, uint32_t i) 
 template <bool kWithSpin>
 __global__ void __launch_bounds__(kTelThreads) passRemnant(AstraeaParticles p, uint32_t n, double targetRadius,
                                                            int living) {
+    chained();
     const TelState s = g_state;                                  // written by the previous launch
     if (s.stop) return;
     constexpr int kCnt = kWithSpin ? kSlotsB : kRMR2 + 1;
@@ -490,6 +492,7 @@ __device__ __forceinline__ Verdict diskTest(const Remnant& q, const Rel& d) {
 
 // Final classification (:1176-1230).
 __global__ void __launch_bounds__(kTelThreads) passClassify(AstraeaParticles p, uint32_t n) {
+    chained();
     const TelState s = g_state;
     double v[kSlotsD] = {0.0, 0.0, 0.0, 0.0};
     const double rSoft = s.rSoft;
@@ -547,11 +550,11 @@ cudaError_t launchTelemetry(const AstraeaParticles& p, uint32_t n, double target
     const uint32_t blocks = std::max<uint32_t>(
         1u, std::min<uint32_t>(static_cast<uint32_t>(std::min(2 * sms, kTelMaxBlocks)),
                                (n + kTelThreads - 1) / kTelThreads));
-    passA<<<blocks, kTelThreads, 0, st>>>(p, n, targetRadiusPsu);
-    passRemnant<true><<<blocks, kTelThreads, 0, st>>>(p, n, targetRadiusPsu, livingBodyPresent);
-    for (int it = 1; it < 5; ++it) passRemnant<false><<<blocks, kTelThreads, 0, st>>>(p, n, targetRadiusPsu, 0);
-    passClassify<<<blocks, kTelThreads, 0, st>>>(p, n);
-    e = cudaGetLastError();
+    e = launchChained(passA, blocks, kTelThreads, st, p, n, targetRadiusPsu);
+    if (e == cudaSuccess) e = launchChained(passRemnant<true>, blocks, kTelThreads, st, p, n, targetRadiusPsu, livingBodyPresent);
+    for (int it = 1; it < 5 && e == cudaSuccess; ++it)
+        e = launchChained(passRemnant<false>, blocks, kTelThreads, st, p, n, targetRadiusPsu, 0);
+    if (e == cudaSuccess) e = launchChained(passClassify, blocks, kTelThreads, st, p, n);
     if (e != cudaSuccess) return e;
     e = cudaMemcpyFromSymbolAsync(hostOut, g_out, sizeof(AstraeaTelemetry), 0, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return e;
