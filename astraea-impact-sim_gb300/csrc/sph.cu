@@ -8,9 +8,9 @@
 //     particle, the list of j with r_ij < max(Hs_i, Hs_j) -- a superset of the
 //     pass-1, pass-2 and next-drift neighbour sets (see common.cuh);
 //   * pass 1, pass 2 and the drift work on the lists, re-applying the engine's
-//     exact FP32 range test, one thread per particle in a large scene; in a
-//     small one, whose threads would not fill the GPU, two or four lanes share
-//     a particle's list and add up their sums (lanesFor);
+//     exact FP32 range test, one thread per particle; in a small scene, whose
+//     threads would not fill the GPU, two or four lanes share a particle's list
+//     in pass 1 and the drift and add up their sums (lanesFor);
 //   * neighbour data is read from packed records (pass 1: position + Hs
 //     and velocity + volume m/rho in one 32-byte record; drift: position + H and
 //     velocity + density; pass 2: a 96-byte record written by the EOS
@@ -788,7 +788,11 @@ __device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const W
     }
 }
 
-template <int kLanes>
+// A thread a particle at every size, the terms added in list order: a warp's
+// lanes sharing a list (as in pass 1 and the drift) made it 27 instead of 45 us
+// at 16k, but the other order of the sums moves du/dt and drho/dt by 1e-6 of
+// their norm, and the strength of iron just below its melting point amplifies an
+// ulp of rho a thousandfold.
 __global__ void __launch_bounds__(kPassThreads, 4) pass2Kernel(AstraeaParticles p, Work w, uint32_t n,
                                                               const uint32_t* livingFlags) {
     chained();
@@ -800,12 +804,11 @@ __global__ void __launch_bounds__(kPassThreads, 4) pass2Kernel(AstraeaParticles 
         }
         return;
     }
-    const uint32_t t = (blockIdx.x - kHeavyBlocks) * kPassThreads + threadIdx.x;
-    const uint32_t i = min(t / kLanes, n - 1u), c = __ldg(&w.nbrCount[i]);
-    if (kLanes == 1 && t >= n) return;
+    const uint32_t i = (blockIdx.x - kHeavyBlocks) * kPassThreads + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t c = __ldg(&w.nbrCount[i]);
     const bool listed = c <= w.maxNbr;
-    pass2Particle<kLanes>(p, w, n, i, listOf(w, i, listed ? c : 0u), t % kLanes, !listed && c != kHeavyMark,
-                          t / kLanes < n && c != kHeavyMark, livingFlags);
+    pass2Particle<1>(p, w, n, i, listOf(w, i, listed ? c : 0u), 0u, !listed && c != kHeavyMark, c != kHeavyMark, livingFlags);
 }
 
 // ----------------------------------------------------------------- drift ---
@@ -933,22 +936,20 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_
     return launchChained(poolListsKernel, static_cast<uint32_t>(std::max(1, sms)), kPoolWarps * 32, st, w, n);
 }
 
-// Lanes per particle of the SPH passes: as many as keep all of the launch's
-// threads resident at once (`wave`: blocks per SM x 128 x 152 SMs).  Below that
-// a launch lasts as long as one thread's list; above it a lane more per particle
-// only adds sums and partial last fours.  Drift / pass 1 / pass 2 with 1, 2, 4
-// lanes, us: n = 16k 41.6 / 26.6 / 45.2, 25.9 / 18.4 / 30.7, 19.4 / 15.4 / 26.6
-// (8 lanes: 24.6 / 18.4 / 30.7); 32k 39.4 / 27.1 / 48.6, 27.7 / 20.5 / 38.9,
-// 31.8 / 23.1 / 43.0; 50k 40.0 / 28.7 / 53.2, 30.8 / 25.1 / 59.9, 36.9 / 28.7 /
-// 59.9; 70k 44.2 / 31.7 / 62.0, 47.9 / 34.8 / 65.5; 200k 87.6 / 63.0 / 164,
-// 95.0 / 70.1 / 173.
-constexpr uint32_t kWave6 = 6u * 128u * 152u, kWave4 = 4u * 128u * 152u;
+// Lanes per particle of pass 1 and the drift: as many as keep all of the launch's
+// threads resident at once (6 blocks per SM x 128 x 152 SMs).  Below that a
+// launch lasts as long as one thread's list; above it a lane more per particle
+// only adds sums and partial last fours.  Drift / pass 1 with 1, 2, 4 lanes, us:
+// n = 16k 41.6 / 26.6, 25.9 / 18.4, 19.4 / 15.4 (8 lanes: 24.6 / 18.4); 32k
+// 39.4 / 27.1, 27.7 / 20.5, 31.8 / 23.1; 50k 40.0 / 28.7, 30.8 / 25.1, 36.9 /
+// 28.7; 70k 44.2 / 31.7, 47.9 / 34.8; 200k 87.6 / 63.0, 95.0 / 70.1.
+constexpr uint32_t kPassWave = 6u * 128u * 152u;
 static uint32_t passBlocks(uint32_t n, int lanes) { return kHeavyBlocks + gridFor(n, static_cast<int>(kPassThreads) / lanes); }
-static int lanesFor(uint32_t n, uint32_t wave) { return n <= wave / 4u ? 4 : (n <= wave / 2u ? 2 : 1); }
+static int lanesFor(uint32_t n) { return n <= kPassWave / 4u ? 4 : (n <= kPassWave / 2u ? 2 : 1); }
 
 cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const int lanes = lanesFor(n, kWave6);
+    const int lanes = lanesFor(n);
     const auto kernel = lanes == 4 ? pass1Kernel<4> : (lanes == 2 ? pass1Kernel<2> : pass1Kernel<1>);
     return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n);
 }
@@ -956,15 +957,13 @@ cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, cu
 cudaError_t launchPass2(const AstraeaParticles& p, const Work& w, uint32_t n, const uint32_t* livingFlags,
                         cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const int lanes = lanesFor(n, kWave4);
-    const auto kernel = lanes == 4 ? pass2Kernel<4> : (lanes == 2 ? pass2Kernel<2> : pass2Kernel<1>);
-    return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n, livingFlags);
+    return launchChained(pass2Kernel, passBlocks(n, 1), kPassThreads, st, p, w, n, livingFlags);
 }
 
 cudaError_t launchDrift(const AstraeaParticles& p, const Work& w, uint32_t n, const float* dtDev, float dtHost,
                         bool useList, bool toScratch, uint32_t* boundsWords, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const int lanes = lanesFor(n, kWave6);
+    const int lanes = lanesFor(n);
     const auto kernel = lanes == 4 ? driftKernel<4> : (lanes == 2 ? driftKernel<2> : driftKernel<1>);
     return launchChained(kernel, passBlocks(n, lanes), kPassThreads, st, p, w, n,
                          DriftArgs{dtDev, dtHost, useList, toScratch}, boundsWords);
