@@ -169,11 +169,12 @@ __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticle
 
 // Leaf records from the caller's current SoA (used before tree walks that are
 // not preceded by this library's own permutation).
-__global__ void __launch_bounds__(256) refreshLeavesKernel(AstraeaParticles p, Work w, uint32_t n, bool withVelRho) {
+__global__ void __launch_bounds__(256) refreshLeavesKernel(AstraeaParticles p, Work w, uint32_t n, bool withVelRho,
+                                                           bool arm) {
     chained();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (i == 0u) armNeighborBuild(w);
+    if (i == 0u && arm) armNeighborBuild(w);
     const float hI = fmaxf(__ldg(&p.h[i]), 1.0e-6f);
     const float h0I = fmaxf(__ldg(&p.h0[i]), 1.0e-6f);
     const float m = __ldg(&p.mass[i]);
@@ -662,8 +663,8 @@ cudaError_t launchPermuteLeavesKarras(const AstraeaParticles& p, const AstraeaPa
 }
 
 cudaError_t launchRefreshLeaves(const AstraeaParticles& p, const Work& w, uint32_t n, bool withVelRho,
-                                cudaStream_t st) {
-    return launchChained(refreshLeavesKernel, gridFor(n, 256), 256, st, p, w, n, withVelRho);
+                                cudaStream_t st, bool arm) {
+    return launchChained(refreshLeavesKernel, gridFor(n, 256), 256, st, p, w, n, withVelRho, arm);
 }
 
 uint32_t refitBlocks(uint32_t n) { return (n + kRefitBlock - 1) / kRefitBlock; }

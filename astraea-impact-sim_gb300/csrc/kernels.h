@@ -61,8 +61,9 @@ cudaError_t launchBounds(const AstraeaParticles& p, uint32_t n, uint32_t* words,
 cudaError_t launchPermuteLeavesKarras(const AstraeaParticles& p, const AstraeaParticles& alt,
                                       const AstraeaRadixBvh& bvh, const float4* posSrc, const Work& w, uint32_t n,
                                       uint32_t* livingFlags, bool allFields, cudaStream_t st);
+// arm: clear the words of the next neighbour build, which ends the lists there are
 cudaError_t launchRefreshLeaves(const AstraeaParticles& p, const Work& w, uint32_t n, bool withVelRho,
-                                cudaStream_t st);
+                                cudaStream_t st, bool arm = true);
 cudaError_t launchRefit(const AstraeaRadixBvh& bvh, const Work& w, uint32_t n, bool moments, cudaStream_t st);
 // node masses and COMs in the engine's FP32 bottom-up rounding (after launchRefit)
 cudaError_t launchEngineNodeMoments(const AstraeaParticles& p, const AstraeaRadixBvh& bvh, const Work& w, uint32_t n,
