@@ -137,7 +137,20 @@ struct Workspace {
     cudaEvent_t stageEv[kStageCount + 1] = {};
     bool stageRecorded = false;
     FfBuffers ff;                  // far-field mode 2 (created on first use)
+    // the step's gravity walk beside the SPH chain (kShareMax): a stream and the
+    // events that fork it from the caller's stream and join it again
+    cudaStream_t side = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
 };
+// The walk over the tree for gravity and the one for neighbours, pass 1 and the
+// EOS read the tree and write different arrays.  In a small scene each is a chain of a
+// few warps per SM that leaves the SMs idle: they run side by side.  Larger
+// scenes fill the GPU with either, and gain the other's last blocks.  Step, one
+// after the other / side by side / side by side on the same SMs (LaunchAt):
+// 8k 276 / 208 / 211 us, 16k 310 / 254 / 234, 32k 364 / 387 / 280, 50k 418 / 432 /
+// 337, 100k 605 / 578 / 529, 262k 1172 / 1083 / 1071, 1M 3730 / 3640 / 3661, so SMs
+// are shared up to kShareMax.
+constexpr uint32_t kShareMax = 1u << 19;
 std::map<std::pair<int, const void*>, Workspace*> g_work;
 
 uint32_t maxNeighbors() {
@@ -211,6 +224,11 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     w.status = ds->status;
     ws->dtSlots = reinterpret_cast<float*>(b + oDt);
     ws->rawMin = reinterpret_cast<uint32_t*>(b + oDt + 16);
+    if (ws->side == nullptr) {
+        AG_CUDA(cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking));
+        AG_CUDA(cudaEventCreateWithFlags(&ws->forked, cudaEventDisableTiming));
+        AG_CUDA(cudaEventCreateWithFlags(&ws->joined, cudaEventDisableTiming));
+    }
     AG_CUDA(cudaMemset(w.words, 0, kWCount * 4));
     AG_CUDA(cudaMemset(b + oDt, 0, 64));
     ws->treeBuilt = false;
@@ -244,6 +262,9 @@ void dropWorkspace(const void* leftChild) {
     for (auto it = g_work.begin(); it != g_work.end(); ++it) {
         if (it->first.second == leftChild) {
             cudaFree(it->second->block);
+            if (it->second->side) cudaStreamDestroy(it->second->side);
+            if (it->second->forked) cudaEventDestroy(it->second->forked);
+            if (it->second->joined) cudaEventDestroy(it->second->joined);
             for (cudaEvent_t e : it->second->stageEv)
                 if (e) cudaEventDestroy(e);
             it->second->ff.release();
@@ -456,7 +477,7 @@ AstraeaStatus learnedGravity(AstraeaParticles* p, Workspace* ws, uint32_t n, flo
 
 // The gravity walk of far-field modes 0, 1 and 3 on a built workspace.
 cudaError_t modeGravity(const AstraeaParticles& p, const Work& w0, uint32_t n, float theta, int mode, bool moments,
-                        int sms, cudaStream_t st, int warps) {
+                        int sms, LaunchAt st, int warps) {
     if (mode == 3 && moments) {
         Work w = w0;
         w.leafBucket = g_leafBucket.load();
@@ -1565,21 +1586,43 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
     marks.mark(ASTRAEA_STAGE_SORT);
     s = buildTree(p, alt, bvh, ws, w.driftPos, false, marks);
     if (s != ASTRAEA_OK) return s;
+    const int mode = g_farField.load();
+    const bool learned = ws->momentsBuilt && mode == 2;
+    auto gravity = [&](LaunchAt on) {
+        return modeGravity(*p, w, n, theta, mode, ws->momentsBuilt, sms, on,
+                           static_cast<int>(gravityWarpsFor(n, gravityVariant(mode, ws->momentsBuilt, theta))));
+    };
+    // (timed stages run one after the other)
+    const bool beside = n >= 2u && !learned && marks.ev == nullptr, share = beside && n <= kShareMax;
+    struct Join {                      // also where a launch in between fails
+        cudaStream_t st;
+        cudaEvent_t ev;
+        ~Join() { if (ev != nullptr) (void)cudaStreamWaitEvent(st, ev, 0); }
+    } join{st, nullptr};
+    if (beside) {
+        AG_CUDA(cudaEventRecord(ws->forked, st));
+        AG_CUDA(cudaStreamWaitEvent(ws->side, ws->forked, 0));
+        const cudaError_t e = gravity(LaunchAt(ws->side, share));
+        AG_CUDA(cudaEventRecord(ws->joined, ws->side));
+        join.ev = ws->joined;
+        AG_LAUNCH(e);
+    }
     // 4. neighbour lists for pass 1, pass 2 and the next drift
     marks.mark(ASTRAEA_STAGE_NEIGHBOURS);
-    AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps), true));
+    AG_LAUNCH(launchBuildNeighbors(w, n, sms, LaunchAt(st, share), static_cast<int>(tune.neighborWarps), true));
     marks.mark(ASTRAEA_STAGE_PASS1);
-    AG_LAUNCH(launchPass1(*p, w, n, st));
+    AG_LAUNCH(launchPass1(*p, w, n, LaunchAt(st, share)));
     marks.mark(ASTRAEA_STAGE_EOS);
-    AG_LAUNCH(launchEos(*p, &w, n, st));
+    AG_LAUNCH(launchEos(*p, &w, n, LaunchAt(st, share)));
     marks.mark(ASTRAEA_STAGE_GRAVITY);
-    if (ws->momentsBuilt && g_farField.load() == 2) {
+    if (beside) {
+        join.ev = nullptr;
+        AG_CUDA(cudaStreamWaitEvent(st, ws->joined, 0));
+    } else if (learned) {
         s = learnedGravity(p, ws, n, theta, true);
         if (s != ASTRAEA_OK) return s;
     } else {
-        const int mode = g_farField.load();
-        AG_LAUNCH(modeGravity(*p, w, n, theta, mode, ws->momentsBuilt, sms, st,
-                              static_cast<int>(gravityWarpsFor(n, gravityVariant(mode, ws->momentsBuilt, theta)))));
+        AG_LAUNCH(gravity(st));
     }
     marks.mark(ASTRAEA_STAGE_PASS2);
     AG_LAUNCH(launchPass2(*p, w, n, livingPtr(bvh, ws), st));

@@ -1148,7 +1148,7 @@ __global__ void __launch_bounds__(kOrdWarps * 32, 28 / kOrdWarps) gravityOrdered
 }  // namespace
 
 cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, float theta, bool quadrupole, int sms,
-                          cudaStream_t st, const FarCapture* far, int warps, bool expansion) {
+                          LaunchAt st, const FarCapture* far, int warps, bool expansion) {
     if (n == 0) return cudaSuccess;
     const float th = fmaxf(0.0f, theta);
     const float theta2 = th * th;
@@ -1158,7 +1158,7 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     // The pair kernel also clears the counter.  (The learned mode's fallback,
     // runIf, walks the records its first walk wrote.)
     cudaError_t e = n >= 2u && w.runIf == nullptr ? launchChained(pairNodesKernel, (n - 1u + 255u) / 256u, 256, st, w, n)
-                                                  : cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
+                                                  : cudaMemsetAsync(counter, 0, sizeof(uint32_t), st.stream);
     if (e != cudaSuccess) return e;
     if (n > kOrderedAbove && !quadrupole && far == nullptr && w.runIf == nullptr && w.traceList == nullptr &&
         w.groupCounts == nullptr) {

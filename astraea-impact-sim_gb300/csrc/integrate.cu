@@ -280,7 +280,7 @@ cudaError_t launchClearStats(const AstraeaParticles& p, uint32_t n, cudaStream_t
     return launchChained(clearStatsKernel, gridFor(n, 256), 256, st, p, n);
 }
 
-cudaError_t launchEos(const AstraeaParticles& p, const Work* w, uint32_t n, cudaStream_t st) {
+cudaError_t launchEos(const AstraeaParticles& p, const Work* w, uint32_t n, LaunchAt st) {
     if (n == 0) return cudaSuccess;
     Work none{};
     return launchChained(eosKernel, gridFor(n, 256), 256, st, p, w ? *w : none, w != nullptr, n);

@@ -22,24 +22,36 @@ namespace astraea_gb300 {
 // running kernel happens to leave room, and the walks, whose few blocks a small
 // scene has no second wave to even out, ran 16k 344 us, gravity at 60k 157.
 __device__ __forceinline__ void chained() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Where a kernel is launched: the stream, and whether it is to run beside the
+// kernels of another stream.  An SM divides its memory between L1 and shared
+// memory anew only when it is empty, so kernels for which the driver chooses
+// different splits do not meet on one; those that should meet ask for the same
+// one (all shared memory).
+struct LaunchAt {
+    cudaStream_t stream;
+    bool beside;
+    LaunchAt(cudaStream_t s, bool b = false) : stream(s), beside(b) {}
+};
 template <class... P, class... A>
-cudaError_t launchChainedSmem(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
-                              A&&... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+cudaError_t launchChainedSmem(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, LaunchAt at, A&&... args) {
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.stream = at.stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = at.beside ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 template <class... P, class... A>
-cudaError_t launchChained(void (*kernel)(P...), uint32_t grid, uint32_t block, cudaStream_t st, A&&... args) {
-    return launchChainedSmem(kernel, grid, block, 0, st, static_cast<A&&>(args)...);
+cudaError_t launchChained(void (*kernel)(P...), uint32_t grid, uint32_t block, LaunchAt at, A&&... args) {
+    return launchChainedSmem(kernel, grid, block, 0, at, static_cast<A&&>(args)...);
 }
 
 constexpr int kSortThreads = 512;

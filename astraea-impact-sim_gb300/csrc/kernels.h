@@ -119,7 +119,7 @@ struct FarCapture {
 // buckets and the group expansion of nodes far against the group,
 // w.expandGamma2); needs quadrupole.
 cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, float theta, bool quadrupole, int sms,
-                          cudaStream_t st, const FarCapture* far = nullptr, int warps = 4, bool expansion = false);
+                          LaunchAt st, const FarCapture* far = nullptr, int warps = 4, bool expansion = false);
 
 // ---------------------------------------------------------------- ff.cu ---
 namespace ff {
@@ -165,8 +165,8 @@ cudaError_t launchGate(const AstraeaParticles& p, const Work& w, uint32_t n, uin
 // warps: 2, 4 or 8 warps per block (the autotuner's choice; results do not depend on it)
 // armed: the words of the build were cleared by the permutation or the leaf
 // refresh and no build has run since.
-cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_t st, int warps = 4, bool armed = false);
-cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, cudaStream_t st);
+cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st, int warps = 4, bool armed = false);
+cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, LaunchAt st);
 cudaError_t launchPass2(const AstraeaParticles& p, const Work& w, uint32_t n, const uint32_t* livingFlags,
                         cudaStream_t st);
 // XSPH drift; new positions go to w.driftPos when toScratch, else back into
@@ -178,7 +178,7 @@ cudaError_t launchDrift(const AstraeaParticles& p, const Work& w, uint32_t n, co
 // -------------------------------------------------------- integrate.cu ---
 cudaError_t launchClearStats(const AstraeaParticles& p, uint32_t n, cudaStream_t st);
 // EOS; when w != nullptr also writes the pass-2 neighbour records.
-cudaError_t launchEos(const AstraeaParticles& p, const Work* w, uint32_t n, cudaStream_t st);
+cudaError_t launchEos(const AstraeaParticles& p, const Work* w, uint32_t n, LaunchAt st);
 // Half kick.  dtMode 0: halfDt = halfDtHost.  dtMode 1 (opening kick of a
 // fused step): dt = clamp of the raw minimum *rawMinIn against the previous
 // dt dtSlots[parity] (the host clamp of launchReduceDtPsu), written to

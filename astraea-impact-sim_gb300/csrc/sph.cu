@@ -916,11 +916,11 @@ inline unsigned gridFor(uint32_t n, int block) { return static_cast<unsigned>((n
 
 }  // namespace
 
-cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, cudaStream_t st, int warps, bool armed) {
+cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st, int warps, bool armed) {
     if (n == 0) return cudaSuccess;
     const uint32_t groups = (n + 31u) / 32u;
     uint32_t* counter = w.words + kWNbrCounter;          // with the pool's words behind it
-    cudaError_t e = armed ? cudaSuccess : cudaMemsetAsync(counter, 0, 4 * sizeof(uint32_t), st);
+    cudaError_t e = armed ? cudaSuccess : cudaMemsetAsync(counter, 0, 4 * sizeof(uint32_t), st.stream);
     if (e != cudaSuccess) return e;
     using NbFn = void (*)(Work, uint32_t, uint32_t, uint32_t*);
     const int wps = (warps == 2 || warps == 8) ? warps : kNbWarps;
@@ -947,7 +947,7 @@ constexpr uint32_t kPassWave = 6u * 128u * 152u;
 static uint32_t passBlocks(uint32_t n, int lanes) { return kHeavyBlocks + gridFor(n, static_cast<int>(kPassThreads) / lanes); }
 static int lanesFor(uint32_t n) { return n <= kPassWave / 4u ? 4 : (n <= kPassWave / 2u ? 2 : 1); }
 
-cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, cudaStream_t st) {
+cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, LaunchAt st) {
     if (n == 0) return cudaSuccess;
     const int lanes = lanesFor(n);
     const auto kernel = lanes == 4 ? pass1Kernel<4> : (lanes == 2 ? pass1Kernel<2> : pass1Kernel<1>);

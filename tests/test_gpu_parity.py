@@ -579,3 +579,27 @@ def test_sph_passes_lanes_and_long_lists(n):
     flags, counters = engine.read_device_status()
     assert counters["fallback_walks"] == 0
     assert bool(flags & abi.DEVFLAG_NEIGHBOR_OVERFLOW) == (n > 1000)
+
+
+@pytest.mark.parametrize("n", [2, 33, 4097, 40_001, (1 << 19) + 1])
+def test_step_walks_side_by_side_change_nothing(n):
+    """The step runs the gravity walk beside the neighbour lists, pass 1 and the
+    EOS; with stage timing on it runs them one after the other.  Same bits."""
+    m = max(n, 64)
+    st = {k: v[:n].copy() for k, v in c1_state(n_t=m - m // 4, n_i=m // 4).items()}
+    st["originalId"] = np.arange(n, dtype=np.uint32)
+    out = []
+    for timed in (False, True):
+        sim = engine.Simulation(n)
+        sim.p.upload(st)
+        sim.alt.count = n
+        sim.evaluate_initial_forces(0.5)
+        engine.set_stage_timing(timed)
+        try:
+            dts = [sim.step(5.0e-3, 0.5) for _ in range(3)]
+        finally:
+            engine.set_stage_timing(False)
+        out.append((dts, sim.p.download()))
+    assert out[0][0] == out[1][0]
+    for f in out[0][1]:
+        assert np.array_equal(out[0][1][f], out[1][1][f], equal_nan=out[0][1][f].dtype.kind == "f"), f
