@@ -620,7 +620,9 @@ __global__ void __launch_bounds__(kPassThreads, 6) pass1Kernel(AstraeaParticles 
 // Reads the pass-2 records written by the EOS kernel (layout and derived
 // values: integrate.cu, writePass2Record): one 256-bit load per 32-byte
 // piece, and no per-pair division for quantities of the neighbour alone.
-template <int kLanes>
+// kWhole: all of a record is loaded with its first piece, before the test.
+struct Rec96 { F8 q01, q23, q45; };
+template <int kLanes, bool kWhole>
 __device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const Work& w, uint32_t n, uint32_t i,
                                               const List& l, uint32_t sub, bool walk, bool write,
                                               const uint32_t* livingFlags) {
@@ -646,8 +648,16 @@ __device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const W
     uint32_t nPairs = 0;
     // records in 32-byte pieces: {q0, q1} for every candidate (one sector),
     // {q2, q3} and {q4, q5} for the candidates in range
-    auto first = [&](uint32_t j) { return ldg256(&R[kRec2Width * static_cast<size_t>(j)]); };
-    auto tested = [&](uint32_t j, const F8& q01) {
+    auto first = [&](uint32_t j) {
+        const float4* rj = &R[kRec2Width * static_cast<size_t>(j)];
+        if constexpr (kWhole)
+            return Rec96{ldg256(rj), ldg256(rj + 2), ldg256(rj + 4)};
+        else
+            return ldg256(rj);
+    };
+    auto tested = [&](uint32_t j, const auto& rec) {
+        F8 q01;
+        if constexpr (kWhole) q01 = rec.q01; else q01 = rec;
         const float4 b0 = q01.a;
         const float dx = __fsub_rn(xi, b0.x), dy = __fsub_rn(yi, b0.y), dz = __fsub_rn(zi, b0.z);
         const float r2 = len2Engine(dx, dy, dz);
@@ -655,8 +665,14 @@ __device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const W
         const float Hm = fmaxf(Hi, Hj);
         if (!(r2 < __fmul_rn(Hm, Hm))) return;          // sph_gravity.cu:1071
         ++nPairs;
-        const F8 q23 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 2]);
-        const F8 q45 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 4]);
+        F8 q23, q45;
+        if constexpr (kWhole) {
+            q23 = rec.q23;
+            q45 = rec.q45;
+        } else {
+            q23 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 2]);
+            q45 = ldg256(&R[kRec2Width * static_cast<size_t>(j) + 4]);
+        }
         const float4 b1 = q01.b, b2 = q23.a, b3 = q23.b, b4 = q45.a, b5 = q45.b;
         const float mj = b1.w, rhoJ = b2.x, pOverRho2J = b2.y, csJ = b2.z, fBalJ = b2.w;
         const float volJ = b5.x;
@@ -792,15 +808,18 @@ __device__ __forceinline__ void pass2Particle(const AstraeaParticles& p, const W
 // lanes sharing a list (as in pass 1 and the drift) made it 27 instead of 45 us
 // at 16k, but the other order of the sums moves du/dt and drho/dt by 1e-6 of
 // their norm, and the strength of iron just below its melting point amplifies an
-// ulp of rho a thousandfold.
-__global__ void __launch_bounds__(kPassThreads, 4) pass2Kernel(AstraeaParticles p, Work w, uint32_t n,
+// ulp of rho a thousandfold.  While two blocks per SM hold the scene there are
+// registers to load whole records ahead (kBlocks 2, 180 registers): 16k 45.6 -> 43.0
+// us, 30k 48.6 -> 45.1; beyond, four blocks (70k: 61 us, two 81).
+template <int kBlocks>
+__global__ void __launch_bounds__(kPassThreads, kBlocks) pass2Kernel(AstraeaParticles p, Work w, uint32_t n,
                                                               const uint32_t* livingFlags) {
     chained();
     if (blockIdx.x < kHeavyBlocks) {
         const uint32_t lane = threadIdx.x & 31u, total = heavyCount(w);
         for (uint32_t e = blockIdx.x * (kPassThreads / 32u) + (threadIdx.x >> 5); e < total; e += kHeavyWarps) {
             const uint4 h = __ldg(&w.heavy[e]);
-            if (h.z != 0u) pass2Particle<32>(p, w, n, h.x, List{w.pool + h.y, 1u, h.z}, lane, false, true, livingFlags);
+            if (h.z != 0u) pass2Particle<32, false>(p, w, n, h.x, List{w.pool + h.y, 1u, h.z}, lane, false, true, livingFlags);
         }
         return;
     }
@@ -808,7 +827,7 @@ __global__ void __launch_bounds__(kPassThreads, 4) pass2Kernel(AstraeaParticles 
     if (i >= n) return;
     const uint32_t c = __ldg(&w.nbrCount[i]);
     const bool listed = c <= w.maxNbr;
-    pass2Particle<1>(p, w, n, i, listOf(w, i, listed ? c : 0u), 0u, !listed && c != kHeavyMark, c != kHeavyMark, livingFlags);
+    pass2Particle<1, kBlocks == 2>(p, w, n, i, listOf(w, i, listed ? c : 0u), 0u, !listed && c != kHeavyMark, c != kHeavyMark, livingFlags);
 }
 
 // ----------------------------------------------------------------- drift ---
@@ -943,6 +962,7 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st
 // n = 16k 41.6 / 26.6, 25.9 / 18.4, 19.4 / 15.4 (8 lanes: 24.6 / 18.4); 32k
 // 39.4 / 27.1, 27.7 / 20.5, 31.8 / 23.1; 50k 40.0 / 28.7, 30.8 / 25.1, 36.9 /
 // 28.7; 70k 44.2 / 31.7, 47.9 / 34.8; 200k 87.6 / 63.0, 95.0 / 70.1.
+constexpr uint32_t kPass2Wave = 2u * 128u * 152u;   // threads of two blocks per SM (pass2Kernel)
 constexpr uint32_t kPassWave = 6u * 128u * 152u;
 static uint32_t passBlocks(uint32_t n, int lanes) { return kHeavyBlocks + gridFor(n, static_cast<int>(kPassThreads) / lanes); }
 static int lanesFor(uint32_t n) { return n <= kPassWave / 4u ? 4 : (n <= kPassWave / 2u ? 2 : 1); }
@@ -957,7 +977,8 @@ cudaError_t launchPass1(const AstraeaParticles& p, const Work& w, uint32_t n, La
 cudaError_t launchPass2(const AstraeaParticles& p, const Work& w, uint32_t n, const uint32_t* livingFlags,
                         cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    return launchChained(pass2Kernel, passBlocks(n, 1), kPassThreads, st, p, w, n, livingFlags);
+    const auto kernel = n <= kPass2Wave ? pass2Kernel<2> : pass2Kernel<4>;
+    return launchChained(kernel, passBlocks(n, 1), kPassThreads, st, p, w, n, livingFlags);
 }
 
 cudaError_t launchDrift(const AstraeaParticles& p, const Work& w, uint32_t n, const float* dtDev, float dtHost,
