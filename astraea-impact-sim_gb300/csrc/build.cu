@@ -72,13 +72,17 @@ __device__ __forceinline__ void armNeighborBuild(const Work& w) {
 template <bool kAllFields>
 __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticles p, AstraeaParticles alt,
                                                                  AstraeaRadixBvh bvh, const float4* __restrict__ posSrc,
-                                                                 Work w, uint32_t n, uint32_t* livingFlags) {
+                                                                 Work w, uint32_t n, uint32_t* livingFlags,
+                                                                 uint32_t karrasFrom) {
     chained();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0u) armNeighborBuild(w);
+    // blocks below karrasFrom move particles; those from it on, or, when it is 0,
+    // the same ones, find the internal nodes
+    const bool moves = karrasFrom == 0u || blockIdx.x < karrasFrom, finds = karrasFrom == 0u || !moves;
+    const uint32_t i = (moves ? blockIdx.x : blockIdx.x - karrasFrom) * blockDim.x + threadIdx.x;
+    if (i == 0u && moves) armNeighborBuild(w);
     bool tracer = false, intact = false;
     uint32_t massBits = 0u;                         // |m| as bits: ordered like the values
-    if (i < n) {
+    if (i < n && moves) {
         // min(): keeps the gather in bounds even if a failed sort (look-back
         // timeout, flagged in the status word) left a non-permutation here.
         const uint32_t s = min(__ldg(&bvh.indicesSorted[i]), n - 1u);
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(256) permuteLeavesKarrasKernel(AstraeaParticle
         // scale of the refit's sums; the word only grows, so a stale read costs one extra atomic at most
         if (warpMassBits > __ldcg(&w.words[kWMassMax])) atomicMax(&w.words[kWMassMax], warpMassBits);
     }
-    if (i + 1u < n) {                               // internal node i (Karras 2012)
+    if (i + 1u < n && finds) {                      // internal node i (Karras 2012)
         const int ii = static_cast<int>(i);
         const int nn = static_cast<int>(n);
         const uint64_t* codes = bvh.mortonCodesSorted;
@@ -583,13 +587,11 @@ __global__ void __launch_bounds__(1024) refitScanKernel(Work w, uint32_t nb) {
     }
 }
 
-// Up to three levels of the sparse table of block extremes per launch
+// Up to three levels of the sparse table of block extremes at block b
 // (the levels are latency-bound, so the extra loads are cheap): with
 // s = 2^(lev-1) and A_k = T[lev-1][b + k s], T[lev-1+j][b] joins
 // A_0 .. A_(2^j - 1) (it covers blocks b .. b + 2^j s - 1), j = 1 .. count.
-__global__ void __launch_bounds__(256) refitLevelKernel(Work w, uint32_t nb, uint32_t lev, uint32_t count) {
-    chained();
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void tableLevels(const Work& w, uint32_t nb, uint32_t lev, uint32_t count, uint32_t b) {
     const uint32_t s = 1u << (lev - 1);
     if (b + 2u * s > nb) return;
     const float4* src = w.blockTable + 2 * static_cast<size_t>(lev - 1) * nb;
@@ -605,6 +607,56 @@ __global__ void __launch_bounds__(256) refitLevelKernel(Work w, uint32_t nb, uin
         for (uint32_t k = width >> 1; k < width; ++k) acc = extJoin(acc, a[k]);
         extStore(w.blockTable + 2 * (static_cast<size_t>(lev - 1 + j) * nb + b), acc);
     }
+}
+__global__ void __launch_bounds__(256) refitLevelKernel(Work w, uint32_t nb, uint32_t lev, uint32_t count) {
+    chained();
+    tableLevels(w, nb, lev, count, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Scan and table of at most kTopBlocks blocks of leaves in one launch: block 0
+// scans, a thread a total; block 1 fills the table, barriers between its levels.
+// Latency bound, and so are the up to four launches it stands for: step at 16k
+// 231.5 -> 228 us, at 70k 409 -> 402; with 1,024 blocks (262k) no difference, with
+// 4,096 (1M) 44 us slower.
+constexpr uint32_t kTopBlocks = 512u;
+template <bool kMoments>
+__global__ void __launch_bounds__(kTopBlocks) refitTopKernel(Work w, uint32_t nb, uint32_t levels) {
+    chained();
+    constexpr int kW = kMoments ? kMomW : 4;
+    constexpr uint32_t kWarps = kTopBlocks / 32u;
+    __shared__ long long warpSum[kW][kWarps];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    if (blockIdx.x != 0u) {
+        for (uint32_t lev = 1; lev < levels; lev += 3) {
+            tableLevels(w, nb, lev, min(3u, levels - lev), t);
+            __syncthreads();
+        }
+        return;
+    }
+    long long own[kW], inc[kW];
+#pragma unroll
+    for (int k = 0; k < kW; ++k) {
+        own[k] = t < nb ? __ldcg(&w.blockMom[static_cast<size_t>(kMomW) * t + k]) : 0;
+        inc[k] = own[k];
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+        for (int k = 0; k < kW; ++k) {
+            const long long o = __shfl_up_sync(0xffffffffu, inc[k], d);
+            if (lane >= static_cast<uint32_t>(d)) inc[k] += o;
+        }
+    if (lane == 31u)
+#pragma unroll
+        for (int k = 0; k < kW; ++k) warpSum[k][warp] = inc[k];
+    __syncthreads();
+    if (t < nb)
+#pragma unroll
+        for (int k = 0; k < kW; ++k) {
+            long long before = inc[k] - own[k];
+            for (uint32_t q = 0; q < warp; ++q) before += warpSum[k][q];
+            w.blockMom[static_cast<size_t>(kMomW) * t + k] = before;
+        }
 }
 
 // Nodes whose range spans blocks.
@@ -656,10 +708,15 @@ cudaError_t launchBounds(const AstraeaParticles& p, uint32_t n, uint32_t* words,
 cudaError_t launchPermuteLeavesKarras(const AstraeaParticles& p, const AstraeaParticles& alt,
                                       const AstraeaRadixBvh& bvh, const float4* posSrc, const Work& w, uint32_t n,
                                       uint32_t* livingFlags, bool allFields, cudaStream_t st) {
-    if (allFields)
-        return launchChained(permuteLeavesKarrasKernel<true>, gridFor(n, 256), 256, st, p, alt, bvh, posSrc, w, n, livingFlags);
-    else
-        return launchChained(permuteLeavesKarrasKernel<false>, gridFor(n, 256), 256, st, p, alt, bvh, posSrc, w, n, livingFlags);
+    // The moves and the searches for the nodes are two chains of dependent loads;
+    // while the blocks of both fit at once (8 x 152 of 128 threads) each runs in
+    // its own: permutation at 16k 18.7 -> 16.5 us, at 70k 20.5 -> 18.0.
+    constexpr uint32_t kSplitMax = 4u * 152u * 128u;
+    const uint32_t block = n <= kSplitMax ? 128u : 256u, blocks = gridFor(n, static_cast<int>(block));
+    const bool split = n <= kSplitMax;
+    const auto kernel = allFields ? permuteLeavesKarrasKernel<true> : permuteLeavesKarrasKernel<false>;
+    return launchChained(kernel, split ? 2u * blocks : blocks, block, st, p, alt, bvh, posSrc, w, n, livingFlags,
+                         split ? blocks : 0u);
 }
 
 cudaError_t launchRefreshLeaves(const AstraeaParticles& p, const Work& w, uint32_t n, bool withVelRho,
@@ -741,11 +798,17 @@ cudaError_t launchRefit(const AstraeaRadixBvh& bvh, const Work& w, uint32_t n, b
     const uint32_t levels = refitLevels(nb);
     cudaError_t e = moments ? launchChained(refitBlockKernel<true>, nb, kRefitBlock, st, bvh, w, n)
                             : launchChained(refitBlockKernel<false>, nb, kRefitBlock, st, bvh, w, n);
-    if (e == cudaSuccess)
-        e = moments ? launchChained(refitScanKernel<true>, 1, 1024, st, w, nb)
-                    : launchChained(refitScanKernel<false>, 1, 1024, st, w, nb);
-    for (uint32_t lev = 1; lev < levels && e == cudaSuccess; lev += 3)
-        e = launchChained(refitLevelKernel, gridFor(nb, 256), 256, st, w, nb, lev, std::min(3u, levels - lev));
+    if (nb <= kTopBlocks) {
+        if (e == cudaSuccess)
+            e = moments ? launchChained(refitTopKernel<true>, 2, kTopBlocks, st, w, nb, levels)
+                        : launchChained(refitTopKernel<false>, 2, kTopBlocks, st, w, nb, levels);
+    } else {
+        if (e == cudaSuccess)
+            e = moments ? launchChained(refitScanKernel<true>, 1, 1024, st, w, nb)
+                        : launchChained(refitScanKernel<false>, 1, 1024, st, w, nb);
+        for (uint32_t lev = 1; lev < levels && e == cudaSuccess; lev += 3)
+            e = launchChained(refitLevelKernel, gridFor(nb, 256), 256, st, w, nb, lev, std::min(3u, levels - lev));
+    }
     if (e != cudaSuccess) return e;
     return moments ? launchChained(refitCrossKernel<true>, gridFor(n, 256), 256, st, bvh, w, n, nb)
                    : launchChained(refitCrossKernel<false>, gridFor(n, 256), 256, st, bvh, w, n, nb);

@@ -603,3 +603,27 @@ def test_step_walks_side_by_side_change_nothing(n):
     assert out[0][0] == out[1][0]
     for f in out[0][1]:
         assert np.array_equal(out[0][1][f], out[1][1][f], equal_nan=out[0][1][f].dtype.kind == "f"), f
+
+
+@pytest.mark.parametrize("n", [2, 255, 257, 513, 77_824, 77_825, 131_072, 131_073])
+def test_permutation_and_refit_at_block_counts(n):
+    """Both sides of the sizes where the permutation and the node search share
+    their blocks and where the refit's scan and table share one launch: order,
+    topology and boxes bit for bit, exact moment sums within 1e-6 of the FP32
+    refit as in test_sort_and_build_bit_exact."""
+    m = max(n, 64)
+    st = {k: v[:n].copy() for k, v in c1_state(n_t=m - m // 4, n_i=m // 4).items()}
+    st["originalId"] = np.arange(n, dtype=np.uint32)
+    p, alt, bvh = gpu_setup(st)
+    engine.sort_and_build_bvh(p, alt, bvh)
+    torch.cuda.synchronize()
+    o = oracle.Oracle(st)
+    o.sort_and_build()
+    b = o.bvh.a
+    assert np.array_equal(tnp(bvh.t["indicesSorted"], n, np.uint32), b["indicesSorted"])
+    assert np.array_equal(tnp(bvh.t["leftChild"], n - 1), b["leftChild"][: n - 1])
+    assert np.array_equal(tnp(bvh.t["parent"], 2 * n - 1), b["parent"])
+    for f in ("aabbMinX", "aabbMinY", "aabbMinZ", "aabbMaxX", "aabbMaxY", "aabbMaxZ", "nodeMaxH"):
+        assert np.array_equal(tnp(bvh.t[f], 2 * n - 1), b[f]), f
+    for f in ("nodeMass", "comX", "comY", "comZ"):
+        assert rel_rms(tnp(bvh.t[f], 2 * n - 1), b[f]) < 1e-6, f
