@@ -488,6 +488,35 @@ cudaError_t modeGravity(const AstraeaParticles& p, const Work& w0, uint32_t n, f
     return launchGravity(p, w0, n, theta, moments && mode == 1, sms, st, nullptr, warps);
 }
 
+// Launches of one walk on the workspace's side stream, beside what the caller
+// launches on its own until join(); joins also where something in between fails.
+class Beside {
+ public:
+    Beside(Workspace* ws, cudaStream_t st) : ws_(ws), st_(st) {}
+    ~Beside() {
+        if (open_) (void)join();
+    }
+    template <class F>
+    cudaError_t fork(bool share, F&& walk) {
+        cudaError_t e = cudaEventRecord(ws_->forked, st_);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ws_->side, ws_->forked, 0);
+        if (e != cudaSuccess) return e;
+        const cudaError_t launched = walk(LaunchAt(ws_->side, share));
+        e = cudaEventRecord(ws_->joined, ws_->side);
+        open_ = e == cudaSuccess;
+        return launched != cudaSuccess ? launched : e;
+    }
+    cudaError_t join() {
+        open_ = false;
+        return cudaStreamWaitEvent(st_, ws_->joined, 0);
+    }
+
+ private:
+    Workspace* ws_;
+    cudaStream_t st_;
+    bool open_ = false;
+};
+
 uint32_t* livingPtr(const AstraeaRadixBvh* bvh, Workspace* ws) {
     return (bvh->livingFlags != nullptr) ? bvh->livingFlags : ws->w.words + kWLiving;
 }
@@ -1041,20 +1070,38 @@ AstraeaStatus astraea_gb300_relax_single_body(AstraeaParticles* p, AstraeaPartic
 #define AG_STAGE(call) do { s = (call); if (s != ASTRAEA_OK) return s; } while (0)
     // One neighbour build serves pass 1, pass 2 and the next drift, as in the
     // fused step (the lists are a superset for every h that pass 1 may set, and
-    // a kick moves nothing); positions change in the drift, which the build
-    // follows, and in the recentring, after which the forces build again
-    // (`lists` false).  31 builds -> 13 for four steps; 25k 5.79 -> 4.53 ms.
-    auto forces = [&](bool lists) -> AstraeaStatus {                         // :616 / :709-711
-        AstraeaStatus r = astraea_gb300_evaluate_eos(p);
-        if (r == ASTRAEA_OK) r = gravityBarnesHut(p, bvh, 0.5f, lists);
-        if (r == ASTRAEA_OK) r = pass2Forces(p, bvh, lists);
-        return r;
+    // a kick moves nothing); positions change in the drift, which the sort and
+    // build follow, and in the recentring, after which the forces build again.
+    // 31 builds -> 13 for four steps: 25k 5.79 -> 4.53 ms; the gravity walk beside
+    // the lists, pass 1 and the EOS, also as there: -> 3.57 ms.
+    auto forces = [&](bool sorted) -> AstraeaStatus {   // sorted: after build(), with pass 1 (:616 / :709-711)
+        Workspace* ws = nullptr;
+        AstraeaStatus r = builtWorkspace(bvh, n, &ws);
+        if (r != ASTRAEA_OK) return r;
+        const int mode = g_farField.load();
+        if (n < 2u || mode == 2 || (mode != 0 && !ws->momentsBuilt)) {
+            if (sorted) r = astraea_gb300_sph_pass1_neighbors(p, bvh);
+            if (r == ASTRAEA_OK) r = astraea_gb300_evaluate_eos(p);
+            if (r == ASTRAEA_OK) r = gravityBarnesHut(p, bvh, 0.5f, sorted);
+            if (r == ASTRAEA_OK) r = pass2Forces(p, bvh, sorted);
+            return r;
+        }
+        cudaStream_t st = stream();
+        const int sms = smCount();
+        const bool share = n <= kShareMax;
+        AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
+        Beside walks(ws, st);
+        AG_LAUNCH(walks.fork(share, [&](LaunchAt at) {
+            return modeGravity(*p, ws->w, n, 0.5f, mode, true, sms, at,
+                               static_cast<int>(gravityWarpsFor(n, gravityVariant(mode, true, 0.5f))));
+        }));
+        AG_LAUNCH(launchBuildNeighbors(ws->w, n, sms, LaunchAt(st, share), static_cast<int>(tuningFor(n).neighborWarps), true));
+        if (sorted) AG_LAUNCH(launchPass1(*p, ws->w, n, LaunchAt(st, share)));
+        AG_LAUNCH(launchEos(*p, nullptr, n, LaunchAt(st, share)));
+        AG_CUDA(walks.join());
+        return pass2Forces(p, bvh, true);
     };
-    auto build = [&]() -> AstraeaStatus {
-        AstraeaStatus r = astraea_gb300_sort_and_build_bvh(p, alt, bvh);
-        if (r == ASTRAEA_OK) r = astraea_gb300_sph_pass1_neighbors(p, bvh);
-        return r;
-    };
+    auto build = [&]() -> AstraeaStatus { return astraea_gb300_sort_and_build_bvh(p, alt, bvh); };
     float prevDt = 0.0f;
     auto step = [&]() -> AstraeaStatus {                                     // :604-616
         float dt = 0.0f;
@@ -1594,19 +1641,8 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
     };
     // (timed stages run one after the other)
     const bool beside = n >= 2u && !learned && marks.ev == nullptr, share = beside && n <= kShareMax;
-    struct Join {                      // also where a launch in between fails
-        cudaStream_t st;
-        cudaEvent_t ev;
-        ~Join() { if (ev != nullptr) (void)cudaStreamWaitEvent(st, ev, 0); }
-    } join{st, nullptr};
-    if (beside) {
-        AG_CUDA(cudaEventRecord(ws->forked, st));
-        AG_CUDA(cudaStreamWaitEvent(ws->side, ws->forked, 0));
-        const cudaError_t e = gravity(LaunchAt(ws->side, share));
-        AG_CUDA(cudaEventRecord(ws->joined, ws->side));
-        join.ev = ws->joined;
-        AG_LAUNCH(e);
-    }
+    Beside walks(ws, st);
+    if (beside) AG_LAUNCH(walks.fork(share, gravity));
     // 4. neighbour lists for pass 1, pass 2 and the next drift
     marks.mark(ASTRAEA_STAGE_NEIGHBOURS);
     AG_LAUNCH(launchBuildNeighbors(w, n, sms, LaunchAt(st, share), static_cast<int>(tune.neighborWarps), true));
@@ -1616,8 +1652,7 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
     AG_LAUNCH(launchEos(*p, &w, n, LaunchAt(st, share)));
     marks.mark(ASTRAEA_STAGE_GRAVITY);
     if (beside) {
-        join.ev = nullptr;
-        AG_CUDA(cudaStreamWaitEvent(st, ws->joined, 0));
+        AG_CUDA(walks.join());
     } else if (learned) {
         s = learnedGravity(p, ws, n, theta, true);
         if (s != ASTRAEA_OK) return s;
