@@ -16,7 +16,8 @@
 //     has both children's COM, mass, size and reference in two loads, already
 //     in the register pairs of the packed FP32 pipes; a leaf child brings its
 //     particle, so a leaf is never loaded again.  32 opened nodes (64
-//     children) are taken a round, and the stack holds opened nodes only;
+//     children) are taken a round (the monopole walk, gravityOrderedKernel: 16
+//     nodes, a child a lane), and the stack holds opened nodes only;
 //   * a child is accepted when a sound lower bound on every member's distance
 //     to its COM (the larger of the group-box distance and the distance to the
 //     supporting plane of the group in the octant diagonal the COM lies in)
@@ -24,7 +25,8 @@
 //     furthest in that diagonal fails; the members and planes of the eight
 //     diagonals are found once a group;
 //   * children neither decides wait in a ring in shared memory; 32 of them at
-//     a time, one a lane, are tested exactly against every member;
+//     a time, one a lane, are tested exactly against every member (the monopole
+//     walk: in their round, a member a lane);
 //   * accepted monopoles and reached leaves are appended to two per-warp
 //     interaction lists in shared memory; every 32 entries the warp evaluates
 //     them with each lane summing its own particle's force from broadcast
@@ -32,11 +34,11 @@
 //     pipes (add/mul/fma.rn.f32x2) plus one rsqrt per pair;
 //   * a persistent grid pulls groups from an atomic counter.
 // 1M impact, theta 0.5, per group of 32: 1,600 opened nodes, 2,940 tested
-// children of which 295 wait for the exact test, 51,254 interactions; warp
-// instructions at 262k 46.1k -> 32.5k a group, of which the evaluation is about
-// half (it runs at the FP32 pipes' rate); launch 1.69 -> 1.34 ms (quadrupole,
-// theta 0.7: 1.63 -> 1.35; 4M Plummer sphere, quadrupole: 9.5 -> 7.9; 60k
-// spheres: 139 -> 110 us), of which the records of the children cost 0.04 ms.
+// children of which 295 wait for the exact test, 51,254 interactions; the
+// evaluation, at the FP32 pipes' rate, is about half of the instructions.  Launch at 1M: monopole,
+// theta 0.5, 1.69 -> 1.37 ms; quadrupole, theta 0.7, 1.63 -> 1.35; 4M Plummer
+// sphere, quadrupole, 9.5 -> 7.9; 60k spheres, monopole, 139 -> 120 us; of which the
+// records of the children cost 0.04 ms at 1M.
 #include <type_traits>
 
 #include "kernels.h"
@@ -917,42 +919,51 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
     }
 }
 
-// The monopole walk of scenes above kOrderedAbove particles: the same sets, with
-// the terms of a particle added in one fixed order -- rounds of 32 children (16
-// opened nodes), accepted nodes and leaves appended in the children's order,
-// undecided children settled within their round, each list evaluated when it
-// holds 32 -- which is the order the results of large scenes have always had.
-// gravityKernel adds in another order (64 children a round, undecided ones
-// later), which changes the last bit of a third of the accelerations; in a gas
-// giant impact at 32 km/s the velocities' last bits then change strain rates by
-// up to 1e-3 of their rms (17 of 24M components of dS above 8e-4 of it at 8M, none at
-// 1M or in the rocky scenes).  Bound, like that kernel, by instruction issue; it
-// shares the child records, the octant planes and the list layout, and takes the
-// 16M step from 59.8 to 57.1 ms (gravityKernel: 54.8).
-constexpr uint32_t kOrderedAbove = 1u << 20;
-constexpr int kOrdRing = 64, kOrdWarps = 4;
+// The monopole walk: the same sets, with the terms of a particle added in one
+// fixed order -- rounds of 32 children (16 opened nodes), accepted nodes and leaves
+// appended in the children's order, undecided children settled within their round,
+// each list evaluated when it holds 32 -- the order in which the library's results have always
+// been added up.  gravityKernel's order (64 children a round, undecided ones
+// later) changes the last bit of a third of the accelerations (at 1M it takes the
+// same time, at 60k 106 instead of 120 us), and a step amplifies that: in a
+// gas giant impact at 32 km/s the velocities' last bits move strain rates by up to
+// 1e-3 of their rms, and iron just below its melting point turns an ulp of rho
+// into 1e-4 of its strength.  Bound, like that kernel, by instruction issue; it
+// shares the child records, the octant planes and the list layout.  Against the walk over
+// nodes before it (one node a lane, leaves loaded again): 1M 1.69 -> 1.37 ms, 60k
+// 139 -> 120 us.  Resident warps per SM the registers are bounded for, 1M: theta 0.5
+// 28 1.54, 32 1.50, 36 1.40, 40 (spills) 1.42 ms; theta 0.7, whose box test needs more
+// registers, 24 1.07, 28 0.99, 32 1.01, 36 (spills) 1.04.
+constexpr int kOrdRing = 64;
 struct __align__(16) OrderedSmem {
     int stack[kGravStack];
     float mlist[4 * kOrdRing];
     float plist[5 * kOrdRing];
-    float und[4 * 32];                 // undecided children, field by field: COM, dNode^2
+    float4 und[32];                    // undecided children: COM, dNode^2
     int undRef[32];
     float4 dirPos[8];                  // see GravWarpSmem
 };
 static_assert(offsetof(OrderedSmem, mlist) % 16 == 0 && offsetof(OrderedSmem, plist) % 16 == 0 &&
               offsetof(OrderedSmem, und) % 16 == 0 && offsetof(OrderedSmem, dirPos) % 16 == 0, "vector loads");
-template <bool kInside>
-__global__ void __launch_bounds__(kOrdWarps * 32, 28 / kOrdWarps) gravityOrderedKernel(AstraeaParticles p, Work w, uint32_t n,
-                                                                                      float theta2, uint32_t numGroups,
-                                                                                      uint32_t* groupCounter) {
+template <int kWarps, bool kInside>
+__global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gravityOrderedKernel(AstraeaParticles p, Work w, uint32_t n,
+                                                                                float theta2, uint32_t numGroups,
+                                                                                uint32_t* groupCounter, FarCapture) {
     chained();
-    __shared__ OrderedSmem smem[kOrdWarps];
+    __shared__ OrderedSmem smem[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     OrderedSmem& S = smem[warp];
     unsigned long long nInter = 0;
     uint32_t nTests = 0, nUndecided = 0, nRounds = 0;
     int spPeak = 0;
     bool overflowed = false;
+    if (w.runIf != nullptr && *w.runIf == 0u) return;   // the gate of the learned mode passed
+    if (n == 1u) {                                   // sph_gravity.cu:824-832
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            p.accX[0] = 0.0f; p.accY[0] = 0.0f; p.accZ[0] = 0.0f; p.phiGrav[0] = 0.0f;
+        }
+        return;
+    }
     for (;;) {
         uint32_t g = 0;
         if (lane == 0) g = atomicAdd(groupCounter, 1u);
@@ -1041,15 +1052,16 @@ __global__ void __launch_bounds__(kOrdWarps * 32, 28 / kOrdWarps) gravityOrdered
                 const int nu = __popc(und), slot = __popc(und & laneMaskLt());
                 nUndecided += static_cast<uint32_t>(nu);
                 if (undecided) {
-                    S.und[slot] = x; S.und[32 + slot] = y; S.und[64 + slot] = z; S.und[96 + slot] = dd;
-                    S.undRef[slot] = ref;
+                    S.und[slot] = make_float4(x, y, z, dd);
+                    if (kInside) S.undRef[slot] = ref;
                 }
                 __syncwarp();
                 unsigned bits = 0u;
+#pragma unroll (kInside ? 2 : 1)
                 for (int k = 0; k < nu; ++k) {
-                    const float m2 = len2Engine(__fsub_rn(xi, S.und[k]), __fsub_rn(yi, S.und[32 + k]),
-                                                __fsub_rn(zi, S.und[64 + k]));
-                    bool ok = S.und[96 + k] < __fmul_rn(theta2, m2) && m2 > 1.0e-20f;
+                    const float4 q = S.und[k];
+                    const float m2 = len2Engine(__fsub_rn(xi, q.x), __fsub_rn(yi, q.y), __fsub_rn(zi, q.z));
+                    bool ok = q.w < __fmul_rn(theta2, m2) && m2 > 1.0e-20f;
                     if (kInside) {
                         const float4 mn = __ldg(&w.node[4 * static_cast<size_t>(S.undRef[k]) + 2]);
                         const float4 mx = __ldg(&w.node[4 * static_cast<size_t>(S.undRef[k]) + 3]);
@@ -1160,16 +1172,6 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     cudaError_t e = n >= 2u && w.runIf == nullptr ? launchChained(pairNodesKernel, (n - 1u + 255u) / 256u, 256, st, w, n)
                                                   : cudaMemsetAsync(counter, 0, sizeof(uint32_t), st.stream);
     if (e != cudaSuccess) return e;
-    if (n > kOrderedAbove && !quadrupole && far == nullptr && w.runIf == nullptr && w.traceList == nullptr &&
-        w.groupCounts == nullptr) {
-        const auto ordered = checkInside ? gravityOrderedKernel<true> : gravityOrderedKernel<false>;
-        int perSm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, ordered, kOrdWarps * 32, 0);
-        if (e != cudaSuccess) return e;
-        const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(std::max(1, perSm) * sms),
-                                                   (groups + kOrdWarps - 1) / kOrdWarps);
-        return launchChained(ordered, blocks, kOrdWarps * 32u, st, p, w, n, theta2, groups, counter);
-    }
     FarCapture ff{};
     using GravFn = void (*)(AstraeaParticles, Work, uint32_t, float, uint32_t, uint32_t*, FarCapture);
     GravFn kernel = nullptr;
@@ -1199,13 +1201,13 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     } else if (quadrupole) {
         kernel = checkInside ? gravityKernel<kGravWarps, true, true, false> : gravityKernel<kGravWarps, false, true, false>;
     } else if (warps == 2) {
-        kernel = checkInside ? gravityKernel<2, true, false, false> : gravityKernel<2, false, false, false>;
+        kernel = checkInside ? gravityOrderedKernel<2, true> : gravityOrderedKernel<2, false>;
         wps = 2;
     } else if (warps == 8) {
-        kernel = checkInside ? gravityKernel<8, true, false, false> : gravityKernel<8, false, false, false>;
+        kernel = checkInside ? gravityOrderedKernel<8, true> : gravityOrderedKernel<8, false>;
         wps = 8;
     } else {
-        kernel = checkInside ? gravityKernel<kGravWarps, true, false, false> : gravityKernel<kGravWarps, false, false, false>;
+        kernel = checkInside ? gravityOrderedKernel<kGravWarps, true> : gravityOrderedKernel<kGravWarps, false>;
     }
     int perSm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, wps * 32, 0);

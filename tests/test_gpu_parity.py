@@ -520,8 +520,8 @@ def test_gravity_walk_sets_at_edges(n, shape):
 @pytest.mark.parametrize("n", [(1 << 20) + 1, (1 << 20) + 63])
 @pytest.mark.parametrize("theta", [0.3, 0.5, 0.7])
 def test_gravity_walk_of_large_scenes(n, theta):
-    """Above 2^20 particles the terms are added in another order: the walk takes
-    the interactions of the general one, which the counting call runs, and the
+    """The monopole walk adds its terms in another order than the general one:
+    it takes the interactions of that walk, which the counting call runs, and the
     forces agree within the parity bound (they differ in rounding only)."""
     rng = np.random.default_rng(n)
     st = scenarios.empty_state(n)
