@@ -596,9 +596,10 @@ __device__ __forceinline__ void pass1Particle(const AstraeaParticles& p, const W
     w.driftAux[i] = make_float2(mi, 1.0f / Hd);
 }
 
-// 6 blocks per SM (80 registers): no spills; 7 blocks (72) spilled and ran 1.6 % slower
+// 7 blocks per SM (72 registers, 4 words spilled): 250 us at 1M, 74 at 262k; 6 blocks (80)
+// 267 and 82, 5 (84) 295 at 1M.
 template <int kLanes>
-__global__ void __launch_bounds__(kPassThreads, 6) pass1Kernel(AstraeaParticles p, Work w, uint32_t n) {
+__global__ void __launch_bounds__(kPassThreads, 7) pass1Kernel(AstraeaParticles p, Work w, uint32_t n) {
     chained();
     if (blockIdx.x < kHeavyBlocks) {
         const uint32_t lane = threadIdx.x & 31u, total = heavyCount(w);
@@ -956,7 +957,7 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st
 }
 
 // Lanes per particle of pass 1 and the drift: as many as keep all of the launch's
-// threads resident at once (6 blocks per SM x 128 x 152 SMs).  Below that a
+// threads resident at once (taken at 6 blocks per SM x 128 x 152 SMs).  Below that a
 // launch lasts as long as one thread's list; above it a lane more per particle
 // only adds sums and partial last fours.  Drift / pass 1 with 1, 2, 4 lanes, us:
 // n = 16k 41.6 / 26.6, 25.9 / 18.4, 19.4 / 15.4 (8 lanes: 24.6 / 18.4); 32k
