@@ -693,25 +693,34 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                 const bool farOk = !accept && isNode && emitFar && boxApart && Fb2 > 2.0e-20f &&
                                    dd < ff.thetaFar2 * Fb2 * 0.99999f &&
                                    gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);
-                unsigned todo = __ballot_sync(0xffffffffu, farOk);
+                // only an undecided one needs the exact test of every member here (a
+                // box of such a node holds no member)
+                bool all = false;
+                unsigned todo = __ballot_sync(0xffffffffu, farOk && undecided);
                 while (todo) {
                     const int src = __ffs(todo) - 1;
                     todo &= todo - 1u;
                     const float qx = __shfl_sync(0xffffffffu, x, src), qy = __shfl_sync(0xffffffffu, y, src),
                                 qz = __shfl_sync(0xffffffffu, z, src), qd = __shfl_sync(0xffffffffu, dd, src);
                     const float m2 = len2Engine(__fsub_rn(xi, qx), __fsub_rn(yi, qy), __fsub_rn(zi, qz));
-                    // boxApart holds for it: no member is inside its box
-                    const bool all = __all_sync(0xffffffffu, !active || (qd < __fmul_rn(theta2, m2) && m2 > 1.0e-20f));
-                    uint32_t slot = 0xffffffffu;
-                    if (!all && lane == src) {
-                        slot = atomicAdd(ff.count, 1u);
-                        if (slot < ff.cap) ff.pairs[slot] = make_uint2(g, static_cast<uint32_t>(ref));
+                    const bool each = __all_sync(0xffffffffu, !active || (qd < __fmul_rn(theta2, m2) && m2 > 1.0e-20f));
+                    if (lane == src) all = each;
+                }
+                const unsigned take = __ballot_sync(0xffffffffu, farOk && !all);
+                if (take) {
+                    uint32_t first = 0;
+                    if (lane == 0) first = atomicAdd(ff.count, static_cast<uint32_t>(__popc(take)));
+                    first = __shfl_sync(0xffffffffu, first, 0);
+                    const uint32_t slot = first + static_cast<uint32_t>(__popc(take & laneMaskLt()));
+                    if (farOk && !all && slot < ff.cap) {           // full buffer: the node is opened
+                        ff.pairs[slot] = make_uint2(g, static_cast<uint32_t>(ref));
+                        all = true;
                     }
-                    if (lane == src) {
-                        accept = all || slot < ff.cap;       // full buffer: the node is opened
-                        open = !accept;
-                        undecided = false;
-                    }
+                }
+                if (farOk) {
+                    accept = all;
+                    open = !all;
+                    undecided = false;
                 }
             }
         };
