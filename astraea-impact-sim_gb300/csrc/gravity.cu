@@ -655,22 +655,19 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             const float r2 = len2Engine(__fsub_rn(dp.x, x), __fsub_rn(dp.y, y), __fsub_rn(dp.z, z));
             bool boundAccepts = Lb2 > 2.0e-20f && dd < theta2 * Lb2;
             bool extreme = dd < __fmul_rn(theta2, r2) && r2 > 1.0e-20f;     // the engine's test, without its box
-            bool boxApart = true;               // no member can lie in the node's box
-            if (kInside || kLearned) {
-                // the box is only looked at where a member may be as near the
-                // COM as its furthest corner
-                if (isNode && (kLearned || ((boundAccepts || extreme) && !(Lb2 > far2)))) {
-                    const float4 bmin = __ldg(&w.node[4 * static_cast<size_t>(ref) + 2]);
-                    const float4 bmax = __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]);
-                    boxApart = bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy || bmax.z < gminz ||
-                               bmin.z > gmaxz;
-                    if (kInside) {
-                        boundAccepts = boundAccepts && boxApart;
-                        if (dp.x >= bmin.x && dp.x <= bmax.x && dp.y >= bmin.y && dp.y <= bmax.y && dp.z >= bmin.z &&
-                            dp.z <= bmax.z)
-                            extreme = false;
-                    }
-                }
+            auto apart = [&](const float4& bmin, const float4& bmax) {    // the group's box from the node's
+                return bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy || bmax.z < gminz ||
+                       bmin.z > gmaxz;
+            };
+            // the box is only looked at where a member may be as near the
+            // COM as its furthest corner
+            if (kInside && isNode && (boundAccepts || extreme) && !(Lb2 > far2)) {
+                const float4 bmin = __ldg(&w.node[4 * static_cast<size_t>(ref) + 2]);
+                const float4 bmax = __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]);
+                boundAccepts = boundAccepts && apart(bmin, bmax);
+                if (dp.x >= bmin.x && dp.x <= bmax.x && dp.y >= bmin.y && dp.y <= bmax.y && dp.z >= bmin.z &&
+                    dp.z <= bmax.z)
+                    extreme = false;
             }
             accept = isNode && boundAccepts;
             undecided = isNode && !boundAccepts && extreme;
@@ -690,9 +687,10 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                                      invDirNorm(abs(sx) + abs(sy) + abs(sz)) -
                                  S.farDir[13 + 9 * sx + 3 * sy + sz].w - 1.0e-6f * (ax + ay + az + gExt);
                 const float Fb2 = fmaxf(gx * gx + gy * gy + gz * gz, Lf > 0.0f ? Lf * Lf : 0.0f);
-                const bool farOk = !accept && isNode && emitFar && boxApart && Fb2 > 2.0e-20f &&
-                                   dd < ff.thetaFar2 * Fb2 * 0.99999f &&
-                                   gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);
+                bool farOk = !accept && isNode && emitFar && Fb2 > 2.0e-20f && dd < ff.thetaFar2 * Fb2 * 0.99999f &&
+                             gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);
+                if (farOk)                       // and the boxes are apart
+                    farOk = apart(__ldg(&w.node[4 * static_cast<size_t>(ref) + 2]), __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]));
                 // only an undecided one needs the exact test of every member here (a
                 // box of such a node holds no member)
                 bool all = false;
