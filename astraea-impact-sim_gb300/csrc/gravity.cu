@@ -371,9 +371,9 @@ __global__ void __launch_bounds__(256) pairNodesKernel(Work w, uint32_t n) {
 // counts, the trace of one group's accepted nodes and leaves); their checks
 // are kept out of the production variants, where they cost 2 % of the walk.
 // kWarpsPerSm: the resident warps the registers are bounded for (72, 80 and 96
-// registers, no spills).  At 1M, theta 0.5: 28 warps 1.39 ms, 24 1.43, 32 (spills)
-// 1.41; quadrupole, theta 0.7: 24 warps 1.36, 20 1.44; expansion: 20 warps 1.58,
-// 16 1.63, 24 (spills) 1.91.
+// registers).  At 1M: quadrupole, theta 0.7, 24 warps 1.36 ms, 20 1.44 (4M Plummer
+// sphere 7.94, 28 with spills 8.08); expansion, theta 0.7, 20 warps 1.55, 16 1.64, 24
+// (spills) 1.62; learned, the walk alone, 28 warps 1.37, 24 1.42, 20 1.42, 32 1.46.
 template <bool kQuad, bool kExpand>
 constexpr int kWarpsPerSm = kExpand ? 20 : (kQuad ? 24 : 28);
 template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = false, bool kDebug = false>
