@@ -60,8 +60,8 @@ __device__ __forceinline__ void storeIf(uint32_t* p, uint32_t v, bool pred) {
                  :: "l"(p), "r"(v), "r"(static_cast<uint32_t>(pred)));
 }
 
-template <int kWarps>
-__global__ void __launch_bounds__(kWarps * 32) buildNeighborsKernel(Work w, uint32_t n, uint32_t numGroups,
+template <int kWarps, int kMinBlocks>
+__global__ void __launch_bounds__(kWarps * 32, kMinBlocks) buildNeighborsKernel(Work w, uint32_t n, uint32_t numGroups,
                                                                     uint32_t* groupCounter) {
     chained();
     __shared__ NbWarpSmem smem[kWarps];
@@ -936,6 +936,12 @@ inline unsigned gridFor(uint32_t n, int block) { return static_cast<unsigned>((n
 
 }  // namespace
 
+// Registers of the group walk: 64 (kMinBlocks for 32 warps per SM) while there are few
+// groups, 56 (36 warps) above.  Pass-1 stage call, 56 / 64 registers: 30k 107 /
+// 102 us, 60k 135 / 129, 262k 305 / 300, 400k 428 / 422, 600k 599 / 599, 800k 768 / 769;
+// build alone at 1M 639 / 652.
+constexpr uint32_t kRoomyMax = 1u << 19;
+
 cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st, int warps, bool armed) {
     if (n == 0) return cudaSuccess;
     const uint32_t groups = (n + 31u) / 32u;
@@ -944,8 +950,10 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st
     if (e != cudaSuccess) return e;
     using NbFn = void (*)(Work, uint32_t, uint32_t, uint32_t*);
     const int wps = (warps == 2 || warps == 8) ? warps : kNbWarps;
-    const NbFn kernel = (wps == 2) ? buildNeighborsKernel<2> : (wps == 8) ? buildNeighborsKernel<8>
-                                                                         : buildNeighborsKernel<kNbWarps>;
+    const bool few = n <= kRoomyMax;
+    const NbFn kernel = (wps == 2)   ? (few ? buildNeighborsKernel<2, 16> : buildNeighborsKernel<2, 0>)
+                        : (wps == 8) ? (few ? buildNeighborsKernel<8, 4> : buildNeighborsKernel<8, 0>)
+                                     : (few ? buildNeighborsKernel<kNbWarps, 8> : buildNeighborsKernel<kNbWarps, 0>);
     int perSm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, wps * 32, 0);
     if (e != cudaSuccess) return e;
