@@ -47,7 +47,12 @@ namespace astraea_gb300 {
 namespace {
 
 constexpr int kGravWarps = 4;
-constexpr int kGravStack = 448;           // opened nodes per warp (peak use: 206 at 1M, 253 on the 1M Plummer sphere)
+// Opened nodes per warp.  Peak use of gravityOrderedKernel / gravityKernel: 1M impact,
+// theta 0.5, 133 / 156; 4M Plummer sphere, theta 0.5, 208 / 282, theta 0.1, full / 359.
+// gravityKernel takes smaller rounds as it fills (walkWidth): without that it ran out at theta 0.2 on the Plummer spheres of 1M and
+// 4M (forces wrong by 2e-2); with it 30.3 -> 31.8 and 150 -> 163 ms there, 698 -> 836 at
+// theta 0.1 (4M), and no difference from theta 0.5 up.
+constexpr int kGravStack = 448;
 // Ring lists: a round appends up to 64 entries behind at most 31 pending ones.
 // The quadrupole's monopole entries are 40 bytes: its list (and mode 3's far
 // list) is emptied between a round's two halves instead.
@@ -612,8 +617,9 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             const uint2 brA = bucketOf(openA, A), brB = kTwo ? bucketOf(openB, B) : make_uint2(1u, 0u);
             unsigned mA = __ballot_sync(0xffffffffu, openA), mB = kTwo ? __ballot_sync(0xffffffffu, openB) : 0u;
             if (sp + __popc(mA) + __popc(mB) > kGravStack) {
-                // Out of stack: the group takes these nodes as monopoles, the
-                // rule of the engine kernel when its stack is full (:933).
+                // Out of stack, only on a corrupted tree (walkWidth): the group takes
+                // these nodes as monopoles, the rule of the engine kernel when its
+                // stack is full (:933).
                 accA = accA || openA;
                 accB = accB || openB;
                 openA = openB = false;
@@ -727,7 +733,9 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                 overflowed = true;
                 break;
             }
-            if (uCount >= 32 || sp == 0) {
+            // every undecided child may still be opened
+            const int width = walkWidth<kGravStack>(sp + uCount);
+            if (uCount >= 32 || sp == 0 || (width == 1 && uCount > 0)) {
                 // The oldest undecided children, up to 32, one a lane, against every
                 // member: the engine's member test (sph_gravity.cu:914-929) with
                 // the engine's rounding of r^2 (len2Engine's operations, packed).
@@ -787,7 +795,7 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             }
             // open up to 32 nodes: both children of each
             spPeak = max(spPeak, sp);
-            const int take = min(sp, 32);
+            const int take = min(sp, width);
             sp -= take;
             int node = (lane < take) ? S.stack[sp + lane] : 0;
             __syncwarp();

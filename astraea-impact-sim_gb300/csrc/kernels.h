@@ -27,6 +27,20 @@ __device__ __forceinline__ float warpSumF(float v) {
     return v;
 }
 
+// Nodes a warp takes off its stack in one round of a walk, `load` of the
+// kStack entries being in use.  A round of 32 leaves up to 32 entries more than
+// before on every level of the tree it comes down; a walk that opens nearly
+// everything of a deep tree would run out.  So rounds get smaller as the stack
+// fills, down to one node, a depth-first walk, which adds at most one entry a
+// level: no path from the root is longer than 63 code bits and 30 of the index
+// that tells equal codes apart, less than kWalkReserve.
+constexpr int kWalkReserve = 96;
+template <int kStack>
+__device__ __forceinline__ int walkWidth(int load) {
+    static_assert(kStack / 2 + 64 <= kStack - kWalkReserve - 8, "a full round and a small one fit below the reserve");
+    return load <= kStack / 2 + 32 ? 32 : (load <= kStack - kWalkReserve - 8 ? 8 : 1);
+}
+
 // Reduce each thread's partial AABB over the block and merge it into the
 // ordered-uint bound words with atomics (engine/sph_gravity.cu:300-324).
 // Every thread of the block must call it.

@@ -1,0 +1,117 @@
+"""Tree walks at the ends of their scratch: deep, wide trees against the walks'
+stacks.
+
+A scene is given by its particles' 63-bit Morton codes: coordinates are whole
+numbers of 2^-17 between 0 and 2^21 - 1, so the codes are reproduced exactly and
+the tree is the one the codes spell.  `spines` spells 2^bits paths of `levels`
+right turns with a balanced clump of 2^leg particles beside each: every level of
+it leaves a batched walk with nodes it has yet to come back to.
+"""
+import numpy as np
+import pytest
+import torch
+
+from astraea_gb300 import engine, scenarios
+from conftest import rel_rms
+
+pytestmark = pytest.mark.gpu
+CELL = 2.0 ** -17
+
+
+def spines(bits, levels, leg):
+    out = []
+    for c in range(1 << bits):
+        for k in range(levels):
+            path = (c << (k + 1)) | (((1 << k) - 1) << 1)
+            used = bits + k + 1 + leg
+            out += [((path << leg) | x) << (63 - used) for x in range(1 << leg)]
+        out.append((c << (63 - bits)) | ((1 << (63 - bits)) - 1))
+    return sorted(out)
+
+
+def scene(codes):
+    n = len(codes)
+    c = np.array(codes, np.uint64)
+    st = scenarios.empty_state(n)
+    for k, f in enumerate(("posX", "posY", "posZ")):
+        q = np.zeros(n, np.uint64)
+        for b in range(21):
+            q |= ((c >> np.uint64(3 * b + 2 - k)) & np.uint64(1)) << np.uint64(b)
+        st[f][:] = q.astype(np.float32) * np.float32(CELL)
+    st["mass"][:] = 1.0 / n
+    st["h"][:] = st["h0"][:] = 1.0e-5
+    st["rho"][:] = 1.0e-3
+    st["materialId"][:] = 1
+    st["originalId"][:] = np.arange(n, dtype=np.uint32)
+    return st
+
+
+def device_setup(st):
+    n = len(st["posX"])
+    p, alt, bvh = engine.DeviceParticles(n), engine.DeviceParticles(n), engine.TorchBvh(n)
+    p.upload(st)
+    alt.count = n
+    return p, alt, bvh
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("bits,levels", [(5, 20), (5, 57), (0, 60)])
+def test_gravity_walks_open_everything_on_deep_trees(mode, bits, levels):
+    """At opening angle 0 every node is opened, whatever the tree leaves on the
+    stack (a group that runs out of it takes nodes as monopoles instead): exactly
+    n (n - 1) interactions.  The learned mode may still take nodes that are tiny
+    against their distance; it only must not run out."""
+    st = scene(spines(bits, levels, 1))
+    n = len(st["posX"])
+    p, alt, bvh = device_setup(st)
+    try:
+        engine.set_far_field(mode)
+        engine.set_far_field_expansion(0, 0.3)
+        if mode == 2:
+            engine.ff_init(1)
+            engine.ff_configure(theta_far=1.0e-6, gamma=0.3)
+        engine.sort_and_build_bvh(p, alt, bvh)
+        engine.reset_device_status()
+        engine.gravity_barnes_hut(p, bvh, 0.0)
+        flags, counters = engine.read_device_status()
+    finally:
+        engine.set_far_field(0)
+        engine.set_far_field_expansion(16, 0.3)
+        engine.ff_configure()
+    assert flags == 0
+    if mode != 2:
+        assert counters["gravity_interactions"] == n * (n - 1)
+
+
+@pytest.mark.parametrize("mode", [1, 3])
+def test_gravity_small_opening_angle(mode):
+    """A million particles at opening angle 0.1: no group runs out of stack, and
+    the quadrupole walk's forces on sampled particles are within the error that
+    angle has (below 1e-4; a group out of stack puts it above 1e-3)."""
+    n = 1 << 20
+    rng = np.random.default_rng(3)
+    st = scenarios.empty_state(n)
+    r = (rng.uniform(1.0e-6, 0.999, n) ** (-2.0 / 3.0) - 1.0) ** -0.5          # Plummer sphere
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    for k, f in enumerate(("posX", "posY", "posZ")):
+        st[f][:] = r * u[:, k]
+    st["mass"][:] = 1.0 / n
+    st["h"][:] = st["h0"][:] = 0.01
+    st["rho"][:] = 1.0e-3
+    p, alt, bvh = device_setup(st)
+    try:
+        engine.set_far_field(mode)
+        engine.sort_and_build_bvh(p, alt, bvh)
+        engine.reset_device_status()
+        engine.gravity_barnes_hut(p, bvh, 0.1)
+        flags, counters = engine.read_device_status()
+    finally:
+        engine.set_far_field(0)
+    g = p.download(["accX", "accY", "accZ"])
+    sel = rng.choice(n, 512, replace=False).astype(np.uint32)
+    ref = engine.direct_gravity_f64(p, torch.from_numpy(sel.astype(np.int64)))[0].cpu().numpy()
+    a = np.stack([g[f][sel] for f in ("accX", "accY", "accZ")], 1)
+    assert flags == 0
+    if mode == 1:                                       # mode 3 adds its expansion's error
+        assert rel_rms(a, ref) < 3e-4
