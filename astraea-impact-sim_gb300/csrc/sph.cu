@@ -28,7 +28,7 @@ namespace astraea_gb300 {
 namespace {
 
 constexpr int kNbWarps = 4;
-constexpr int kNbStack = 384;   // entries per warp (peak use: 80 at 1M, 88 at 16M)
+constexpr int kNbStack = 384;   // entries per warp (peak use: 80 at 1M, 88 at 16M; walkWidth keeps any tree's below it)
 constexpr int kNbList = 64;
 constexpr uint32_t kNbExpand = 32;   // an opened node of at most this many particles is read as its leaf range
 
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) buildNeighborsKernel(
                 stackOverflow = true;
                 break;
             }
-            const int take = min(sp, 32);
+            const int take = min(sp, walkWidth<kNbStack>(sp));
             const int c = (lane < take) ? S.stack[sp - take + lane] : 0;
             sp -= take;
             __syncwarp();
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) buildNeighborsKernel(
             unsigned expandMask = __ballot_sync(0xffffffffu, rng.x <= rng.y);
             unsigned openMask = __ballot_sync(0xffffffffu, open);
             if (sp + 2 * __popc(openMask) > kNbStack) {
-                stackOverflow = true;     // cannot happen for trees of depth < 32
+                stackOverflow = true;     // only on a corrupted tree (walkWidth)
                 openMask = 0u;
                 open = false;
             }
@@ -447,7 +447,7 @@ __device__ __forceinline__ void addCount(DevStatus* st, int which, uint32_t v) {
 // The lists in the pool: a warp per particle walks the tree with its own radius,
 // 32 nodes at a time from a stack in shared memory, and appends the particles
 // inside, which are those the group walk counted (the node test has the same
-// margin; a list never grows past its count).  Latency bound: a walk is some
+// margin); a list that came out longer or was cut is not used.  Latency bound: a walk is some
 // twenty rounds of two dependent loads, and there are few of them; almost always
 // there is none, and the launch, chained to the kernels around it, costs less than 1 us
 // (2.5 to 4 as a plain one).
@@ -470,11 +470,16 @@ __global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint3
         const float4 me = __ldg(&w.leaf[h.x].a);
         uint32_t* list = w.pool + place;
         uint32_t cnt = 0u, rounds = 0u;
+        bool whole = true;
         int sp = 1;
         if (lane == 0u) stack[0] = 0;
         __syncwarp();
-        while (sp > 0 && ++rounds <= 2u * n) {
-            const int take = min(sp, 32);
+        while (sp > 0) {
+            if (++rounds > 2u * n) {                        // only on a corrupted tree
+                whole = false;
+                break;
+            }
+            const int take = min(sp, walkWidth<kPoolStack>(sp));
             const int c = static_cast<int>(lane) < take ? stack[sp - take + lane] : static_cast<int>(n);
             sp -= take;
             __syncwarp();
@@ -500,8 +505,8 @@ __global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint3
             const uint32_t at = cnt + __popc(hits & laneMaskLt());
             if (hit && at < h.z) list[at] = hitJ;
             cnt += __popc(hits);
-            if (sp + 2 * __popc(opens) > kPoolStack) {      // cannot happen for trees of depth < 32
-                if (lane == 0u) atomicOr(&w.status->flags, kFlagStackOverflow);
+            if (sp + 2 * __popc(opens) > kPoolStack) {      // only on a corrupted tree (walkWidth)
+                whole = false;
                 break;
             }
             if (open) {
@@ -513,8 +518,13 @@ __global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint3
             __syncwarp();
         }
         if (lane == 0u) {
-            w.heavy[e] = make_uint4(h.x, static_cast<uint32_t>(place), min(cnt, h.z), 0u);
-            w.nbrCount[h.x] = kHeavyMark;
+            if (whole && cnt <= h.z && cnt != 0u) {
+                w.heavy[e] = make_uint4(h.x, static_cast<uint32_t>(place), cnt, 0u);
+                w.nbrCount[h.x] = kHeavyMark;
+            } else {                                        // its own walk then, as without a place
+                w.heavy[e].z = 0u;
+                if (!whole) atomicOr(&w.status->flags, kFlagStackOverflow);
+            }
         }
         __syncwarp();
     }

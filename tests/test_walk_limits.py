@@ -10,8 +10,10 @@ it leaves a batched walk with nodes it has yet to come back to.
 import numpy as np
 import pytest
 import torch
+from scipy.spatial import cKDTree
 
-from astraea_gb300 import engine, scenarios
+import oracle
+from astraea_gb300 import abi, engine, scenarios
 from conftest import rel_rms
 
 pytestmark = pytest.mark.gpu
@@ -115,3 +117,34 @@ def test_gravity_small_opening_angle(mode):
     assert flags == 0
     if mode == 1:                                       # mode 3 adds its expansion's error
         assert rel_rms(a, ref) < 3e-4
+
+
+@pytest.mark.parametrize("bits,levels,leg", [(1, 40, 6), (0, 24, 10), (0, 24, 12)])
+def test_long_lists_of_deep_trees_are_whole(bits, levels, leg):
+    """One particle reaches the whole scene: the group walk and the walk that
+    fills its list in the pool open every node of a tree that leaves more on their
+    stacks than those hold.  Every pair within range is visited, by count."""
+    st = scene(spines(bits, levels, leg))
+    n = len(st["posX"])
+    big = n // 3
+    st["h"][big] = st["h0"][big] = 40.0
+    p, alt, bvh = device_setup(st)
+    engine.sort_and_build_bvh(p, alt, bvh)
+    engine.reset_device_status()
+    engine.sph_pass1_neighbors(p, bvh)
+    flags, counters = engine.read_device_status()
+    o = oracle.Oracle(st)
+    o.sort_and_build()
+    o.pass1()
+    g, c = p.download(), o.state()
+    i = int(np.flatnonzero(g["originalId"] == big)[0])
+    assert flags == abi.DEVFLAG_NEIGHBOR_OVERFLOW
+    assert counters["fallback_walks"] == 0
+    assert g["h"][i] == c["h"][i]
+    x = np.stack([c[f] for f in ("posX", "posY", "posZ")], 1).astype(np.float64)
+    assert np.linalg.norm(x - x[i], axis=1).max() < 2.0 * 40.0
+    near = cKDTree(x).query_pairs(2.0e-5, output_type="ndarray")             # 2 h of all others
+    pairs = n - 1 + 2 * len(near) - int(np.count_nonzero(near == i))
+    assert engine.read_device_counters()["pass1_pairs"] == pairs
+    for f in ("h", "shepardC", "surfFactor"):
+        assert rel_rms(g[f], c[f]) < 1e-5, f
