@@ -183,8 +183,11 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     const size_t oDrift = take(C * 16);
     const size_t oDRec = take(C * 32), oDAux = take(C * 8);
     const size_t oCnt = take(C * 4), oList = take((C + 31) / 32 * 32 * maxNbr * 4);
-    // lists above maxNbr entries: rare; what does not fit here is walked in each pass
-    const size_t heavyCap = C / 64 + 256, poolCap = std::min<size_t>(C * 4 + 65536, 0xfffffff0u);
+    // Lists above maxNbr entries, all of them or none (sph.cu, heavyCount): one
+    // particle in sixteen with 384 entries each.  Pass 1 and 2 with 1 % / 3 % of
+    // a million particles at 2.5 / 2 times their h: 7.3 / 10.8 ms, walked 18.2 / 19.4,
+    // and 15.7 / 18.3 where a pool of a sixth of this served those that came first.
+    const size_t heavyCap = C / 16 + 256, poolCap = std::min<size_t>(C * 24 + 65536, 0xfffffff0u);
     const size_t oHeavy = take(heavyCap * 16), oPool = take(poolCap * 4), oWords = take(kWCount * 4);
     const size_t oSort = take(sortWords * 4), oDt = take(64);
     void* block = nullptr;

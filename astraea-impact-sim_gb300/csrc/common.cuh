@@ -549,7 +549,7 @@ struct Work {
     float2* driftAux;      // {m, 1 / H}
     uint32_t* nbrCount;    // entries of each list; above maxNbr: no list (kHeavyMark: one in the pool)
     uint32_t* nbrList;     // group-interleaved: entry k of particle i at ((i/32) maxNbr + k) 32 + i%32
-    uint4* heavy;          // lists in the pool: {particle, first word, entries (0: no place), 0}
+    uint4* heavy;          // lists in the pool: {particle, first word, entries (0: not finished), 0}
     uint32_t heavyCap;
     uint32_t* pool;
     uint32_t poolCap;      // words

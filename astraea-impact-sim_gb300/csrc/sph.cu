@@ -20,8 +20,8 @@
 //     large h beside a dense body has thousands of neighbours) gets a list in a
 //     shared pool, and whole warps work on those lists in the first blocks of
 //     each pass: one thread over such a list holds up the launch.
-// When the pool is exhausted too, a particle is served by a per-thread
-// depth-first walk with the same superset test.
+// Where the pool does not hold all of those lists, each of their particles is
+// served by a per-thread depth-first walk with the same superset test.
 #include "kernels.h"
 
 namespace astraea_gb300 {
@@ -58,6 +58,21 @@ __device__ __forceinline__ uint32_t laneMaskLt() {
 __device__ __forceinline__ void storeIf(uint32_t* p, uint32_t v, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.u32 [%0], %1;\n\t}"
                  :: "l"(p), "r"(v), "r"(static_cast<uint32_t>(pred)));
+}
+
+// Pool words that the long lists ask for (64 bits: their sum can pass 2^32).
+__device__ __forceinline__ unsigned long long* poolUsed(const Work& w) {
+    return reinterpret_cast<unsigned long long*>(&w.words[kWPoolUsed]);
+}
+// Lists in the pool: all the long ones, or none where they do not all have a
+// place.  Which of them come first is a matter of timing, and a particle's terms
+// are added in another order with a list (32 lanes) than without (one thread's
+// walk).  Lists for some would gain little: a launch lasts as long as its longest
+// walk (20k particles, 1 % at 2.5 times their h, a quarter of them walked 3.25
+// ms, all walked 3.20, none 0.51).
+__device__ __forceinline__ uint32_t heavyCount(const Work& w) {
+    const uint32_t count = __ldg(&w.words[kWHeavyCount]);
+    return count <= w.heavyCap && __ldg(poolUsed(w)) <= w.poolCap ? count : 0u;
 }
 
 template <int kWarps, int kMinBlocks>
@@ -307,8 +322,9 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) buildNeighborsKernel(
             w.nbrCount[i] = cnt;
             if (cnt > maxNbr) {                     // poolListsKernel goes on with it
                 overflow = true;
+                const unsigned long long place = atomicAdd(poolUsed(w), static_cast<unsigned long long>(cnt));
                 const uint32_t slot = atomicAdd(&w.words[kWHeavyCount], 1u);
-                if (slot < w.heavyCap) w.heavy[slot] = make_uint4(i, 0u, cnt, 0u);
+                if (slot < w.heavyCap) w.heavy[slot] = make_uint4(i, static_cast<uint32_t>(place), cnt, 0u);
             }
         }
         nEntries += cnt;
@@ -433,7 +449,6 @@ __device__ __forceinline__ void sumLanes(uint32_t& v) {
 // per particle; then kLanes threads per particle.
 constexpr uint32_t kHeavyBlocks = 38, kPassThreads = 128;
 constexpr uint32_t kHeavyWarps = kHeavyBlocks * kPassThreads / 32;
-__device__ __forceinline__ uint32_t heavyCount(const Work& w) { return min(__ldg(&w.words[kWHeavyCount]), w.heavyCap); }
 
 // Adds a per-thread count to a device counter with one atomic per group of
 // threads that reach the call together (the running threads of a warp).
@@ -459,16 +474,8 @@ __global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint3
     int* stack = stacks[threadIdx.x >> 5];
     for (uint32_t e = blockIdx.x * kPoolWarps + (threadIdx.x >> 5); e < total; e += gridDim.x * kPoolWarps) {
         const uint4 h = w.heavy[e];
-        unsigned long long place = 0;                    // 64 bits: the sum of what is asked for can pass 2^32
-        if (lane == 0u)
-            place = atomicAdd(reinterpret_cast<unsigned long long*>(&w.words[kWPoolUsed]), static_cast<unsigned long long>(h.z));
-        place = __shfl_sync(0xffffffffu, place, 0);
-        if (place + h.z > w.poolCap) {                 // served by its own walk in each pass
-            if (lane == 0u) w.heavy[e].z = 0u;
-            continue;
-        }
         const float4 me = __ldg(&w.leaf[h.x].a);
-        uint32_t* list = w.pool + place;
+        uint32_t* list = w.pool + h.y;
         uint32_t cnt = 0u, rounds = 0u;
         bool whole = true;
         int sp = 1;
@@ -519,9 +526,9 @@ __global__ void __launch_bounds__(kPoolWarps * 32) poolListsKernel(Work w, uint3
         }
         if (lane == 0u) {
             if (whole && cnt <= h.z && cnt != 0u) {
-                w.heavy[e] = make_uint4(h.x, static_cast<uint32_t>(place), cnt, 0u);
+                w.heavy[e].z = cnt;
                 w.nbrCount[h.x] = kHeavyMark;
-            } else {                                        // its own walk then, as without a place
+            } else {                                        // its own walk then, as without a pool
                 w.heavy[e].z = 0u;
                 if (!whole) atomicOr(&w.status->flags, kFlagStackOverflow);
             }

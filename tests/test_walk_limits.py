@@ -1,5 +1,5 @@
 """Tree walks at the ends of their scratch: deep, wide trees against the walks'
-stacks.
+stacks, and more long neighbour lists than the shared pool holds.
 
 A scene is given by its particles' 63-bit Morton codes: coordinates are whole
 numbers of 2^-17 between 0 and 2^21 - 1, so the codes are reproduced exactly and
@@ -148,3 +148,45 @@ def test_long_lists_of_deep_trees_are_whole(bits, levels, leg):
     assert engine.read_device_counters()["pass1_pairs"] == pairs
     for f in ("h", "shepardC", "surfFactor"):
         assert rel_rms(g[f], c[f]) < 1e-5, f
+
+
+@pytest.mark.parametrize("n,every", [(2000, 33), (4000, 10)])
+def test_lists_that_do_not_fit_the_pool(n, every):
+    """More long lists than the pool has words for (61 of 1,999 entries; it has
+    113,536) or places (all 4,000 particles, each within reach of 400 long ones; it
+    has 506): no particle's sums may then depend on which of them came first, so
+    all of them are walked, and runs agree bit for bit."""
+    rng = np.random.default_rng(n)
+    st = scenarios.empty_state(n)
+    for f in ("posX", "posY", "posZ"):
+        st[f][:] = rng.uniform(-1.0, 1.0, n)
+    st["mass"][:] = 1.0 / n
+    st["h"][:] = st["h0"][:] = 0.02
+    st["h"][::every] = st["h0"][::every] = 3.0
+    st["rho"][:] = rng.uniform(1.0e-3, 2.0e-3, n)
+    st["originalId"][:] = np.arange(n, dtype=np.uint32)
+    for f in ("velX", "velY", "velZ"):
+        st[f][:] = rng.normal(size=n)
+    heavy = len(range(0, n, every)) if n // every < 100 else n
+    outs = []
+    for _ in range(4):
+        p, alt, bvh = device_setup(st)
+        engine.sort_and_build_bvh(p, alt, bvh)
+        engine.reset_device_status()
+        engine.sph_pass1_neighbors(p, bvh)
+        flags, counters = engine.read_device_status()
+        assert flags == abi.DEVFLAG_NEIGHBOR_OVERFLOW
+        assert counters["fallback_walks"] == heavy
+        walks = counters["fallback_walks"]
+        g = p.download(["h", "shepardC", "surfFactor", "divV", "curlVX"])
+        outs.append((walks, g))
+    for walks, g in outs[1:]:
+        assert walks == outs[0][0]
+        for f in g:
+            assert np.array_equal(g[f], outs[0][1][f]), f
+    o = oracle.Oracle(st)
+    o.sort_and_build()
+    o.pass1()
+    c = o.state()
+    for f in ("h", "shepardC", "surfFactor", "divV"):
+        assert rel_rms(outs[0][1][f], c[f]) < 1e-5, f
