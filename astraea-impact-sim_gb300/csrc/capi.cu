@@ -416,13 +416,21 @@ AstraeaStatus ffCapacity(FfBuffers* b, const FfState* f, uint32_t groups) {
     return ASTRAEA_OK;
 }
 
+// What a mode-2 walk of n particles needs besides the tree: the network, if it is
+// to be applied, and buffers.  Asked for before a call touches the workspace's
+// records, so a call that is refused leaves them as they were.
+AstraeaStatus ffReady(Workspace* ws, uint32_t n, bool network, FfState** out) {
+    AstraeaStatus s = ffState(out);
+    if (s != ASTRAEA_OK) return s;
+    if (network && !(*out)->ready)
+        return fail(ASTRAEA_ERR_INVALID, "far-field mode 2 needs network parameters (ff_init / ff_set_params)");
+    return ffCapacity(&ws->ff, *out, (n + 31u) / 32u);
+}
+
 // The mode-2 walk: the theta walk plus the far test; records pairs into the
 // workspace's own buffers.
 AstraeaStatus ffWalk(AstraeaParticles* p, Workspace* ws, uint32_t n, float theta, FfState* f, uint32_t stride) {
-    const uint32_t groups = (n + 31u) / 32u;
     FfBuffers* b = &ws->ff;
-    AstraeaStatus s = ffCapacity(b, f, groups);
-    if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
     AG_CUDA(cudaMemsetAsync(b->word, 0, sizeof(uint32_t), st));
     FarCapture cap{b->pairs, b->pairCap, b->word, b->groups, f->cfg.thetaFar * f->cfg.thetaFar,
@@ -442,9 +450,8 @@ AstraeaStatus ffWalk(AstraeaParticles* p, Workspace* ws, uint32_t n, float theta
 AstraeaStatus learnedGravity(AstraeaParticles* p, Workspace* ws, uint32_t n, float theta, bool gate,
                              cudaEvent_t* ev = nullptr) {
     FfState* f = nullptr;
-    AstraeaStatus s = ffState(&f);
+    AstraeaStatus s = ffReady(ws, n, true, &f);
     if (s != ASTRAEA_OK) return s;
-    if (!f->ready) return fail(ASTRAEA_ERR_INVALID, "far-field mode 2 needs network parameters (ff_init / ff_set_params)");
     cudaStream_t st = stream();
     auto mark = [&](int k) { if (ev != nullptr) cudaEventRecord(ev[k], st); };
     mark(0);
@@ -489,6 +496,14 @@ cudaError_t modeGravity(const AstraeaParticles& p, const Work& w0, uint32_t n, f
         return launchGravity(p, w, n, theta, true, sms, st, nullptr, warps, true);
     }
     return launchGravity(p, w0, n, theta, moments && mode == 1, sms, st, nullptr, warps);
+}
+
+// Leaf records from the caller's state.  Clearing the words of the next neighbour
+// build (arm) ends the lists there are, and with them the fused step's.
+cudaError_t refreshLeaves(const AstraeaParticles& p, Workspace* ws, uint32_t n, bool withVelRho, cudaStream_t st,
+                          bool arm = true) {
+    if (arm) ws->stepCacheValid = false;
+    return launchRefreshLeaves(p, ws->w, n, withVelRho, st, arm);
 }
 
 // Launches of one walk on the workspace's side stream, beside what the caller
@@ -787,12 +802,10 @@ AstraeaStatus astraea_gb300_sort_and_build_bvh(AstraeaParticles* p, AstraeaParti
     AstraeaStatus s = workspaceFor(bvh, std::max(bvh->capacity, n), true, &ws);
     if (s != ASTRAEA_OK) return s;
     if (bvh->livingFlags == nullptr) bvh->livingFlags = ws->w.words + kWLiving;   // sph_gravity.cu:2008-2011
+    ws->stepCacheValid = false;
     AG_LAUNCH(launchInitBounds(ws->w.words, stream()));
     AG_LAUNCH(launchBounds(*p, n, ws->w.words, smCount(), stream()));
-    s = buildTree(p, alt, bvh, ws, nullptr, true);
-    if (s != ASTRAEA_OK) return s;
-    ws->stepCacheValid = false;
-    return ASTRAEA_OK;
+    return buildTree(p, alt, bvh, ws, nullptr, true);
 }
 
 AstraeaStatus astraea_gb300_sph_pass1_neighbors(AstraeaParticles* p, const AstraeaRadixBvh* bvh) {
@@ -803,7 +816,7 @@ AstraeaStatus astraea_gb300_sph_pass1_neighbors(AstraeaParticles* p, const Astra
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, true, st));
     AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchPass1(*p, ws->w, n, st));
     ws->stepCacheValid = false;
@@ -828,10 +841,15 @@ AstraeaStatus gravityBarnesHut(AstraeaParticles* p, const AstraeaRadixBvh* bvh, 
     Workspace* ws = nullptr;
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, stream(), !keepLists));
     const int mode = g_farField.load();
     if (mode != 0 && !ws->momentsBuilt)
         return fail(ASTRAEA_ERR_INVALID, "far-field modes 1, 2 and 3 need a tree built in that mode");
+    if (mode == 2) {
+        FfState* f = nullptr;
+        s = ffReady(ws, n, true, &f);
+        if (s != ASTRAEA_OK) return s;
+    }
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, stream(), !keepLists));
     if (mode == 2) {
         s = learnedGravity(p, ws, n, theta, true);
         if (s != ASTRAEA_OK) return s;
@@ -860,7 +878,7 @@ AstraeaStatus astraea_gb300_debug_gravity_group_trace(AstraeaParticles* p, const
     if (s != ASTRAEA_OK) return s;
     if (g_farField.load() != 0) return fail(ASTRAEA_ERR_INVALID, "the trace is taken in far-field mode 0");
     AG_CUDA(cudaMemsetAsync(trace, 0, sizeof(int32_t), stream()));
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, stream()));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, stream()));
     Work w = ws->w;
     w.traceList = trace;
     w.traceGroup = group;
@@ -880,7 +898,7 @@ AstraeaStatus astraea_gb300_debug_gravity_group_counts(AstraeaParticles* p, cons
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
     if (g_farField.load() != 0) return fail(ASTRAEA_ERR_INVALID, "group counts are taken in far-field mode 0");
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, stream()));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, stream()));
     Work w = ws->w;
     w.groupCounts = groupCounts;
     AG_LAUNCH(launchGravity(*p, w, n, theta, false, smCount(), stream(), nullptr,
@@ -905,7 +923,7 @@ AstraeaStatus pass2Forces(AstraeaParticles* p, const AstraeaRadixBvh* bvh, bool 
     s = deviceState(&ds);
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st, !lists));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, true, st, !lists));
     if (!lists) AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchPackPass2Records(*p, ws->w, n, st));
     const uint32_t* living = (bvh->livingFlags != nullptr) ? bvh->livingFlags : ds->zeroWords;   // :2104
@@ -928,7 +946,7 @@ AstraeaStatus leapfrogDrift(AstraeaParticles* p, float dtPsu, const AstraeaRadix
     Workspace* ws = nullptr;
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st, !lists));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, true, st, !lists));
     if (!lists) AG_LAUNCH(launchBuildNeighbors(ws->w, n, smCount(), st, static_cast<int>(tuningFor(n).neighborWarps), true));
     AG_LAUNCH(launchDrift(*p, ws->w, n, nullptr, dtPsu, true, false, nullptr, st));
     ws->stepCacheValid = false;
@@ -1092,7 +1110,7 @@ AstraeaStatus astraea_gb300_relax_single_body(AstraeaParticles* p, AstraeaPartic
         cudaStream_t st = stream();
         const int sms = smCount();
         const bool share = n <= kShareMax;
-        AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, true, st));
+        AG_LAUNCH(refreshLeaves(*p, ws, n, true, st));
         Beside walks(ws, st);
         AG_LAUNCH(walks.fork(share, [&](LaunchAt at) {
             return modeGravity(*p, ws->w, n, 0.5f, mode, true, sms, at,
@@ -1177,10 +1195,10 @@ AstraeaStatus astraea_gb300_ff_collect(AstraeaParticles* p, const AstraeaRadixBv
     if (s != ASTRAEA_OK) return s;
     if (!ws->momentsBuilt) return fail(ASTRAEA_ERR_INVALID, "ff_collect needs a tree built in far-field mode 2");
     FfState* f = nullptr;
-    s = ffState(&f);
+    s = ffReady(ws, n, false, &f);
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, st));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, st));
     s = ffWalk(p, ws, n, theta, f, groupStride);
     if (s != ASTRAEA_OK) return s;
     uint32_t recorded = 0;
@@ -1326,7 +1344,10 @@ AstraeaStatus astraea_gb300_ff_profile(AstraeaParticles* p, const AstraeaRadixBv
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
     if (!ws->momentsBuilt) return fail(ASTRAEA_ERR_INVALID, "far-field mode 2 needs a tree built in that mode");
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, stream()));
+    FfState* f = nullptr;
+    s = ffReady(ws, n, true, &f);
+    if (s != ASTRAEA_OK) return s;
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, stream()));
     cudaEvent_t ev[6] = {};
     for (auto& e : ev) AG_CUDA(cudaEventCreate(&e));
     s = learnedGravity(p, ws, n, theta, true, ev);
@@ -1380,7 +1401,7 @@ AstraeaStatus astraea_gb300_autotune(AstraeaParticles* p, const AstraeaRadixBvh*
     AstraeaStatus s = builtWorkspace(bvh, n, &ws);
     if (s != ASTRAEA_OK) return s;
     cudaStream_t st = stream();
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, st));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, st));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     AG_CUDA(cudaEventCreate(&e0));
     AG_CUDA(cudaEventCreate(&e1));
@@ -1455,7 +1476,7 @@ AstraeaStatus astraea_gb300_autotune_expansion(AstraeaParticles* p, const Astrae
     for (uint32_t k = 0; k < count; ++k)
         if (candidates[k] > 32u) return fail(ASTRAEA_ERR_INVALID, "leaf bucket must be at most 32 particles");
     cudaStream_t st = stream();
-    AG_LAUNCH(launchRefreshLeaves(*p, ws->w, n, false, st));
+    AG_LAUNCH(refreshLeaves(*p, ws, n, false, st));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     AG_CUDA(cudaEventCreate(&e0));
     AG_CUDA(cudaEventCreate(&e1));
@@ -1614,7 +1635,7 @@ AstraeaStatus astraea_gb300_step(AstraeaParticles* p, AstraeaParticles* alt, Ast
         // Device dt state from the caller's previous dt and the current state.
         AG_LAUNCH(launchSetDtSlots(ws->dtSlots, q, prevDtPsu, ws->rawMin, st));
         AG_LAUNCH(launchReduceDt(*p, n, ws->rawMin + q, sms, st));
-        AG_LAUNCH(launchRefreshLeaves(*p, w, n, false, st));
+        AG_LAUNCH(refreshLeaves(*p, ws, n, false, st));
         if (useBvh) AG_LAUNCH(launchBuildNeighbors(w, n, sms, st, static_cast<int>(tune.neighborWarps), true));
     }
     // 1. opening half kick; dt resolved on the device
