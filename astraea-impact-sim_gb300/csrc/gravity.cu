@@ -372,16 +372,13 @@ __global__ void __launch_bounds__(256) pairNodesKernel(Work w, uint32_t n) {
     o[3] = make_float4(farC[0], farC[1], __uint_as_float(cnt[0]), __uint_as_float(cnt[1]));
 }
 
-// kDebug: the variant that serves the debugging calls (per-group interaction
-// counts, the trace of one group's accepted nodes and leaves); their checks
-// are kept out of the production variants, where they cost 2 % of the walk.
 // kWarpsPerSm: the resident warps the registers are bounded for (72, 80 and 96
 // registers).  At 1M: quadrupole, theta 0.7, 24 warps 1.36 ms, 20 1.44 (4M Plummer
 // sphere 7.94, 28 with spills 8.08); expansion, theta 0.7, 20 warps 1.55, 16 1.64, 24
 // (spills) 1.62; learned, the walk alone, 28 warps 1.37, 24 1.42, 20 1.42, 32 1.46.
 template <bool kQuad, bool kExpand>
 constexpr int kWarpsPerSm = kExpand ? 20 : (kQuad ? 24 : 28);
-template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = false, bool kDebug = false>
+template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = false>
 __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWarps) gravityKernel(AstraeaParticles p, Work w, uint32_t n,
                                                                  float theta2, uint32_t numGroups,
                                                                  uint32_t* groupCounter, FarCapture ff) {
@@ -402,8 +399,6 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
         }
         return;
     }
-    const float invTheta = 1.0f / sqrtf(theta2);     // theta = 0: infinite, nothing is accepted early
-
     for (;;) {
         uint32_t g = 0;
         if (lane == 0) g = atomicAdd(groupCounter, 1u);
@@ -630,12 +625,6 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             sp += __popc(mA);
             if (kTwo && openB) S.stack[sp + __popc(mB & laneMaskLt())] = B.ref;
             sp += __popc(mB);
-            if (kDebug && w.traceList != nullptr && g == w.traceGroup && (accA || accB)) {
-                const uint32_t k = atomicAdd(reinterpret_cast<uint32_t*>(w.traceList), (accA ? 1u : 0u) + (accB ? 1u : 0u));
-                if (accA && k < w.traceCap) w.traceList[1 + k] = A.ref;
-                const uint32_t k2 = k + (accA ? 1u : 0u);
-                if (accB && k2 < w.traceCap) w.traceList[1 + k2] = B.ref;
-            }
             putAccepted(accA, A);
             if (kTwo) putAccepted(accB, B);
             __syncwarp();
@@ -843,10 +832,6 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                     putParticle(S.plist, slot, c.x, c.y, c.z, c.gm, c.w);
                     const uint32_t rel = static_cast<uint32_t>(~c.ref) - base;
                     if (rel < 32u) selfBit |= 1u << rel;
-                    if (kDebug && w.traceList != nullptr && g == w.traceGroup) {
-                        const uint32_t k = atomicAdd(reinterpret_cast<uint32_t*>(w.traceList), 1u);
-                        if (k < w.traceCap) w.traceList[1 + k] = c.ref;
-                    }
                 };
                 if (leafA) putLeaf(A, (pHead + pCount + __popc(lA & laneMaskLt())) & (kGravList - 1));
                 if (leafB) putLeaf(B, (pHead + pCount + __popc(lA) + __popc(lB & laneMaskLt())) & (kGravList - 1));
@@ -915,7 +900,6 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                 S.counts[4] += groupEvals;
                 S.counts[5] += bucketLeaves;
             }
-            if (kDebug && w.groupCounts != nullptr) w.groupCounts[g] = static_cast<uint32_t>(inter);
         }
         __syncwarp();
     }
@@ -960,7 +944,10 @@ struct __align__(16) OrderedSmem {
 };
 static_assert(offsetof(OrderedSmem, mlist) % 16 == 0 && offsetof(OrderedSmem, plist) % 16 == 0 &&
               offsetof(OrderedSmem, und) % 16 == 0 && offsetof(OrderedSmem, dirPos) % 16 == 0, "vector loads");
-template <int kWarps, bool kInside>
+// kDebug: the variant that serves the debugging calls (per-group interaction
+// counts, the trace of one group's accepted nodes and leaves in walk order); their
+// checks are kept out of the production variants.
+template <int kWarps, bool kInside, bool kDebug = false>
 __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gravityOrderedKernel(AstraeaParticles p, Work w, uint32_t n,
                                                                                 float theta2, uint32_t numGroups,
                                                                                 uint32_t* groupCounter, FarCapture) {
@@ -1009,7 +996,8 @@ __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gra
         extremeMembers(S.dirPos, xi, yi, zi, cx, cy, cz, slack, act, lane);
         if (lane == 0) S.stack[0] = 0;   // the root is opened by every group
         int sp = 1, mCount = 0, pCount = 0, mHead = 0, pHead = 0;
-        uint32_t rounds = 0;
+        uint32_t rounds = 0, traced = 0;
+        [[maybe_unused]] const unsigned long long interBefore = nInter;
         const f2 X = pack2(xi, xi), Y = pack2(yi, yi), Z = pack2(zi, zi);
         const f2 E2 = pack2(epsI2, epsI2), HE = pack2(0.5f * epsI, 0.5f * epsI);
         Accum2 acc{0ull, 0ull, 0ull, 0ull};
@@ -1104,6 +1092,13 @@ __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gra
             if (open) S.stack[sp + __popc(openMask & laneMaskLt())] = ref;
             sp += __popc(openMask);
             const unsigned accMask = __ballot_sync(0xffffffffu, accept), leafMask = __ballot_sync(0xffffffffu, isLeaf);
+            if (kDebug && w.traceList != nullptr && g == w.traceGroup) {
+                const unsigned both = accMask | leafMask;
+                const uint32_t k = traced + static_cast<uint32_t>(__popc(both & laneMaskLt()));
+                if ((accept || isLeaf) && k < w.traceCap) w.traceList[1 + k] = ref;
+                traced += static_cast<uint32_t>(__popc(both));
+                if (lane == 0) w.traceList[0] = static_cast<int>(traced);
+            }
             if (accept) {
                 const float e[10] = {x, y, z, gm, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 putMono<false, kOrdRing>(S.mlist, (mHead + mCount + __popc(accMask & laneMaskLt())) & (kOrdRing - 1), e);
@@ -1163,6 +1158,7 @@ __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gra
         }
         nInter += static_cast<unsigned long long>(act) * static_cast<unsigned>(mCount + pCount) -
                   static_cast<unsigned long long>(__popc(selfSeen));
+        if (kDebug && w.groupCounts != nullptr && lane == 0) w.groupCounts[g] = static_cast<uint32_t>(nInter - interBefore);
         nRounds += rounds;
         __syncwarp();
     }
@@ -1198,8 +1194,7 @@ cudaError_t launchGravity(const AstraeaParticles& p, const Work& w, uint32_t n, 
     int wps = kGravWarps;
     if (w.traceList != nullptr || w.groupCounts != nullptr) {
         // the debugging calls (monopole walk, 4-warp blocks)
-        kernel = checkInside ? gravityKernel<kGravWarps, true, false, false, false, true>
-                             : gravityKernel<kGravWarps, false, false, false, false, true>;
+        kernel = checkInside ? gravityOrderedKernel<kGravWarps, true, true> : gravityOrderedKernel<kGravWarps, false, true>;
     } else if (expansion && quadrupole && far == nullptr) {
         if (warps == 2) {
             kernel = checkInside ? gravityKernel<2, true, true, false, true> : gravityKernel<2, false, true, false, true>;
