@@ -654,9 +654,9 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                 return bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy || bmax.z < gminz ||
                        bmin.z > gmaxz;
             };
-            // the box is only looked at where a member may be as near the
-            // COM as its furthest corner
-            if (kInside && isNode && (boundAccepts || extreme) && !(Lb2 > far2)) {
+            // the box is only looked at where the members in question may be as
+            // near the COM as its furthest corner
+            if (kInside && isNode && ((boundAccepts && !(Lb2 > far2)) || (extreme && !(r2 > far2)))) {
                 const float4 bmin = __ldg(&w.node[4 * static_cast<size_t>(ref) + 2]);
                 const float4 bmax = __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]);
                 boundAccepts = boundAccepts && apart(bmin, bmax);
@@ -932,7 +932,10 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
 // nodes before it (one node a lane, leaves loaded again): 1M 1.69 -> 1.37 ms, 60k
 // 139 -> 120 us.  Resident warps per SM the registers are bounded for, 1M: theta 0.5
 // 28 1.54, 32 1.50, 36 1.40, 40 (spills) 1.42 ms; theta 0.7, whose box test needs more
-// registers, 24 1.07, 28 0.99, 32 1.01, 36 (spills) 1.04.
+// registers, 24 1.07, 28 0.99, 32 1.01, 36 (spills) 1.04.  Those boxes are loaded only where
+// a member may be as near as the furthest corner: loaded for every undecided child, a
+// dependent trip each, a call at theta 0.6 took 97 instead of 77 us at 16k, 136
+// instead of 110 at 60k, 1146 instead of 977 at 1M.
 constexpr int kOrdRing = 64;
 struct __align__(16) OrderedSmem {
     int stack[kGravStack];
@@ -940,6 +943,7 @@ struct __align__(16) OrderedSmem {
     float plist[5 * kOrdRing];
     float4 und[32];                    // undecided children: COM, dNode^2
     int undRef[32];
+    float undFar[32];
     float4 dirPos[8];                  // see GravWarpSmem
 };
 static_assert(offsetof(OrderedSmem, mlist) % 16 == 0 && offsetof(OrderedSmem, plist) % 16 == 0 &&
@@ -1036,9 +1040,9 @@ __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gra
             const float r2 = len2Engine(__fsub_rn(dp.x, x), __fsub_rn(dp.y, y), __fsub_rn(dp.z, z));
             bool boundAccepts = Lb2 > 2.0e-20f && dd < theta2 * Lb2;
             bool extreme = dd < __fmul_rn(theta2, r2) && r2 > 1.0e-20f;
+            const float far2 = kInside ? __ldg(reinterpret_cast<const float*>(rec + 3) + (lane & 1)) : 0.0f;
             if (kInside) {
-                const float far2 = __ldg(reinterpret_cast<const float*>(rec + 3) + (lane & 1));
-                if (isNode && (boundAccepts || extreme) && !(Lb2 > far2)) {
+                if (isNode && ((boundAccepts && !(Lb2 > far2)) || (extreme && !(r2 > far2)))) {
                     const float4 bmin = __ldg(&w.node[4 * static_cast<size_t>(ref) + 2]);
                     const float4 bmax = __ldg(&w.node[4 * static_cast<size_t>(ref) + 3]);
                     boundAccepts = boundAccepts && (bmax.x < gminx || bmin.x > gmaxx || bmax.y < gminy || bmin.y > gmaxy ||
@@ -1056,20 +1060,25 @@ __global__ void __launch_bounds__(kWarps * 32, (kInside ? 28 : 36) / kWarps) gra
                 nUndecided += static_cast<uint32_t>(nu);
                 if (undecided) {
                     S.und[slot] = make_float4(x, y, z, dd);
-                    if (kInside) S.undRef[slot] = ref;
+                    if (kInside) {
+                        S.undRef[slot] = ref;
+                        S.undFar[slot] = far2;
+                    }
                 }
                 __syncwarp();
                 unsigned bits = 0u;
                 auto settle = [&](int k) {
                     const float4 q = S.und[k];
                     const float m2 = len2Engine(__fsub_rn(xi, q.x), __fsub_rn(yi, q.y), __fsub_rn(zi, q.z));
-                    bool ok = q.w < __fmul_rn(theta2, m2) && m2 > 1.0e-20f;
-                    if (kInside) {
+                    const bool ok = q.w < __fmul_rn(theta2, m2) && m2 > 1.0e-20f;
+                    bool all = __all_sync(0xffffffffu, !active || ok);
+                    if (kInside && all && __any_sync(0xffffffffu, active && !(m2 > S.undFar[k]))) {
                         const float4 mn = __ldg(&w.node[4 * static_cast<size_t>(S.undRef[k]) + 2]);
                         const float4 mx = __ldg(&w.node[4 * static_cast<size_t>(S.undRef[k]) + 3]);
-                        if (xi >= mn.x && xi <= mx.x && yi >= mn.y && yi <= mx.y && zi >= mn.z && zi <= mx.z) ok = false;
+                        all = __all_sync(0xffffffffu, !active || !(xi >= mn.x && xi <= mx.x && yi >= mn.y && yi <= mx.y &&
+                                                                   zi >= mn.z && zi <= mx.z));
                     }
-                    bits |= (__all_sync(0xffffffffu, !active || ok) ? 1u : 0u) << k;
+                    bits |= (all ? 1u : 0u) << k;
                 };
                 if constexpr (kInside) {
 #pragma unroll 2
