@@ -49,9 +49,10 @@ namespace {
 constexpr int kGravWarps = 4;
 // Opened nodes per warp.  Peak use of gravityOrderedKernel / gravityKernel: 1M impact,
 // theta 0.5, 133 / 156; 4M Plummer sphere, theta 0.5, 208 / 282, theta 0.1, full / 359.
-// gravityKernel takes smaller rounds as it fills (walkWidth): without that it ran out at theta 0.2 on the Plummer spheres of 1M and
-// 4M (forces wrong by 2e-2); with it 30.3 -> 31.8 and 150 -> 163 ms there, 698 -> 836 at
-// theta 0.1 (4M), and no difference from theta 0.5 up.
+// gravityKernel takes smaller rounds as it fills (walkWidth).  Without that it ran
+// out at small angles, so opened nodes became monopoles: rms force error 0.62 at
+// theta 0.2 on the 4M sphere, 0.023 at theta 0.1 on one of 1M (now 1.5e-5, 5.9e-6).
+// It costs 30.3 -> 31.8 ms (1M) and 150 -> 163 (4M) at theta 0.2, nothing from 0.5 up.
 constexpr int kGravStack = 448;
 // Ring lists: a round appends up to 64 entries behind at most 31 pending ones.
 // The quadrupole's monopole entries are 40 bytes: its list (and mode 3's far
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(256) pairNodesKernel(Work w, uint32_t n) {
 
 // kWarpsPerSm: the resident warps the registers are bounded for (72, 80 and 96
 // registers).  At 1M: quadrupole, theta 0.7, 24 warps 1.36 ms, 20 1.44 (4M Plummer
-// sphere 7.94, 28 with spills 8.08); expansion, theta 0.7, 20 warps 1.55, 16 1.64, 24
-// (spills) 1.62; learned, the walk alone, 28 warps 1.37, 24 1.42, 20 1.42, 32 1.46.
+// sphere 7.94, 28 with spills 8.08); expansion, theta 0.7, 20 warps 1.32, 16 1.46, 24
+// (spills) 1.37; learned, the walk alone, 28 warps 1.37, 24 1.42, 20 1.42, 32 1.46.
 template <bool kQuad, bool kExpand>
 constexpr int kWarpsPerSm = kExpand ? 20 : (kQuad ? 24 : 28);
 template <int kWarps, bool kInside, bool kQuad, bool kLearned, bool kExpand = false>
@@ -607,6 +608,11 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
         };
         // Puts the decided nodes among up to two children a lane (kTwo) where
         // they belong: opened ones on the stack, accepted ones into the lists.
+        // The group expansion calls it from one place, and its evaluations stand in
+        // loops over the two sides, to keep the code small: with four copies of
+        // them that walk waited 4 of its 10.8 cycles an instruction for
+        // instructions (1M, theta 0.75, buckets of 8, 1.49 ms; now 1.16).  The other
+        // modes' evaluations are short enough: there one copy costs 3 %.
         auto place = [&](auto two, bool openA, bool accA, const Child& A, bool openB, bool accB, const Child& B) {
             constexpr bool kTwo = decltype(two)::value;
             const uint2 brA = bucketOf(openA, A), brB = kTwo ? bucketOf(openB, B) : make_uint2(1u, 0u);
@@ -625,14 +631,21 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             sp += __popc(mA);
             if (kTwo && openB) S.stack[sp + __popc(mB & laneMaskLt())] = B.ref;
             sp += __popc(mB);
-            putAccepted(accA, A);
-            if (kTwo) putAccepted(accB, B);
-            __syncwarp();
-            if (!kQuad)
-                while (mCount >= 32) flushM();
-            if (kExpand) {
-                putBuckets(brA);
-                if (kTwo) putBuckets(brB);
+            if constexpr (kExpand) {
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side) {
+                    const bool acc = side != 0 ? accB : accA;
+                    if (__any_sync(0xffffffffu, acc)) putAccepted(acc, side != 0 ? B : A);
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side) putBuckets(side != 0 ? brB : brA);
+            } else {
+                putAccepted(accA, A);
+                if (kTwo) putAccepted(accB, B);
+                __syncwarp();
+                if (!kQuad)
+                    while (mCount >= 32) flushM();
             }
         };
         // The cheap tests of one child (u = COM - c): accepted by the bound,
@@ -724,6 +737,8 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
             }
             // every undecided child may still be opened
             const int width = walkWidth<kGravStack>(sp + uCount);
+            Child A, B;
+            bool accA = false, openA = false, accB = false, openB = false;
             if (uCount >= 32 || sp == 0 || (width == 1 && uCount > 0)) {
                 // The oldest undecided children, up to 32, one a lane, against every
                 // member: the engine's member test (sph_gravity.cu:914-929) with
@@ -779,68 +794,73 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                         }
                     }
                 }
-                place(std::false_type{}, has && !all, has && all, c, false, false, c);
-                continue;
-            }
-            // open up to 32 nodes: both children of each
-            spPeak = max(spPeak, sp);
-            const int take = min(sp, width);
-            sp -= take;
-            int node = (lane < take) ? S.stack[sp + lane] : 0;
-            __syncwarp();
-            // indices outside [0, n-2] cannot come from a valid tree
-            const bool has = lane < take && static_cast<uint32_t>(node) < n - 1u;
-            node = has ? node : 0;
-            const PairRec rec = loadPair<kInside || kExpand>(w.pair + 4 * static_cast<size_t>(node));
-            const f2 du = sub2(rec.x, CX), dv = sub2(rec.y, CY), dw = sub2(rec.z, CZ), dd = mul2(rec.w, rec.w);
-            tests += 2u * static_cast<uint32_t>(take);
-            Child A, B;
-            unpack2(rec.x, A.x, B.x);
-            unpack2(rec.y, A.y, B.y);
-            unpack2(rec.z, A.z, B.z);
-            unpack2(rec.gm, A.gm, B.gm);
-            unpack2(rec.w, A.w, B.w);
-            A.ref = rec.refA;
-            B.ref = rec.refB;
-            A.cnt = rec.cntA;
-            B.cnt = rec.cntB;
-            A.right = false;
-            B.right = true;
-            float uxA, uxB, uyA, uyB, uzA, uzB, ddA, ddB;
-            unpack2(du, uxA, uxB);
-            unpack2(dv, uyA, uyB);
-            unpack2(dw, uzA, uzB);
-            unpack2(dd, ddA, ddB);
-            bool accA, openA, undA, accB, openB, undB;
-            decide(has && A.ref >= 0, A.x, A.y, A.z, ddA, uxA, uyA, uzA, A.ref, rec.farA, accA, openA, undA);
-            decide(has && B.ref >= 0, B.x, B.y, B.z, ddB, uxB, uyB, uzB, B.ref, rec.farB, accB, openB, undB);
-            // undecided children of both sides
-            const unsigned uA = __ballot_sync(0xffffffffu, undA), uB = __ballot_sync(0xffffffffu, undB);
-            if (uA | uB) {
-                const int s0 = uHead + uCount + __popc(uA & laneMaskLt());
-                if (undA) S.und[s0 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node);
-                const int s1 = uHead + uCount + __popc(uA) + __popc(uB & laneMaskLt());
-                if (undB) S.und[s1 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node) + 1u;
-                uCount += __popc(uA) + __popc(uB);
-            }
-            // leaves of both sides
-            const bool leafA = has && A.ref < 0, leafB = has && B.ref < 0;
-            const unsigned lA = __ballot_sync(0xffffffffu, leafA), lB = __ballot_sync(0xffffffffu, leafB);
-            if (lA | lB) {
-                unsigned selfBit = 0u;
-                auto putLeaf = [&](const Child& c, int slot) {
-                    putParticle(S.plist, slot, c.x, c.y, c.z, c.gm, c.w);
-                    const uint32_t rel = static_cast<uint32_t>(~c.ref) - base;
-                    if (rel < 32u) selfBit |= 1u << rel;
-                };
-                if (leafA) putLeaf(A, (pHead + pCount + __popc(lA & laneMaskLt())) & (kGravList - 1));
-                if (leafB) putLeaf(B, (pHead + pCount + __popc(lA) + __popc(lB & laneMaskLt())) & (kGravList - 1));
-                selfSeen |= __reduce_or_sync(0xffffffffu, selfBit);
-                const int cnt = __popc(lA) + __popc(lB);
-                pCount += cnt;
-                tests -= static_cast<uint32_t>(cnt);
+                if constexpr (!kExpand) {
+                    place(std::false_type{}, has && !all, has && all, c, false, false, c);
+                    continue;
+                }
+                A = B = c;
+                openA = has && !all;
+                accA = has && all;
+            } else {
+                // open up to 32 nodes: both children of each
+                spPeak = max(spPeak, sp);
+                const int take = min(sp, width);
+                sp -= take;
+                int node = (lane < take) ? S.stack[sp + lane] : 0;
                 __syncwarp();
-                while (pCount >= 32) flushP();
+                // indices outside [0, n-2] cannot come from a valid tree
+                const bool has = lane < take && static_cast<uint32_t>(node) < n - 1u;
+                node = has ? node : 0;
+                const PairRec rec = loadPair<kInside || kExpand>(w.pair + 4 * static_cast<size_t>(node));
+                const f2 du = sub2(rec.x, CX), dv = sub2(rec.y, CY), dw = sub2(rec.z, CZ), dd = mul2(rec.w, rec.w);
+                tests += 2u * static_cast<uint32_t>(take);
+                unpack2(rec.x, A.x, B.x);
+                unpack2(rec.y, A.y, B.y);
+                unpack2(rec.z, A.z, B.z);
+                unpack2(rec.gm, A.gm, B.gm);
+                unpack2(rec.w, A.w, B.w);
+                A.ref = rec.refA;
+                B.ref = rec.refB;
+                A.cnt = rec.cntA;
+                B.cnt = rec.cntB;
+                A.right = false;
+                B.right = true;
+                float uxA, uxB, uyA, uyB, uzA, uzB, ddA, ddB;
+                unpack2(du, uxA, uxB);
+                unpack2(dv, uyA, uyB);
+                unpack2(dw, uzA, uzB);
+                unpack2(dd, ddA, ddB);
+                bool undA, undB;
+                decide(has && A.ref >= 0, A.x, A.y, A.z, ddA, uxA, uyA, uzA, A.ref, rec.farA, accA, openA, undA);
+                decide(has && B.ref >= 0, B.x, B.y, B.z, ddB, uxB, uyB, uzB, B.ref, rec.farB, accB, openB, undB);
+                // undecided children of both sides
+                const unsigned uA = __ballot_sync(0xffffffffu, undA), uB = __ballot_sync(0xffffffffu, undB);
+                if (uA | uB) {
+                    const int s0 = uHead + uCount + __popc(uA & laneMaskLt());
+                    if (undA) S.und[s0 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node);
+                    const int s1 = uHead + uCount + __popc(uA) + __popc(uB & laneMaskLt());
+                    if (undB) S.und[s1 & (kGravList - 1)] = 2u * static_cast<uint32_t>(node) + 1u;
+                    uCount += __popc(uA) + __popc(uB);
+                }
+                // leaves of both sides
+                const bool leafA = has && A.ref < 0, leafB = has && B.ref < 0;
+                const unsigned lA = __ballot_sync(0xffffffffu, leafA), lB = __ballot_sync(0xffffffffu, leafB);
+                if (lA | lB) {
+                    unsigned selfBit = 0u;
+                    auto putLeaf = [&](const Child& c, int slot) {
+                        putParticle(S.plist, slot, c.x, c.y, c.z, c.gm, c.w);
+                        const uint32_t rel = static_cast<uint32_t>(~c.ref) - base;
+                        if (rel < 32u) selfBit |= 1u << rel;
+                    };
+                    if (leafA) putLeaf(A, (pHead + pCount + __popc(lA & laneMaskLt())) & (kGravList - 1));
+                    if (leafB) putLeaf(B, (pHead + pCount + __popc(lA) + __popc(lB & laneMaskLt())) & (kGravList - 1));
+                    selfSeen |= __reduce_or_sync(0xffffffffu, selfBit);
+                    const int cnt = __popc(lA) + __popc(lB);
+                    pCount += cnt;
+                    tests -= static_cast<uint32_t>(cnt);
+                    __syncwarp();
+                    while (pCount >= 32) flushP();
+                }
             }
             place(std::true_type{}, openA, accA, A, openB, accB, B);
         }
