@@ -24,6 +24,7 @@ import json
 import os
 import sys
 import time
+import unittest
 
 import numpy as np
 
@@ -44,6 +45,8 @@ KERNELS = {
 
 class RefKernels:
     def __init__(self, path=CUBIN):
+        if not os.path.exists(path):                # nothing to compare with: a test that gets here is skipped
+            raise unittest.SkipTest("the reference kernels' cubin (built from the reference checkout) is absent")
         import torch
         torch.cuda.init()
         torch.zeros(1, device="cuda")          # primary context current on this thread
