@@ -178,17 +178,20 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     auto take = [&](size_t bytes) { const size_t o = off; off += alignUp(bytes); return o; };
     const size_t oLeaf = take(C * 32), oAux = take(C * 16), oRec = take(C * 16 * kRec2Width);
     const size_t nbMax = refitBlocks(static_cast<uint32_t>(C)), levMax = refitLevels(static_cast<uint32_t>(nbMax));
-    const size_t oNode = take(C * 64), oPair = take(C * 64), oRange = take(C * 8), oLScan = take(C * 64), oMScan = take(C * 80);
+    const size_t oNode = take(C * 64), oPair = take(C * 64), oRange = take(C * 8);
     const size_t oTable = take(levMax * nbMax * 32), oBMom = take(nbMax * 80), oQuad = take(C * 32);
     const size_t oDrift = take(C * 16);
     const size_t oDRec = take(C * 32), oDAux = take(C * 8);
     const size_t oCnt = take(C * 4), oList = take((C + 31) / 32 * 32 * maxNbr * 4);
-    // Lists above maxNbr entries, all of them or none (sph.cu, heavyCount): one
-    // particle in sixteen with 384 entries each.  Pass 1 and 2 with 1 % / 3 % of
-    // a million particles at 2.5 / 2 times their h: 7.3 / 10.8 ms, walked 18.2 / 19.4,
-    // and 15.7 / 18.3 where a pool of a sixth of this served those that came first.
-    const size_t heavyCap = C / 16 + 256, poolCap = std::min<size_t>(C * 24 + 65536, 0xfffffff0u);
-    const size_t oHeavy = take(heavyCap * 16), oPool = take(poolCap * 4), oWords = take(kWCount * 4);
+    // Lists above maxNbr entries, all of them or none (sph.cu, heavyCount).  Their
+    // pool is where the refit's scans were: a list is built after the refit and last
+    // read by the drift, before the next one.  That is 36 words a particle (one in
+    // sixteen with 576 entries).  Pass 1 and 2 with 1 % / 3 % of a million particles
+    // at 2.5 / 2 times their h: 7.3 / 10.8 ms, walked 18.2 / 19.4, and 15.7 / 18.3 where
+    // a pool of 4 words a particle served those that came first.
+    const size_t heavyCap = C / 16 + 256, poolCap = std::min<size_t>(std::max<size_t>(C * 36, C * 4 + 65536), 0xfffffff0u);
+    const size_t scanBytes = alignUp(C * 64) + alignUp(C * 80);
+    const size_t oScan = take(std::max(scanBytes, poolCap * 4)), oHeavy = take(heavyCap * 16), oWords = take(kWCount * 4);
     const size_t oSort = take(sortWords * 4), oDt = take(64);
     void* block = nullptr;
     AG_CUDA(cudaMalloc(&block, off));
@@ -206,8 +209,8 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     w.node = reinterpret_cast<float4*>(b + oNode);
     w.pair = reinterpret_cast<float4*>(b + oPair);
     w.nodeRange = reinterpret_cast<uint2*>(b + oRange);
-    w.leafScan = reinterpret_cast<float4*>(b + oLScan);
-    w.momScan = reinterpret_cast<long long*>(b + oMScan);
+    w.leafScan = reinterpret_cast<float4*>(b + oScan);
+    w.momScan = reinterpret_cast<long long*>(b + oScan + alignUp(C * 64));
     w.blockTable = reinterpret_cast<float4*>(b + oTable);
     w.blockMom = reinterpret_cast<long long*>(b + oBMom);
     w.nodeQuad = reinterpret_cast<float4*>(b + oQuad);
@@ -218,7 +221,7 @@ AstraeaStatus allocWorkspace(Workspace* ws, uint32_t capacity) {
     w.nbrList = reinterpret_cast<uint32_t*>(b + oList);
     w.heavy = reinterpret_cast<uint4*>(b + oHeavy);
     w.heavyCap = static_cast<uint32_t>(heavyCap);
-    w.pool = reinterpret_cast<uint32_t*>(b + oPool);
+    w.pool = reinterpret_cast<uint32_t*>(b + oScan);
     w.poolCap = static_cast<uint32_t>(poolCap);
     w.words = reinterpret_cast<uint32_t*>(b + oWords);
     w.sortScratch = reinterpret_cast<uint32_t*>(b + oSort);

@@ -551,7 +551,7 @@ struct Work {
     uint32_t* nbrList;     // group-interleaved: entry k of particle i at ((i/32) maxNbr + k) 32 + i%32
     uint4* heavy;          // lists in the pool: {particle, first word, entries (0: not finished), 0}
     uint32_t heavyCap;
-    uint32_t* pool;
+    uint32_t* pool;        // shares its memory with leafScan and momScan, which only the refit uses
     uint32_t poolCap;      // words
     uint32_t* words;       // small words, see WordIndex
     uint32_t* sortScratch; // histograms + look-back + tile counters

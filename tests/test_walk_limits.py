@@ -153,7 +153,7 @@ def test_long_lists_of_deep_trees_are_whole(bits, levels, leg):
 @pytest.mark.parametrize("n,every", [(2000, 33), (4000, 10)])
 def test_lists_that_do_not_fit_the_pool(n, every):
     """More long lists than the pool has words for (61 of 1,999 entries; it has
-    113,536) or places (all 4,000 particles, each within reach of 400 long ones; it
+    73,536) or places (all 4,000 particles, each within reach of 400 long ones; it
     has 506): no particle's sums may then depend on which of them came first, so
     all of them are walked, and runs agree bit for bit."""
     rng = np.random.default_rng(n)
