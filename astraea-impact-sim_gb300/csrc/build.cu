@@ -709,9 +709,9 @@ cudaError_t launchPermuteLeavesKarras(const AstraeaParticles& p, const AstraeaPa
                                       const AstraeaRadixBvh& bvh, const float4* posSrc, const Work& w, uint32_t n,
                                       uint32_t* livingFlags, bool allFields, cudaStream_t st) {
     // The moves and the searches for the nodes are two chains of dependent loads;
-    // while the blocks of both fit at once (8 x 152 of 128 threads) each runs in
+    // while the blocks of both fit at once (8 an SM of 128 threads) each runs in
     // its own: permutation at 16k 18.7 -> 16.5 us, at 70k 20.5 -> 18.0.
-    constexpr uint32_t kSplitMax = 4u * 152u * 128u;
+    constexpr uint32_t kSplitMax = 4u * kTunedSms * 128u;
     const uint32_t block = n <= kSplitMax ? 128u : 256u, blocks = gridFor(n, static_cast<int>(block));
     const bool split = n <= kSplitMax;
     const auto kernel = allFields ? permuteLeavesKarrasKernel<true> : permuteLeavesKarrasKernel<false>;

@@ -85,7 +85,7 @@ struct __align__(16) GravWarpSmem {
     float4 memXY[16];
     float2 memZ[16];
     float4 dirPos[8];
-    float4 farDir[kLearned ? 27 : 1];   // mode 2's far test: the extreme members of 26 directions
+    float farDir[kLearned ? 28 : 4];    // mode 2's far test: the group's extent in 26 directions
     // far-field mode 3 only; last, and whole float4s, so the arrays above
     // keep the 16-byte alignment of their vector loads in every variant
     float4 flist4[kExpand ? 10 * kGravListQ / 4 : 1];    // far nodes of the group expansion (mlist layout)
@@ -96,7 +96,7 @@ template <bool kQuad, bool kExpand, bool kLearned>
 constexpr bool gravSmemAligned() {
     using S = GravWarpSmem<kQuad, kExpand, kLearned>;
     return offsetof(S, mlist) % 16 == 0 && offsetof(S, plist) % 16 == 0 && offsetof(S, memXY) % 16 == 0 && offsetof(S, memZ) % 8 == 0 &&
-           offsetof(S, dirPos) % 16 == 0 && offsetof(S, farDir) % 16 == 0 &&
+           offsetof(S, dirPos) % 16 == 0 &&
            offsetof(S, flist4) % 16 == 0 && offsetof(S, facc4) % 16 == 0 && sizeof(S) % 16 == 0;
 }
 static_assert(gravSmemAligned<false, false, false>() && gravSmemAligned<true, false, false>() &&
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                             pz = __shfl_sync(0xffffffffu, zi, m);
                 best = fmaxf(best, (sx * (px - cx) + sy * (py - cy) + sz * (pz - cz)) * inv);
             }
-            if (lane < 27) S.farDir[lane] = make_float4(0.0f, 0.0f, 0.0f, best);
+            if (lane < 27) S.farDir[lane] = best;
         }
         if (lane == 0) S.stack[0] = 0;   // the root is opened by every group
         int sp = 1, mCount = 0, pCount = 0, uCount = 0, fCount = 0;
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(kWarps * 32, kWarpsPerSm<kQuad, kExpand> / kWa
                 const int sx = (ux >= t) - (ux <= -t), sy = (uy >= t) - (uy <= -t), sz = (uz >= t) - (uz <= -t);
                 const float Lf = (static_cast<float>(sx) * ux + static_cast<float>(sy) * uy + static_cast<float>(sz) * uz) *
                                      invDirNorm(abs(sx) + abs(sy) + abs(sz)) -
-                                 S.farDir[13 + 9 * sx + 3 * sy + sz].w - 1.0e-6f * (ax + ay + az + gExt);
+                                 S.farDir[13 + 9 * sx + 3 * sy + sz] - 1.0e-6f * (ax + ay + az + gExt);
                 const float Fb2 = fmaxf(gx * gx + gy * gy + gz * gz, Lf > 0.0f ? Lf * Lf : 0.0f);
                 bool farOk = !accept && isNode && emitFar && Fb2 > 2.0e-20f && dd < ff.thetaFar2 * Fb2 * 0.99999f &&
                              gExt * gExt <= ff.gamma2 * (ux * ux + uy * uy + uz * uz);

@@ -54,6 +54,11 @@ cudaError_t launchChained(void (*kernel)(P...), uint32_t grid, uint32_t block, L
     return launchChainedSmem(kernel, grid, block, 0, at, static_cast<A&&>(args)...);
 }
 
+// SMs of the GPU the size thresholds below were measured on (permutation, lanes a
+// particle, pass 2's records): where one kernel starts to beat another, not
+// limits of a launch.
+constexpr uint32_t kTunedSms = 152u;
+
 constexpr int kSortThreads = 512;
 constexpr int kSortBins = 256;
 constexpr int kSortMaxPasses = 8;

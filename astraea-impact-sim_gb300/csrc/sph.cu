@@ -914,7 +914,7 @@ __device__ __forceinline__ void driftParticle(const AstraeaParticles& p, const W
 }
 
 // 7 blocks per SM (72 registers, 3 words spilled): 295 us at 1M, 6 blocks 319, 8 blocks
-// (80 registers' worth of spills) 340.  The {m, 1 / H} pair is loaded with the
+// (64 registers, more spilled) 340.  The {m, 1 / H} pair is loaded with the
 // record, before it is known whether the candidate is in range: loaded after the
 // test, its latency stood in every pair (354).  With 1 / H there instead of the
 // norm of H, a division less per pair.
@@ -982,14 +982,15 @@ cudaError_t launchBuildNeighbors(const Work& w, uint32_t n, int sms, LaunchAt st
 }
 
 // Lanes per particle of pass 1 and the drift: as many as keep all of the launch's
-// threads resident at once (taken at 6 blocks per SM x 128 x 152 SMs).  Below that a
+// threads resident at once (the lines lie at 6 blocks an SM, where they were
+// measured; the kernels have had 7 since).  Below that a
 // launch lasts as long as one thread's list; above it a lane more per particle
 // only adds sums and partial last fours.  Drift / pass 1 with 1, 2, 4 lanes, us:
 // n = 16k 41.6 / 26.6, 25.9 / 18.4, 19.4 / 15.4 (8 lanes: 24.6 / 18.4); 32k
 // 39.4 / 27.1, 27.7 / 20.5, 31.8 / 23.1; 50k 40.0 / 28.7, 30.8 / 25.1, 36.9 /
 // 28.7; 70k 44.2 / 31.7, 47.9 / 34.8; 200k 87.6 / 63.0, 95.0 / 70.1.
-constexpr uint32_t kPass2Wave = 2u * 128u * 152u;   // threads of two blocks per SM (pass2Kernel)
-constexpr uint32_t kPassWave = 6u * 128u * 152u;
+constexpr uint32_t kPass2Wave = 2u * 128u * kTunedSms;   // threads of two blocks per SM (pass2Kernel)
+constexpr uint32_t kPassWave = 6u * 128u * kTunedSms;
 static uint32_t passBlocks(uint32_t n, int lanes) { return kHeavyBlocks + gridFor(n, static_cast<int>(kPassThreads) / lanes); }
 static int lanesFor(uint32_t n) { return n <= kPassWave / 4u ? 4 : (n <= kPassWave / 2u ? 2 : 1); }
 

@@ -3,8 +3,9 @@
 // Replaces the host loops of Simulation::Impl::computeTelemetryFromDevice
 // (engine/simulation.cpp:948-1285) and sumDeviceRadPowerW (:567-582), which
 // copy 17 particle arrays to the host and walk them seven times.  Here every
-// loop is a device pass in FP64 (the engine's arithmetic), and the scalar
-// state between passes (COMs, the remnant estimate) stays on the device:
+// loop is a device pass that sums in FP64 and decides as the engine's FP64
+// arithmetic does (see Cost), and the scalar state between passes (COMs, the
+// remnant estimate) stays on the device:
 //
 //   pass A   totals: mass, COMs and mean velocities per body (body 0 vs the
 //            rest), kinetic / potential / internal energy, momentum, angular
@@ -36,9 +37,10 @@
 // each pass is one wave of latency: loads, the reduction, the last block).
 //
 // Determinism: each pass is a grid-stride loop over a fixed grid, a block
-// reduction in a fixed order, per-block partials in global memory, and a
-// final sum over the blocks in block order by the last block to finish (an
-// atomic ticket; nothing waits).  Results are identical run to run; against
+// reduction in a fixed order, per-block partials in global memory, and a final
+// sum over the blocks by the last block to finish (an atomic ticket; nothing
+// waits), also in a fixed order: every 32nd block in a lane, then over the
+// lanes.  Results are identical run to run; against
 // the engine's serial loops they differ only by FP64 summation order.
 //
 // Scratch (partials, pass state, result) is file-scope device memory: the
